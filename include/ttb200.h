@@ -208,8 +208,9 @@ int ttb_qr_static(const ttb_qr_t* problems, int count, void* stream);
 
 /* ------------------------------------------------------------------------
  * Thin SVD of an m x k strided matrix, a = u diag(s) vh with s descending,
- * p = min(m, k): u (m x p), s (p), vh (p x k).  Householder QR followed by
- * one-sided Jacobi on the triangular factor.  Replaces the LAPACK gesdd /
+ * p = min(m, k): u (m x p), s (p), vh (p x k).  Either u or vh may be NULL
+ * (not wanted; s times it is then the other factor's product with a).
+ * Householder QR followed by one-sided Jacobi on the triangular factor.  Replaces the LAPACK gesdd /
  * gesvd calls of left_svd / right_svd (ttnumpy/utils.py:336-460) and of
  * _truncate_core_right / _left (ttnumpy/solvers/amen.py:254-260, 301-307).
  * ``status`` (device int, may be NULL) receives the Jacobi sweeps used or

@@ -17,8 +17,10 @@ ROOT = os.path.dirname(HERE)
 OUT = os.path.join(HERE, "libttb200.so")
 
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
-FLAGS = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-shared",
-         "--expt-relaxed-constexpr"]
+# relocatable device code: the factorisations (ttb_factor.cu) are compiled once
+# and linked into the kernels that call them
+FLAGS = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-shared", "-rdc=true",
+         "--threads", "0", "--expt-relaxed-constexpr"]
 
 
 def nvcc() -> str:

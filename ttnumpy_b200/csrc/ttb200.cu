@@ -14,10 +14,11 @@
 
 #include "ttb200.h"
 #include "ttb_device.cuh"
+#include "ttb_factor.cuh"
 
 using namespace ttb;
 
-namespace {
+namespace ttb_grouped {
 
 std::atomic<long long> g_launches{0};
 inline void counted() { g_launches.fetch_add(1, std::memory_order_relaxed); }
@@ -345,8 +346,9 @@ __global__ void __launch_bounds__(TTB_THREADS) k_qr(const __grid_constant__ QBat
   if (m <= 0 || k <= 0) return;
   if (qb.mode[blockIdx.x] == 0) {
     double* W = dsm;
-    double* tau = W + (i64)m * k;
-    cta_qr(CMat{q.a, q.a_rs, q.a_cs}, m, k, W, tau, Mat{q.q, q.q_rs, q.q_cs},
+    const int ldw = odd_step(m);
+    double* tau = W + (i64)ldw * k;
+    cta_qr(CMat{q.a, q.a_rs, q.a_cs}, m, k, W, ldw, tau, Mat{q.q, q.q_rs, q.q_cs},
            Mat{q.r, q.r_rs, q.r_cs}, red);
   } else {
     double* Y = dsm;
@@ -357,7 +359,7 @@ __global__ void __launch_bounds__(TTB_THREADS) k_qr(const __grid_constant__ QBat
   }
 }
 
-i64 qr_need(int m, int k) { return (i64)m * k + std::min(m, k); }
+i64 qr_need(int m, int k) { return (i64)odd_step(m) * k + std::min(m, k); }
 i64 blocked_smem(int k) { return (i64)LNB * std::min(std::max(k, 1), YCH) + 2 * LNB * LNB; }
 
 constexpr int kMaxS = 16;
@@ -368,7 +370,9 @@ struct SBatch {
 };
 
 // doubles of the tall SVD work area for an M x K (M >= K) problem
-i64 svd_tall_need(int M, int K) { return (i64)M * K + 2 * (i64)K * K + 3 * (i64)K + 2; }
+i64 svd_tall_need(int M, int K) {
+  return (i64)odd_step(M) * K + 2 * (i64)svd_step(K) * K + 4 * (i64)K + 6;
+}
 
 __global__ void __launch_bounds__(TTB_THREADS) k_svd(const __grid_constant__ SBatch sb) {
   extern __shared__ double dsm[];
@@ -381,25 +385,27 @@ __global__ void __launch_bounds__(TTB_THREADS) k_svd(const __grid_constant__ SBa
   const int mode = sb.mode[blockIdx.x];
   double* base = mode == 0 ? dsm : q.work;
   double* W = base;
-  double* tau = W + (i64)M * K;
-  double* Bsq = tau + K;
-  double* V = Bsq + (i64)K * K;
-  double* sv = V + (i64)K * K;
+  const int ldw = odd_step(M);
+  double* tau = W + (i64)ldw * K;
+  double* Bsq = align2(tau + K);
+  double* V = Bsq + (i64)svd_step(K) * K;
+  double* sv = V + (i64)svd_step(K) * K;
   int* order = reinterpret_cast<int*>(sv + K);
-  int* flag = reinterpret_cast<int*>(sv + 2 * K);
+  double* tau2 = sv + 2 * K;
+  int* flag = reinterpret_cast<int*>(sv + 3 * K);
   CMat A = tall ? CMat{q.a, q.a_rs, q.a_cs} : CMat{q.a, q.a_cs, q.a_rs};
   // a^T = U' S Vh'  =>  a = Vh'^T S U'^T : U' goes to vh^T, Vh' to u^T
   Mat U = tall ? Mat{q.u, q.u_rs, q.u_cs} : Mat{q.vh, q.vh_cs, q.vh_rs};
   Mat Vh = tall ? Mat{q.vh, q.vh_rs, q.vh_cs} : Mat{q.u, q.u_cs, q.u_rs};
   int st;
   if (mode == 0) {
-    st = cta_svd_tall(A, M, K, W, tau, Bsq, V, sv, order, flag, U, q.s, Vh, red);
+    st = cta_svd_tall(A, M, K, W, ldw, tau, Bsq, V, sv, order, flag, tau2, U, q.s, Vh, red);
   } else {
     double* Y = dsm;
     double* G = Y + (i64)LNB * min(K, YCH);
     double* Tm = G + LNB * LNB;
-    st = cta_svd_tall_blocked(A, M, K, W, tau, Bsq, V, sv, order, flag, U, q.s, Vh, Y, G, Tm,
-                              red, gsm);
+    st = cta_svd_tall_blocked(A, M, K, W, tau, Bsq, V, sv, order, flag, tau2, U, q.s, Vh, Y, G,
+                              Tm, red, gsm);
   }
   if (q.status && threadIdx.x == 0) *q.status = st;
 }
@@ -1197,12 +1203,13 @@ __global__ void __launch_bounds__(TTB_THREADS) k_round(const __grid_constant__ t
   double* Sv = Vh + qslot;
   // shared factorisation area
   double* W = dsm;
-  double* tau = W + (i64)kRoundMaxRows * kRoundMaxBond;
-  double* Bsq = tau + kRoundMaxBond;
-  double* V = Bsq + kRoundMaxBond * kRoundMaxBond;
-  double* sv = V + kRoundMaxBond * kRoundMaxBond;
+  double* tau = W + (i64)odd_step(kRoundMaxRows) * kRoundMaxBond;
+  double* Bsq = align2(tau + kRoundMaxBond);
+  double* V = Bsq + svd_step(kRoundMaxBond) * kRoundMaxBond;
+  double* sv = V + svd_step(kRoundMaxBond) * kRoundMaxBond;
   int* order = reinterpret_cast<int*>(sv + kRoundMaxBond);
-  int* flag = reinterpret_cast<int*>(sv + 2 * kRoundMaxBond);
+  double* tau2 = sv + 2 * kRoundMaxBond;
+  int* flag = reinterpret_cast<int*>(sv + 3 * kRoundMaxBond);
   int status = 0;
   const int RS = kRoundMaxBond;  // row stride of Rm
   // shapes outside the shared-memory plan are refused (status -2)
@@ -1243,8 +1250,8 @@ __global__ void __launch_bounds__(TTB_THREADS) k_round(const __grid_constant__ t
     rows_of[k] = rl;  // rows of core k before its factorisation
     if (k == d - 1) break;
     const int pq = m < r_out ? m : r_out;
-    cta_qr(CMat{X, r_out, 1}, m, r_out, W, tau, Mat{qcores + (i64)k * qslot, pq, 1},
-           Mat{Rm, RS, 1}, red);
+    cta_qr(CMat{X, r_out, 1}, m, r_out, W, odd_step(m), tau,
+           Mat{qcores + (i64)k * qslot, pq, 1}, Mat{Rm, RS, 1}, red);
     rl = pq;
   }
   // ---- norm of the last core and the per-split budget
@@ -1265,12 +1272,13 @@ __global__ void __launch_bounds__(TTB_THREADS) k_round(const __grid_constant__ t
     const int c = n * bond;
     const int p = r < c ? r : c;
     int st;
+    // the right factor only: U S is the matrix times its rows
     if (r >= c) {
-      st = cta_svd_tall(CMat{X, c, 1}, r, c, W, tau, Bsq, V, sv, order, flag, Mat{U, p, 1}, Sv,
-                        Mat{Vh, c, 1}, red);
+      st = cta_svd_tall(CMat{X, c, 1}, r, c, W, odd_step(r), tau, Bsq, V, sv, order, flag, tau2,
+                        Mat{nullptr, 0, 0}, Sv, Mat{Vh, c, 1}, red);
     } else {
-      st = cta_svd_tall(CMat{X, 1, c}, c, r, W, tau, Bsq, V, sv, order, flag, Mat{Vh, 1, c}, Sv,
-                        Mat{U, 1, p}, red);
+      st = cta_svd_tall(CMat{X, 1, c}, c, r, W, odd_step(c), tau, Bsq, V, sv, order, flag, tau2,
+                        Mat{Vh, 1, c}, Sv, Mat{nullptr, 0, 0}, red);
     }
     if (st < 0) status = -1;
     __syncthreads();
@@ -1280,17 +1288,13 @@ __global__ void __launch_bounds__(TTB_THREADS) k_round(const __grid_constant__ t
     // core i = Vh[:nb] as (nb, n, bond)
     double* oc = out + (i64)i * slot;
     for (int e = threadIdx.x; e < nb * c; e += TTB_THREADS) oc[e] = Vh[e];
-    // U[:, :nb] *= S[:nb]
-    for (int e = threadIdx.x; e < r * nb; e += TTB_THREADS) {
-      int a = e / nb, j = e % nb;
-      U[(i64)a * p + j] *= Sv[j];
-    }
-    __syncthreads();
-    // X <- Qcore_{i-1} (rows*n_{i-1} x r) @ U[:, :nb]
+    // U S = X Vh[:nb]^T
+    cta_gemm(CMat{X, c, 1}, CMat{Vh, 1, c}, Mat{U, nb, 1}, r, nb, c, 1.0, 0.0, gsm);
+    // X <- Qcore_{i-1} (rows*n_{i-1} x r) @ (U S)
     const int rows = rows_of[i - 1];
     const int mprev = rows * P.modes[i - 1];
-    cta_gemm(CMat{qcores + (i64)(i - 1) * qslot, r, 1}, CMat{U, p, 1}, Mat{X, nb, 1}, mprev, nb, r,
-             1.0, 0.0, gsm);
+    cta_gemm(CMat{qcores + (i64)(i - 1) * qslot, r, 1}, CMat{U, nb, 1}, Mat{X, nb, 1}, mprev, nb,
+             r, 1.0, 0.0, gsm);
     if (threadIdx.x == 0) P.bonds[(i64)pair * (d + 1) + i] = nb;
     bond = nb;
     r = rows;
@@ -1321,7 +1325,8 @@ __global__ void __launch_bounds__(TTB_THREADS) k_fma_peak(double* out, int iters
   if (s == 12345.678) out[0] = s;  // keeps the chains live
 }
 
-}  // namespace
+}  // namespace ttb_grouped
+using namespace ttb_grouped;
 
 // ---------------------------------------------------------------------------
 // Fixed scratch for ttb_qr_static: one array in the module's own device
@@ -1334,7 +1339,7 @@ __global__ void __launch_bounds__(TTB_THREADS) k_fma_peak(double* out, int iters
 
 static __device__ __align__(256) double g_qr_static[TTB_QR_STATIC_DOUBLES];
 
-namespace {
+namespace ttb_grouped {
 
 constexpr int kStaticDevices = 64;
 constexpr i64 kStaticAlign = 32;  // doubles: every slice starts on 256 bytes
@@ -1361,7 +1366,7 @@ int qr_static_base(double** out) {
   return 0;
 }
 
-}  // namespace
+}  // namespace ttb_grouped
 
 namespace ttb {
 void count_launch() { counted(); }
@@ -1953,8 +1958,8 @@ long long ttb_round_work_doubles(int d, int max_mode, int max_bond) {
 int ttb_round_batch(const ttb_round_t* P, void* stream) {
   if (P->pairs <= 0) return 0;
   if (P->d < 2 || P->d > kRoundMaxD) return (int)cudaErrorInvalidValue;
-  const size_t smem = ((size_t)kRoundMaxRows * kRoundMaxBond + kRoundMaxBond +
-                       2 * (size_t)kRoundMaxBond * kRoundMaxBond + 3 * kRoundMaxBond + 2) *
+  const size_t smem = ((size_t)odd_step(kRoundMaxRows) * kRoundMaxBond + kRoundMaxBond +
+                       2 * (size_t)svd_step(kRoundMaxBond) * kRoundMaxBond + 3 * kRoundMaxBond + 6) *
                       sizeof(double);
   if (int e = smem_limit_once((const void*)k_round, (int)smem, g_smem_round)) return e;
   const long long qslot = (long long)kRoundMaxRows * kRoundMaxBond;

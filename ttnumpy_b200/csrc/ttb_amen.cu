@@ -16,13 +16,14 @@
 
 #include "ttb200.h"
 #include "ttb_device.cuh"
+#include "ttb_factor.cuh"
 #include "ttb_tc_block.cuh"
 
 namespace ttb {
 void count_launch();  // the library's launch counter (ttb200.cu)
 }
 
-namespace {
+namespace ttb_solve {
 
 using namespace ttb;
 
@@ -915,8 +916,9 @@ __device__ __noinline__ void project(Ctx& c, const double* left, int a, int i, c
 // Economic QR of the m x k view A: Q (m x p) and R (p x k) strided outputs.
 __device__ __noinline__ void qr(Ctx& c, CMat A, int m, int k, Mat Q, Mat R) {
   const int p = min(m, k);
-  if ((i64)m * k + p <= kPoolD) {
-    cta_qr(A, m, k, c.pool, c.pool + (i64)m * k, Q, R, c.sm->red);
+  const int ldw = odd_step(m);
+  if ((i64)ldw * k + p <= kPoolD) {
+    cta_qr(A, m, k, c.pool, ldw, c.pool + (i64)ldw * k, Q, R, c.sm->red, false);
     return;
   }
   const i64 mark = c.top;
@@ -931,7 +933,7 @@ __device__ __noinline__ void qr(Ctx& c, CMat A, int m, int k, Mat Q, Mat R) {
       if (c.status) return;
       cta_qr_blocked(A, m, k, W, W + (i64)m * k, Mat{nullptr, 0, 0}, Mat{R1, k, 1}, c.pool,
                      c.pool + (i64)LNB * YCH, c.pool + (i64)LNB * YCH + LNB * LNB, c.sm->red,
-                     *c.gsm);
+                     *c.gsm, nullptr, false);
       double dsq = 0.0, rsq = 0.0;
       for (i64 e = threadIdx.x; e < (i64)p * k; e += TTB_THREADS) {
         const int i = (int)(e / k), j = (int)(e % k);
@@ -950,7 +952,7 @@ __device__ __noinline__ void qr(Ctx& c, CMat A, int m, int k, Mat Q, Mat R) {
   double* Y = c.pool;
   double* G = Y + (i64)LNB * YCH;
   double* Tm = G + LNB * LNB;
-  cta_qr_blocked(A, m, k, W, W + (i64)m * k, Q, R, Y, G, Tm, c.sm->red, *c.gsm, c.ring);
+  cta_qr_blocked(A, m, k, W, W + (i64)m * k, Q, R, Y, G, Tm, c.sm->red, *c.gsm, c.ring, false);
   c.top = mark;
 }
 
@@ -961,7 +963,8 @@ __device__ __noinline__ void svd(Ctx& c, CMat A, int m, int k, Mat U, double* S,
   CMat At = tall ? A : CMat{A.p, A.cs, A.rs};
   Mat Ut = tall ? U : Mat{Vh.p, Vh.cs, Vh.rs};
   Mat Vt = tall ? Vh : Mat{U.p, U.cs, U.rs};
-  const i64 need = (i64)M * K + 2 * (i64)K * K + 3 * (i64)K + 2;
+  const int ldw = odd_step(M);
+  const i64 need = (i64)ldw * K + 2 * (i64)svd_step(K) * K + 4 * (i64)K + 6;
   const i64 mark = c.top;
   double* base;
   const bool in_pool = need <= kPoolD;
@@ -972,20 +975,22 @@ __device__ __noinline__ void svd(Ctx& c, CMat A, int m, int k, Mat U, double* S,
     if (c.status) return;
   }
   double* W = base;
-  double* tau = W + (i64)M * K;
-  double* Bsq = tau + K;
-  double* V = Bsq + (i64)K * K;
-  double* sv = V + (i64)K * K;
+  double* tau = W + (i64)ldw * K;
+  double* Bsq = align2(tau + K);
+  double* V = Bsq + (i64)svd_step(K) * K;
+  double* sv = V + (i64)svd_step(K) * K;
   int* order = reinterpret_cast<int*>(sv + K);
-  int* flag = reinterpret_cast<int*>(sv + 2 * K);
+  double* tau2 = sv + 2 * K;
+  int* flag = reinterpret_cast<int*>(sv + 3 * K);
   if (in_pool) {
-    cta_svd_tall(At, M, K, W, tau, Bsq, V, sv, order, flag, Ut, S, Vt, c.sm->red);
+    cta_svd_tall(At, M, K, W, ldw, tau, Bsq, V, sv, order, flag, tau2, Ut, S, Vt, c.sm->red,
+                 false);
   } else {
     double* Y = c.pool;
     double* G = Y + (i64)LNB * YCH;
     double* Tm = G + LNB * LNB;
-    cta_svd_tall_blocked(At, M, K, W, tau, Bsq, V, sv, order, flag, Ut, S, Vt, Y, G, Tm,
-                         c.sm->red, *c.gsm, c.ring);
+    cta_svd_tall_blocked(At, M, K, W, tau, Bsq, V, sv, order, flag, tau2, Ut, S, Vt, Y, G, Tm,
+                         c.sm->red, *c.gsm, c.ring, false);
   }
   c.top = mark;
 }
@@ -2488,7 +2493,8 @@ __global__ void __launch_bounds__(TTB_THREADS, 1)
   }
 }
 
-}  // namespace
+}  // namespace ttb_solve
+using namespace ttb_solve;
 
 extern "C" {
 
@@ -2528,7 +2534,7 @@ long long ttb_amen_slab_doubles(int d, const int* dims, int kickrank, int rmax,
   const long long iter = N + std::max(6 * N, (kRestart + 3) * (N + 32) + 2048) + apply;
   const long long rank = 4 * N + 2LL * kRankChunk * R * n * r + R * r * r + r * r + apply;
   const long long fact = r * n * r + r + r * n * r        // U S Vh
-                         + (r * n) * r + 2 * r * r + 4 * r  // svd work
+                         + (r * n) * r + 2 * r * (r + 16) + 6 * r + 6  // svd work
                          + (r * n) * cols + 2 * cols * n * r + r * r  // enriched, padded, svh
                          + r * n * cols + cols * cols + cols * n * r  // Q, R, next
                          + r * n * cols + cols + r * n * K;            // qr work, block

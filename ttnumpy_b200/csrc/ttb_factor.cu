@@ -1,0 +1,1688 @@
+// Factorisations executed by one thread block of TTB_THREADS threads:
+// Householder QR, Jacobi SVD and pivoted Gaussian elimination.
+//
+// The matrices of tensor-train work are small (columns a bond, rows a bond
+// times a mode), so what bounds their factorisation on one SM is the chain
+// of column steps: a reduction, a scale factor, an update, a barrier.  The
+// register-tiled routines keep whole columns in registers, eight lanes to a
+// column where the rows allow it: a column step is one dot product per
+// column, three shuffle levels for four columns of a warp together, one
+// update, and one block barrier in all.
+//
+// They are compiled once, here, and called from the kernels of the other
+// files (relocatable device code): inlined into every kernel, ptxas spent
+// minutes on each.
+#include "ttb_factor.cuh"
+
+namespace ttb {
+
+// W (column major, column step ldw) <- the m x k view A, reading along A's
+// unit-stride direction.
+static __device__ __forceinline__ void cta_load(CMat A, double* W, i64 ldw, int m, int k) {
+  const int total = m * k;
+  if (A.cs == 1) {
+    for (int e = threadIdx.x; e < total; e += TTB_THREADS) {
+      const int i = e / k, j = e - i * k;
+      W[i + j * ldw] = A(i, j);
+    }
+  } else {
+    for (int e = threadIdx.x; e < total; e += TTB_THREADS) {
+      const int j = e / m, i = e - j * m;
+      W[i + j * ldw] = A(i, j);
+    }
+  }
+}
+
+// ---------------------------------------------------------------------------
+// Householder QR
+// ---------------------------------------------------------------------------
+
+// In-place Householder QR of the m x k matrix W (column step ``ldw``, unit
+// row step), as LAPACK dgeqr2 lays it out: on return R is in the upper
+// triangle and the reflector vectors v_j (v_j[j] = 1 implied) below the
+// diagonal, with the scalars in tau[0 .. min(m,k)-1].  Each reflector is
+// H = I - tau v v^T built as in dlarfg: beta = -sign(alpha) ||x||,
+// tau = (beta - alpha) / beta, v = x / (alpha - beta); a column whose
+// sub-diagonal part is exactly zero gets tau = 0.
+static __device__ void cta_householder(double* W, int m, int k, i64 ldw, double* tau, double* red) {
+  // The whole block works on every reflector: the trailing columns are
+  // taken HC at a time, their dot products with v accumulated per thread
+  // over a row stripe and reduced together, and the squared norm of the
+  // next column is gathered during its update (one pass fewer per column).
+  constexpr int HC = 16;
+  __shared__ double hred[TTB_WARPS][HC];
+  __shared__ double hw[HC];
+  const int p = m < k ? m : k;
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  double part = 0.0;
+  for (int i = 1 + tid; i < m; i += TTB_THREADS) part = fma(W[i], W[i], part);
+  double sigma = block_sum(part, red);
+  for (int j = 0; j < p; ++j) {
+    double* col = W + j * ldw;
+    const double alpha = col[j];
+    double t = 0.0, beta = alpha, scale = 0.0;
+    if (sigma != 0.0) {
+      const double nrm = sqrt(alpha * alpha + sigma);
+      beta = (alpha >= 0.0) ? -nrm : nrm;
+      t = (beta - alpha) / beta;
+      scale = 1.0 / (alpha - beta);
+    }
+    __syncthreads();  // everyone has read col[j] before it is overwritten
+    if (sigma != 0.0) {
+      for (int i = j + 1 + tid; i < m; i += TTB_THREADS) col[i] *= scale;
+    }
+    if (tid == 0) {
+      col[j] = beta;
+      tau[j] = t;
+    }
+    __syncthreads();
+    double next = 0.0;  // this thread's part of |column j+1, rows > j+1|^2
+    for (int c0 = j + 1; c0 < k; c0 += HC) {
+      const int nc = min(HC, k - c0);
+      double* cb = W + (i64)c0 * ldw;
+      if (t != 0.0) {
+        double w[HC];
+#pragma unroll
+        for (int q = 0; q < HC; ++q) w[q] = 0.0;
+        for (int i = j + 1 + tid; i < m; i += TTB_THREADS) {
+          const double v = col[i];
+#pragma unroll
+          for (int q = 0; q < HC; ++q)
+            if (q < nc) w[q] = fma(v, cb[i + q * ldw], w[q]);
+        }
+#pragma unroll
+        for (int q = 0; q < HC; ++q) {
+          const double sw = warp_sum(w[q]);
+          if (lane == 0) hred[wid][q] = sw;
+        }
+        __syncthreads();
+        if (tid < nc) {
+          double sw = 0.0;
+          for (int q = 0; q < TTB_WARPS; ++q) sw += hred[q][tid];
+          const double wv = t * (sw + cb[j + tid * ldw]);
+          hw[tid] = wv;
+          cb[j + tid * ldw] -= wv;
+        }
+        __syncthreads();
+        for (int i = j + 1 + tid; i < m; i += TTB_THREADS) {
+          const double v = col[i];
+#pragma unroll
+          for (int q = 0; q < HC; ++q) {
+            if (q < nc) {
+              const double x = fma(-hw[q], v, cb[i + q * ldw]);
+              cb[i + q * ldw] = x;
+              if (q == 0 && c0 == j + 1 && i > j + 1) next = fma(x, x, next);
+            }
+          }
+        }
+        __syncthreads();  // hred and hw are reused by the next chunk
+      } else if (c0 == j + 1) {
+        for (int i = j + 2 + tid; i < m; i += TTB_THREADS) next = fma(cb[i], cb[i], next);
+      }
+    }
+    if (j + 1 < p) sigma = block_sum(next, red);
+  }
+}
+
+// Overwrite the m x q matrix X (strided) with H_0 H_1 ... H_{p-1} X, the
+// reflectors of cta_householder (applied last to first).
+static __device__ void cta_apply_q(const double* W, int m, int p, i64 ldw, const double* tau, Mat X,
+                            int q) {
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  for (int j = p - 1; j >= 0; --j) {
+    const double t = tau[j];
+    if (t != 0.0) {
+      const double* v = W + j * ldw;
+      for (int c = wid; c < q; c += TTB_WARPS) {
+        double w = 0.0;
+        for (int i = j + 1 + lane; i < m; i += 32) w = fma(v[i], X(i, c), w);
+        w = warp_sum(w) + X(j, c);
+        w *= t;
+        if (lane == 0) X(j, c) -= w;
+        for (int i = j + 1 + lane; i < m; i += 32) X(i, c) = fma(-w, v[i], X(i, c));
+      }
+    }
+    __syncthreads();
+  }
+}
+
+// ---------------------------------------------------------------------------
+// register-tiled Householder QR
+// ---------------------------------------------------------------------------
+
+// A register tile gives a matrix column to LPC lanes of a warp: lane q of the
+// column's group holds the row pairs 2 q + 2 LPC t + {0, 1}, RP rows in all
+// (RP LPC rows at most).  A warp works on 32 / LPC columns at once, one per
+// group, in each of its SL slots; slot s of warp w holds the columns
+// G TTB_WARPS s + G w + group, G = 32 / LPC.
+template <int LPC>
+static __device__ __forceinline__ int tile_row(int r) {
+  return 2 * LPC * (r >> 1) + 2 * (threadIdx.x & (LPC - 1)) + (r & 1);
+}
+template <int LPC>
+static __device__ __forceinline__ int tile_col(int s) {
+  constexpr int G = 32 / LPC;
+  return G * (TTB_WARPS * s + (threadIdx.x >> 5)) + (threadIdx.x & 31) / LPC;
+}
+
+// Sum over a column's lanes, every one of them getting it.
+template <int LPC>
+static __device__ __forceinline__ double group_sum(double v) {
+#pragma unroll
+  for (int o = LPC / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
+// Inner product over this lane's rows, four chains deep.
+template <int RP>
+static __device__ __forceinline__ double lane_dot(const double (&x)[RP], const double (&y)[RP]) {
+  constexpr int C = RP >= 8 ? 4 : 2;
+  double a[C];
+#pragma unroll
+  for (int q = 0; q < C; ++q) a[q] = 0.0;
+#pragma unroll
+  for (int r = 0; r < RP; ++r) a[r % C] = fma(x[r], y[r], a[r % C]);
+#pragma unroll
+  for (int q = 2; q < C; q += 2) {
+    a[0] += a[q];
+    a[1] += a[q + 1];
+  }
+  return a[0] + a[1];
+}
+
+// Column ``col`` of a matrix with unit row step, rows below m (zeros beyond).
+template <int LPC, int RP>
+static __device__ __forceinline__ void tile_load(const double* col, int m, double (&x)[RP]) {
+  const bool even = (reinterpret_cast<uintptr_t>(col) & 15) == 0;
+#pragma unroll
+  for (int r = 0; r < RP; r += 2) {
+    const int i = tile_row<LPC>(r);
+    if (2 * LPC * (r >> 1) + 2 * LPC <= m && even) {
+      const double2 p = *reinterpret_cast<const double2*>(col + i);
+      x[r] = p.x;
+      x[r + 1] = p.y;
+    } else {
+      x[r] = i < m ? col[i] : 0.0;
+      x[r + 1] = i + 1 < m ? col[i + 1] : 0.0;
+    }
+  }
+}
+
+// Reflector j of the factored panel in W (unit row step, column step ld,
+// v[j] = 1 implied, zeros above).  A panel has at most 64 columns, so only
+// the first 64 rows need the test.
+constexpr int kPanelMax = 64;
+template <int LPC, int RP, int TEST = kPanelMax>
+static __device__ __forceinline__ void hh_load(const double* W, i64 ld, int m, int j,
+                                               double (&v)[RP]) {
+  tile_load<LPC, RP>(W + j * ld, m, v);
+#pragma unroll
+  for (int r = 0; r < RP; ++r) {
+    if (2 * LPC * (r >> 1) >= TEST) break;
+    const int i = tile_row<LPC>(r);
+    if (i <= j) v[r] = i == j ? 1.0 : 0.0;
+  }
+}
+
+// beta, tau and the scale of a column's reflector (LAPACK dlarfg): alpha its
+// pivot entry, sigma the squared norm below it.
+static __device__ __forceinline__ void hh_scalars(double alpha, double sigma, double& beta,
+                                                  double& tau, double& scale) {
+  beta = alpha;
+  tau = 0.0;
+  scale = 0.0;
+  if (sigma != 0.0) {
+    const double nrm = sqrt(alpha * alpha + sigma);
+    beta = (alpha >= 0.0) ? -nrm : nrm;
+    tau = (beta - alpha) / beta;
+    scale = __drcp_rn(alpha - beta);
+  }
+}
+
+// A column in registers becomes reflector j (every group of the warp makes
+// its own; the caller keeps the owner's): scaled in place below row j, beta
+// at row j.  Returns tau.
+template <int LPC, int RP, int TEST = kPanelMax>
+static __device__ __forceinline__ double hh_make(double (&x)[RP], int j) {
+  double a = 0.0, y[RP];
+#pragma unroll
+  for (int r = 0; r < RP; ++r) {
+    const int i = tile_row<LPC>(r);
+    y[r] = x[r];
+    if (2 * LPC * (r >> 1) >= TEST) continue;
+    if (i == j) a = x[r];
+    if (i <= j) y[r] = 0.0;
+  }
+  // row j is held by lane (j / 2) mod LPC of each group
+  a = __shfl_sync(0xffffffffu, a, (threadIdx.x & 31 & ~(LPC - 1)) + ((j >> 1) & (LPC - 1)));
+  const double sigma = group_sum<LPC>(lane_dot<RP>(y, y));
+  double beta, tau, scale;
+  hh_scalars(a, sigma, beta, tau, scale);
+  if (tau != 0.0) {
+#pragma unroll
+    for (int r = 0; r < RP; ++r) {
+      const int i = tile_row<LPC>(r);
+      if (2 * LPC * (r >> 1) >= TEST) {
+        x[r] *= scale;
+      } else {
+        if (i > j) x[r] *= scale;
+        if (i == j) x[r] = beta;
+      }
+    }
+  }
+  return tau;
+}
+
+// dst = x[at] for a warp-uniform ``at``: a chain of moves the compiler does
+// not turn into an indexed array (which would put x in local memory).
+template <int RP, int SL>
+static __device__ __forceinline__ void pick_slot(const double (&x)[SL][RP], int at,
+                                                 double (&dst)[RP]) {
+#pragma unroll
+  for (int r = 0; r < RP; ++r) dst[r] = x[0][r];
+#pragma unroll
+  for (int s = 1; s < SL; ++s)
+    if (s == at) {
+#pragma unroll
+      for (int r = 0; r < RP; ++r) asm volatile("mov.f64 %0, %1;" : "=d"(dst[r]) : "d"(x[s][r]));
+    }
+}
+
+// x[s] -= t (v . x[s]) v in every slot from ``first`` on.
+template <int LPC, int RP, int SL>
+static __device__ __forceinline__ void hh_reflect(double (&x)[SL][RP], const double (&v)[RP],
+                                                  double t, int first) {
+  double w[SL];
+#pragma unroll
+  for (int s = 0; s < SL; ++s) w[s] = s < first ? 0.0 : lane_dot<RP>(v, x[s]);
+#pragma unroll
+  for (int s = 0; s < SL; ++s) w[s] = -t * group_sum<LPC>(w[s]);
+#pragma unroll
+  for (int s = 0; s < SL; ++s) {
+    if (s < first) continue;
+#pragma unroll
+    for (int r = 0; r < RP; ++r) x[s][r] = fma(w[s], v[r], x[s][r]);
+  }
+}
+
+// Householder QR of the m x k panel in W, m <= LPC RP, k <= 32 / LPC *
+// TTB_WARPS * SL <= 64, in place in LAPACK dgeqr2's layout (see
+// cta_householder).  The warp that owns column j + 1 makes the next reflector
+// as soon as reflector j has been applied to it, so that a column step has
+// one barrier.  Bound by the chain of a column step (about 2000 cycles at 256
+// rows: two reductions, a square root and two reciprocals).  256 x 64 with
+// its Q took 2.92 ms column by column (a block-wide reduction and three
+// barriers per 16 columns of every step) and takes 0.21 ms, its R alone 0.44
+// and 0.14 ms; 64 x 64 with Q 0.96 and 0.11 ms.
+template <int LPC, int RP, int SL>
+static __device__ __noinline__ void hh_panel(double* W, i64 ld, int m, int k, double* tau) {
+  constexpr int G = 32 / LPC;
+  const int warp = threadIdx.x >> 5;
+  const int p = m < k ? m : k;
+  double x[SL][RP];
+#pragma unroll
+  for (int s = 0; s < SL; ++s) {
+    const int c = tile_col<LPC>(s);
+    tile_load<LPC, RP>(W + c * ld, c < k ? m : 0, x[s]);
+  }
+  for (int j = -1; j < p; ++j) {
+    __syncthreads();  // reflector j is in W (first: every warp has its columns)
+    const double t = j >= 0 ? tau[j] : 0.0;
+    // columns past j: those of slots from ``first`` on (a finished column's
+    // registers are not used again)
+    const int first = SL > 1 && G * (warp + 1) <= j + 1 - G * TTB_WARPS * (SL - 2) ? SL - 1 : 0;
+    if (t != 0.0 && G * (TTB_WARPS * (SL - 1) + warp + 1) > j + 1) {
+      double v[RP];
+      hh_load<LPC, RP>(W, ld, m, j, v);
+      hh_reflect<LPC, RP, SL>(x, v, t, first);
+    }
+    if (j + 1 < p && warp == ((j + 1) / G) % TTB_WARPS) {  // the next reflector
+      double col[RP];
+      const int s = (j + 1) / (G * TTB_WARPS);
+      pick_slot<RP, SL>(x, s, col);
+      const double tn = hh_make<LPC, RP>(col, j + 1);
+      if (tile_col<LPC>(s) == j + 1) {
+        if ((threadIdx.x & (LPC - 1)) == 0) tau[j + 1] = tn;
+        double* wc = W + (j + 1) * ld;
+#pragma unroll
+        for (int r = 0; r < RP; ++r) {
+          const int i = tile_row<LPC>(r);
+          if (i < m) wc[i] = col[r];
+        }
+      }
+    }
+  }
+#pragma unroll
+  for (int s = 0; s < SL; ++s) {
+    const int c = tile_col<LPC>(s);
+    if (c < p || c >= k) continue;
+#pragma unroll
+    for (int r = 0; r < RP; ++r) {
+      const int i = tile_row<LPC>(r);
+      if (i < m) W[i + c * ld] = x[s][r];
+    }
+  }
+  __syncthreads();
+}
+
+// Where the columns of hh_columns start: the matrix X itself, the identity,
+// or [top(:, order); 0] with top kt x kt column major (column step ktop).
+enum { HH_X = 0, HH_IDENT = 1, HH_TOP = 2 };
+
+// A panel's p <= 64 reflectors in W applied to ncols columns of X (m x
+// ncols, any strides), first to last (FWD: H^T) or last to first (Q).  Each
+// column stays with its lanes, so no barrier is needed.  From an identity
+// start (column c the unit vector c) reflector j leaves the columns below j
+// alone.
+template <int LPC, int RP, int SL, bool FWD>
+static __device__ __noinline__ void hh_columns(const double* W, i64 ld, int m, int p,
+                                               const double* tau, Mat X, int ncols, int start,
+                                               const double* top, int kt, i64 ktop,
+                                               const int* order) {
+  constexpr int G = 32 / LPC, STEP = G * TTB_WARPS * SL;
+  const int warp = threadIdx.x >> 5;
+  for (int g0 = 0; g0 < ncols; g0 += STEP) {
+    if (g0 + G * warp >= ncols) break;
+    double x[SL][RP];
+#pragma unroll
+    for (int s = 0; s < SL; ++s) {
+      const int c = g0 + tile_col<LPC>(s);
+      if (start == HH_TOP) {
+        const bool in = c < ncols;
+        tile_load<LPC, RP>(in ? top + order[c] * ktop : top, in ? kt : 0, x[s]);
+      } else {
+#pragma unroll
+        for (int r = 0; r < RP; ++r) {
+          const int i = tile_row<LPC>(r);
+          x[s][r] = 0.0;
+          if (start == HH_IDENT) x[s][r] = i == c ? 1.0 : 0.0;
+          else if (c < ncols && i < m) x[s][r] = X(i, c);
+        }
+      }
+    }
+    const int last = start == HH_IDENT
+                         ? min(p - 1, g0 + G * (TTB_WARPS * (SL - 1) + warp + 1) - 1)
+                         : p - 1;
+    for (int q = 0; q <= last; ++q) {
+      const int j = FWD ? q : last - q;
+      const double t = tau[j];
+      if (t == 0.0) continue;
+      double v[RP];
+      hh_load<LPC, RP>(W, ld, m, j, v);
+      hh_reflect<LPC, RP, SL>(x, v, t, 0);
+    }
+#pragma unroll
+    for (int s = 0; s < SL; ++s) {
+      const int c = g0 + tile_col<LPC>(s);
+      if (c >= ncols) continue;
+#pragma unroll
+      for (int r = 0; r < RP; ++r) {
+        const int i = tile_row<LPC>(r);
+        if (i < m) X(i, c) = x[s][r];
+      }
+    }
+  }
+}
+
+// Most rows the register tiles take.
+constexpr int kHHRows = 2048;
+
+// The tile for a panel of ``rows`` rows: eight lanes a column up to 256 rows
+// (64 columns in a block), 16 up to 512 (32), the whole warp beyond (16 up to
+// 1024 rows, then 8): 64 doubles of a thread's registers at most.
+#define TTB_HH_TILE(rows, CALL)        \
+  if ((rows) <= 32) { CALL(8, 4, 2); } \
+  else if ((rows) <= 64) { CALL(8, 8, 2); }    \
+  else if ((rows) <= 128) { CALL(8, 16, 2); }  \
+  else if ((rows) <= 256) { CALL(8, 32, 2); }  \
+  else if ((rows) <= 512) { CALL(16, 32, 2); } \
+  else if ((rows) <= 1024) { CALL(32, 32, 2); } \
+  else { CALL(32, 64, 1); }
+
+static __device__ __forceinline__ int hh_width(int m) {
+  return m <= 256 ? 64 : m <= 512 ? 32 : m <= 1024 ? 16 : 8;
+}
+
+// One panel's reflectors applied to columns (see hh_columns).
+template <bool FWD>
+static __device__ __noinline__ void cta_hh_panel_apply(const double* W, i64 ld, int m, int p,
+                                                       const double* tau, Mat X, int ncols,
+                                                       int start, const double* top, int kt,
+                                                       i64 ktop, const int* order) {
+#define TTB_HH_APPLY(L, R, S) \
+  hh_columns<L, R, S, FWD>(W, ld, m, p, tau, X, ncols, start, top, kt, ktop, order)
+  TTB_HH_TILE(m, TTB_HH_APPLY)
+#undef TTB_HH_APPLY
+  __syncthreads();
+}
+
+// The p reflectors in W applied to X's ncols columns, last to first: Q X,
+// Q [top(:, order); 0] or, from the identity, Q itself.  Up to kPanelMax
+// reflectors at a time; only the last group can start from anything but X.
+static __device__ void cta_hh_apply(const double* W, i64 ld, int m, int p, const double* tau,
+                                    Mat X, int ncols, int start, const double* top = nullptr,
+                                    int kt = 0, i64 ktop = 0, const int* order = nullptr) {
+  if (p > kPanelMax && start != HH_X) {
+    for (int e = threadIdx.x; e < m * ncols; e += TTB_THREADS) {
+      const int i = e / ncols, c = e % ncols;
+      X(i, c) = start == HH_IDENT ? (i == c ? 1.0 : 0.0)
+                                  : (i < kt ? top[i + order[c] * ktop] : 0.0);
+    }
+    __syncthreads();
+  }
+  for (int j0 = ((p - 1) / kPanelMax) * kPanelMax; j0 >= 0; j0 -= kPanelMax) {
+    const bool whole = p <= kPanelMax;
+    // from the identity, columns below j0 are still unit vectors there
+    const int c0 = start == HH_IDENT ? j0 : 0;
+    cta_hh_panel_apply<false>(W + j0 + j0 * ld, ld, m - j0, min(kPanelMax, p - j0), tau + j0,
+                              Mat{X.p + j0 * X.rs + c0 * X.cs, X.rs, X.cs}, ncols - c0,
+                              whole ? start : HH_X, top, kt, ktop, order);
+  }
+}
+
+// cta_householder for m <= kHHRows: column panels as wide as the registers
+// allow, each panel's reflectors applied to the columns right of it.
+static __device__ __noinline__ void cta_hh(double* W, i64 ld, int m, int k, double* tau) {
+  const int p = m < k ? m : k;
+  const int width = hh_width(m);
+  for (int j0 = 0; j0 < p; j0 += width) {
+    const int cols = min(width, k - j0), rows = m - j0;
+    double* P = W + j0 + j0 * ld;
+#define TTB_HH_PANEL(L, R, S) hh_panel<L, R, S>(P, ld, rows, cols, tau + j0)
+    TTB_HH_TILE(rows, TTB_HH_PANEL)
+#undef TTB_HH_PANEL
+    const int rest = k - j0 - cols;
+    if (rest > 0)
+      cta_hh_panel_apply<true>(P, ld, rows, min(cols, rows), tau + j0,
+                               Mat{P + cols * ld, 1, ld}, rest, HH_X, nullptr, 0, 0, nullptr);
+  }
+}
+
+// Economic QR of the m x k matrix ``A`` (any strides): Q (m x p) and R
+// (p x k), p = min(m, k).  ``W`` is a column-major work area (unit row step,
+// column step ldw >= m; an odd one spreads a row over the shared-memory
+// banks), ``tau`` p doubles; both may be shared or global memory.  Q and R
+// may be NULL to skip them.
+__device__ __noinline__ void cta_qr(CMat A, int m, int k, double* W, i64 ldw, double* tau, Mat Q,
+                                    Mat R, double* red, bool tiled) {
+  const int p = m < k ? m : k;
+  cta_load(A, W, ldw, m, k);
+  __syncthreads();
+  const bool tiles = tiled && m <= kHHRows;
+  if (tiles)
+    cta_hh(W, ldw, m, k, tau);
+  else
+    cta_householder(W, m, k, ldw, tau, red);
+  if (R.p) {
+    for (int e = threadIdx.x; e < p * k; e += TTB_THREADS) {
+      int i = e / k, j = e % k;
+      R(i, j) = (i <= j) ? W[i + j * ldw] : 0.0;
+    }
+  }
+  if (Q.p) {
+    if (tiles) {
+      cta_hh_apply(W, ldw, m, p, tau, Q, p, HH_IDENT);
+    } else {
+      for (int e = threadIdx.x; e < m * p; e += TTB_THREADS) {
+        int i = e % m, j = e / m;
+        Q(i, j) = (i == j) ? 1.0 : 0.0;
+      }
+      __syncthreads();
+      cta_apply_q(W, m, p, ldw, tau, Q, p);
+    }
+  }
+  __syncthreads();
+}
+
+// ---------------------------------------------------------------------------
+// one-sided Jacobi SVD
+// ---------------------------------------------------------------------------
+
+// Hestenes one-sided Jacobi on the columns of the k x k matrix B (column
+// major, leading dimension ldb): finds an orthogonal J with B J having
+// orthogonal columns.  On return B holds B J and V (column major, ldv; may be
+// NULL) V J.
+// Pairs are visited in round-robin tournament order
+// (k/2 disjoint pairs per round, one warp per pair).  A pair is rotated when
+// |b_p . b_q| > tol sqrt(|b_p|^2 |b_q|^2); sweeps stop when one sweep
+// rotates nothing, or after ``max_sweeps``.  Returns the sweeps used, or -1
+// when the cap was hit.
+static __device__ int cta_jacobi(double* B, int k, i64 ldb, double* V, i64 ldv, int max_sweeps,
+                          double tol, int* flag) {
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  if (k < 2) {
+    __syncthreads();
+    return 0;
+  }
+  const int kk = (k + 1) & ~1;  // players, one dummy when k is odd
+  const int half = kk / 2;
+  for (int sweep = 0; sweep < max_sweeps; ++sweep) {
+    if (threadIdx.x == 0) *flag = 0;
+    __syncthreads();
+    int rotated = 0;
+    for (int round = 0; round < kk - 1; ++round) {
+      for (int pr = wid; pr < half; pr += TTB_WARPS) {
+        int pa = (pr == 0) ? 0 : ((pr - 1 + round) % (kk - 1)) + 1;
+        int pos = kk - 1 - pr;
+        int pb = ((pos - 1 + round) % (kk - 1)) + 1;
+        int p = pa < pb ? pa : pb, q = pa < pb ? pb : pa;
+        if (q >= k) continue;  // paired with the dummy player
+        double* bp = B + p * ldb;
+        double* bq = B + q * ldb;
+        double al = 0.0, be = 0.0, ga = 0.0;
+        for (int i = lane; i < k; i += 32) {
+          double x = bp[i], y = bq[i];
+          al = fma(x, x, al);
+          be = fma(y, y, be);
+          ga = fma(x, y, ga);
+        }
+        al = warp_sum(al);
+        be = warp_sum(be);
+        ga = warp_sum(ga);
+        if (ga != 0.0 && fabs(ga) > tol * sqrt(al) * sqrt(be)) {
+          double zeta = (be - al) / (2.0 * ga);
+          double t = (zeta >= 0.0 ? 1.0 : -1.0) / (fabs(zeta) + sqrt(1.0 + zeta * zeta));
+          double c = 1.0 / sqrt(1.0 + t * t);
+          double s = c * t;
+          for (int i = lane; i < k; i += 32) {
+            double x = bp[i], y = bq[i];
+            bp[i] = c * x - s * y;
+            bq[i] = s * x + c * y;
+          }
+          double* vp = V + p * ldv;
+          double* vq = V + q * ldv;
+          for (int i = lane; V && i < k; i += 32) {
+            double x = vp[i], y = vq[i];
+            vp[i] = c * x - s * y;
+            vq[i] = s * x + c * y;
+          }
+          rotated = 1;
+        }
+      }
+      __syncthreads();
+    }
+    if (rotated) *flag = 1;  // benign race: every writer stores 1
+    __syncthreads();
+    int any = *flag;
+    __syncthreads();
+    if (!any) return sweep + 1;
+  }
+  return -1;
+}
+
+// Column-pivoted Householder QR of the upper-triangular k x k matrix R
+// (column major, column step ld), k <= 8 RP and 32 SL: R P = Q R1, in place
+// in LAPACK dgeqr2's layout; perm[j] is the column of R that came j-th, nrm
+// (k) work.  Each step takes the remaining column of largest norm below the
+// pivot row, the norms recomputed from the updated columns.
+template <int RP, int SL>
+static __device__ __noinline__ void hh_pivot(double* R, int k, i64 ld, int* perm, double* nrm,
+                                             double* tau) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  double x[SL][RP];
+  unsigned done = 0;  // the slots whose column (this lane group's) is taken
+#pragma unroll
+  for (int s = 0; s < SL; ++s) {
+    const int c = tile_col<8>(s);
+    tile_load<8, RP>(R + c * ld, c < k ? k : 0, x[s]);
+    if (c >= k) done |= 1u << s;
+  }
+  for (int j = -1; j < k; ++j) {
+    if (j >= 0) {
+      __syncthreads();  // the norms of this step
+      // every warp finds the same pivot: the lowest column on ties, a NaN
+      // before any number (a taken column, at -1, must never win)
+      double best = -1.0;
+      int at = -1;
+#pragma unroll
+      for (int s = 0; s < SL; ++s) {
+        const int c = lane + 32 * s;
+        double v = c < k ? nrm[c] : -1.0;
+        if (v != v) v = INFINITY;
+        if (c < k && (at < 0 || v > best)) {
+          best = v;
+          at = c;
+        }
+      }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        const double b2 = __shfl_xor_sync(0xffffffffu, best, o);
+        const int a2 = __shfl_xor_sync(0xffffffffu, at, o);
+        if (a2 >= 0 && (at < 0 || b2 > best || (b2 == best && a2 < at))) {
+          best = b2;
+          at = a2;
+        }
+      }
+      at = __shfl_sync(0xffffffffu, at, 0);
+      __syncthreads();  // every warp has read the norms
+      if (warp == (at >> 2) % TTB_WARPS) {
+        double col[RP];
+        const int s = at >> 5;
+        pick_slot<RP, SL>(x, s, col);
+        const double t = hh_make<8, RP, 8 * RP>(col, j);
+        if (tile_col<8>(s) == at) {
+          done |= 1u << s;
+          if ((lane & 7) == 0) {
+            tau[j] = t;
+            perm[j] = at;
+            nrm[at] = -1.0;
+          }
+#pragma unroll
+          for (int r = 0; r < RP; ++r) {
+            const int i = tile_row<8>(r);
+            if (i < k) R[i + j * ld] = col[r];
+          }
+        }
+      }
+      __syncthreads();  // reflector j is in R
+      const double t = tau[j];
+      if (t != 0.0) {
+        double v[RP];
+        hh_load<8, RP, 8 * RP>(R, ld, k, j, v);
+        hh_reflect<8, RP, SL>(x, v, t, 0);
+      }
+    } else {
+      __syncthreads();  // every warp has its columns of R
+    }
+    // squared norms of the remaining columns below row j
+#pragma unroll
+    for (int s = 0; s < SL; ++s) {
+      double y[RP];
+#pragma unroll
+      for (int r = 0; r < RP; ++r) y[r] = tile_row<8>(r) > j ? x[s][r] : 0.0;
+      const double n2 = group_sum<8>(lane_dot<RP>(y, y));
+      if ((lane & 7) == 0 && !(done & (1u << s))) nrm[tile_col<8>(s)] = n2;
+    }
+  }
+  __syncthreads();
+}
+
+// Cosine and sine of the Jacobi rotation of two columns with squared norms
+// al and be and inner product ga, the rotation of smaller angle that makes
+// them orthogonal, for squared norms whose products leave the exponent range.
+static __device__ __noinline__ bool jacobi_angle_wide(double al, double be, double ga, double tol,
+                                                      double& c, double& s) {
+  if (!(fabs(ga) > tol * sqrt(al) * sqrt(be))) return false;
+  const double zeta = (be - al) / (2.0 * ga);
+  const double t = (zeta >= 0.0 ? 1.0 : -1.0) / (fabs(zeta) + sqrt(1.0 + zeta * zeta));
+  c = 1.0 / sqrt(1.0 + t * t);
+  s = c * t;
+  return true;
+}
+
+// 1e-100 < a < 1e100, by its exponent.
+static __device__ __forceinline__ bool mid_range(double a) {
+  return (unsigned)(__double2hiint(a) - 0x2b400000) < 0x54b00000u - 0x2b400000u;
+}
+
+// The same in the ordinary range; false (c = 1, s = 0) when
+// |ga| <= tol sqrt(al be).  With d = be - al and h = hypot(d, 2 ga),
+// c^2 = (1 + |d| / h) / 2 and |s| = |ga| / (h c): two reciprocal square roots
+// in all, then one step towards c^2 + s^2 = 1.
+static __device__ __forceinline__ bool jacobi_angle(double al, double be, double ga, double tol,
+                                                    double tol2, double& c, double& s) {
+  c = 1.0;
+  s = 0.0;
+  if (ga == 0.0) return false;
+  if (!mid_range(al) || !mid_range(be)) return jacobi_angle_wide(al, be, ga, tol, c, s);
+  const double g2 = ga * ga, d = be - al;
+  if (g2 <= tol2 * (al * be)) return false;
+  const double rh = rsqrt(fma(d, d, 4.0 * g2));
+  const double c2 = fma(0.5 * fabs(d), rh, 0.5);
+  const double ic = rsqrt(c2);
+  c = c2 * ic;
+  s = (d >= 0.0 ? ga : -ga) * rh * ic;
+  const double e = 0.5 * fma(-s, s, fma(-c, c, 1.0));
+  c = fma(c, e, c);
+  s = fma(s, e, s);
+  return true;
+}
+
+// Two column slots of a warp, x and y: four pairs, one per eight lanes.
+template <int RP>
+struct Pairs {
+  double x[RP], y[RP];
+  double nx, ny;  // their squared norms
+
+  __device__ __forceinline__ void norms() {
+    nx = group_sum<8>(lane_dot<RP>(x, x));
+    ny = group_sum<8>(lane_dot<RP>(y, y));
+  }
+
+  // x <- c x - s y, y <- s x + c y
+  __device__ __forceinline__ void rotate(double c, double s) {
+#pragma unroll
+    for (int r = 0; r < RP; ++r) {
+      const double a = x[r], b = y[r];
+      x[r] = c * a - s * b;
+      y[r] = s * a + c * b;
+    }
+  }
+
+  // The next pairing.  all: the circle method on the eight columns (the
+  // first x fixed, the others moved round one place: seven steps meet all 28
+  // pairs); else the y columns move round the groups (four steps meet the 16
+  // pairs across).  Either way the last step returns every column to its
+  // place.
+  __device__ __forceinline__ void next(bool all) {
+    const int lane = threadIdx.x & 31, g = lane >> 3;
+    if (all) {
+#pragma unroll
+      for (int r = 0; r < RP; ++r) {
+        const double up = __shfl_sync(0xffffffffu, g == 0 ? y[r] : x[r], (lane + 24) & 31);
+        const double down = __shfl_sync(0xffffffffu, y[r], (lane + 8) & 31);
+        y[r] = g == 3 ? x[r] : down;
+        if (g != 0) x[r] = up;
+      }
+    } else {
+#pragma unroll
+      for (int r = 0; r < RP; ++r) y[r] = __shfl_sync(0xffffffffu, y[r], (lane + 8) & 31);
+    }
+  }
+
+  __device__ __forceinline__ void next_norms(bool all) {
+    const int lane = threadIdx.x & 31, g = lane >> 3;
+    const double down = __shfl_sync(0xffffffffu, ny, (lane + 8) & 31);
+    if (all) {
+      const double up = __shfl_sync(0xffffffffu, g == 0 ? ny : nx, (lane + 24) & 31);
+      ny = g == 3 ? nx : down;
+      if (g != 0) nx = up;
+    } else {
+      ny = down;
+    }
+  }
+
+  // Columns ca + group and cb + group of the k x k matrix M (column step
+  // ld), zeros beyond it; and back.
+  __device__ __forceinline__ void load(const double* M, i64 ld, int k, int ca, int cb) {
+    const int g = (threadIdx.x & 31) >> 3;
+    const int a = ca + g, b = cb + g;
+    tile_load<8, RP>(M + a * ld, a < k ? k : 0, x);
+    tile_load<8, RP>(M + b * ld, b < k ? k : 0, y);
+  }
+  __device__ __forceinline__ void store(double* M, i64 ld, int k, int ca, int cb) const {
+    const int g = (threadIdx.x & 31) >> 3;
+    const int a = ca + g, b = cb + g;
+#pragma unroll
+    for (int r = 0; r < RP; ++r) {
+      const int i = tile_row<8>(r);
+      if (i >= k) continue;
+      if (a < k) M[i + a * ld] = x[r];
+      if (b < k) M[i + b * ld] = y[r];
+    }
+  }
+};
+
+// Hestenes' one-sided Jacobi on the columns of the k x k matrix B (column
+// step ld; see cta_jacobi, which it replaces up to k = 256) and, with VACC,
+// V (k x k, the same step) multiplied by the same rotations.  Columns go in
+// blocks of four; a warp loads a pair of blocks into registers, eight lanes
+// to a column, and rotates all their column pairs, four disjoint pairs at a
+// time: each pair belongs to eight lanes, which reduce its inner product in
+// three shuffle levels and compute its angle; squared norms are summed when
+// the blocks are loaded and follow the rotations until they are stored (a
+// sweep without rotations, which ends the iteration, has only summed ones).
+// Between steps the second columns move on to the next lanes.  Blocks meet in
+// round-robin order, one block barrier per meeting: a sweep of 64 columns has
+// 15 barriers and moves the matrices through shared memory 15 times, where
+// pairing single columns took 63.  What bounds a step is its chain (sums,
+// two reciprocal square roots, rotation: about 500 cycles) and, with V, the
+// issue of FP64 and shuffle instructions.  V rides along in registers up to
+// RP = 16 and is rotated afterwards beyond.
+template <int RP, bool VACC>
+static __device__ __noinline__ int jacobi_blocks(double* B, int k, i64 ld, double* V,
+                                                 int max_sweeps, double tol, int* flag) {
+  constexpr bool kRide = VACC && RP <= 16, kReplay = VACC && !kRide;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int nb = ((k + 7) >> 3) << 1, half = nb / 2;
+  const double tol2 = tol * tol;
+  for (int sweep = 0; sweep < max_sweeps; ++sweep) {
+    __syncthreads();
+    if (threadIdx.x == 0) *flag = 0;
+    __syncthreads();
+    bool rotated = false;
+    for (int round = 0; round < nb - 1; ++round) {
+      const bool all = round == 0;
+      const int steps = all ? 7 : 4;
+      for (int pr = warp; pr < half; pr += TTB_WARPS) {
+        const int pa = (pr == 0) ? 0 : ((pr - 1 + round) % (nb - 1)) + 1;
+        const int pb = ((nb - 2 - pr + round) % (nb - 1)) + 1;
+        const int ca = 4 * min(pa, pb), cb = 4 * max(pa, pb);
+        Pairs<RP> p;
+        Pairs<kRide ? RP : 2> q;
+        double cs[kReplay ? 7 : 1], sn[kReplay ? 7 : 1];
+        p.load(B, ld, k, ca, cb);
+        if constexpr (kRide) q.load(V, ld, k, ca, cb);
+        p.norms();
+        bool turned = false;
+#pragma unroll 1
+        for (int t = 0; t < steps; ++t) {
+          const double ga = group_sum<8>(lane_dot<RP>(p.x, p.y));
+          double c, s;
+          const bool rot = jacobi_angle(p.nx, p.ny, ga, tol, tol2, c, s);
+          if (__any_sync(0xffffffffu, rot)) {
+            turned = true;
+            const double tg = ga * s * __drcp_rn(c);
+            p.nx -= tg;
+            p.ny += tg;
+            p.rotate(c, s);
+            if constexpr (kRide) q.rotate(c, s);
+          }
+          if constexpr (kReplay) {
+            cs[t] = c;
+            sn[t] = s;
+          }
+          p.next(all);
+          p.next_norms(all);
+          if constexpr (kRide) q.next(all);
+        }
+        if (!turned) continue;
+        rotated = true;
+        p.store(B, ld, k, ca, cb);
+        if constexpr (kRide) q.store(V, ld, k, ca, cb);
+        if constexpr (kReplay) {
+          p.load(V, ld, k, ca, cb);
+#pragma unroll 1
+          for (int t = 0; t < steps; ++t) {
+            p.rotate(cs[t], sn[t]);
+            p.next(all);
+          }
+          p.store(V, ld, k, ca, cb);
+        }
+      }
+      __syncthreads();
+    }
+    if (rotated && lane == 0) *flag = 1;  // benign race: every writer stores 1
+    __syncthreads();
+    if (!*flag) return sweep + 1;
+  }
+  return -1;
+}
+
+// Orthonormal rows for the singular values that are exactly zero (their rows
+// of M are not defined by the iteration): each is the unit vector furthest
+// from the rows so far, orthogonalised against them twice.  Singular value
+// number order[r], the last ones the zeros, belongs to row order[r] of M
+// (``rows`` given) or row r.
+static __device__ __noinline__ void cta_complete_rows(int k, const double* sv, const int* rows,
+                                                      const int* order, Mat M, double* red) {
+  __shared__ int redi[TTB_WARPS];
+  const int* ord = rows ? rows : order;
+  auto row = [&](int r) { return rows ? rows[r] : r; };
+  for (int r = 0; r < k; ++r) {
+    if (sv[ord[r]] != 0.0) continue;
+    const int rr = row(r);
+    double best = -1.0;
+    int at = -1;
+    for (int i = threadIdx.x; i < k; i += TTB_THREADS) {
+      double s = 0.0;
+      for (int q = 0; q < r; ++q) s = fma(M(row(q), i), M(row(q), i), s);
+      const double left = fmax(2.0 - s, 0.0);
+      if (left > best) { best = left; at = i; }
+    }
+    at = max(block_argmax_abs(best, at, red, redi), 0);
+    for (int i = threadIdx.x; i < k; i += TTB_THREADS) M(rr, i) = i == at ? 1.0 : 0.0;
+    __syncthreads();
+    for (int pass = 0; pass < 2; ++pass)
+      for (int q = 0; q < r; ++q) {
+        double s = 0.0;
+        for (int i = threadIdx.x; i < k; i += TTB_THREADS) s = fma(M(row(q), i), M(rr, i), s);
+        s = block_sum(s, red);
+        for (int i = threadIdx.x; i < k; i += TTB_THREADS) M(rr, i) -= s * M(row(q), i);
+      }
+    double n2 = 0.0;
+    for (int i = threadIdx.x; i < k; i += TTB_THREADS) n2 = fma(M(rr, i), M(rr, i), n2);
+    const double inv = 1.0 / sqrt(block_sum(n2, red));
+    for (int i = threadIdx.x; i < k; i += TTB_THREADS) M(rr, i) *= inv;
+    __syncthreads();
+  }
+}
+
+// Largest k of the register-blocked Jacobi iteration, and of the pivoted
+// preconditioner in registers.
+constexpr int kJacobiMax = 256, kPivotMax = 128;
+
+template <bool VACC>
+static __device__ int cta_jacobi_blocks(double* B, int k, i64 ld, double* V, int max_sweeps,
+                                        double tol, int* flag) {
+  if (k <= 16) return jacobi_blocks<2, VACC>(B, k, ld, V, max_sweeps, tol, flag);
+  if (k <= 32) return jacobi_blocks<4, VACC>(B, k, ld, V, max_sweeps, tol, flag);
+  if (k <= 64) return jacobi_blocks<8, VACC>(B, k, ld, V, max_sweeps, tol, flag);
+  if (k <= 96) return jacobi_blocks<12, VACC>(B, k, ld, V, max_sweeps, tol, flag);
+  if (k <= 128) return jacobi_blocks<16, VACC>(B, k, ld, V, max_sweeps, tol, flag);
+  return jacobi_blocks<32, VACC>(B, k, ld, V, max_sweeps, tol, flag);
+}
+
+// M's upper triangle becomes its transpose in the lower one, the upper
+// zeros (k x k, column step ld); with ``to`` another matrix instead of M.
+static __device__ void cta_transpose_upper(const double* M, double* to, int k, i64 ld) {
+  for (int e = threadIdx.x; e < k * k; e += TTB_THREADS) {
+    const int i = e / k, j = e % k;  // i <= j is done by one thread for (j, i) too
+    if (i > j) continue;
+    const double v = M[i + j * ld];
+    to[j + i * ld] = v;
+    if (i != j) to[i + j * ld] = 0.0;
+  }
+  __syncthreads();
+}
+
+// Column norms of the k x k matrix B (column step ld) into sv and their
+// descending order; *flag tells whether one is zero.
+static __device__ void cta_sort_columns(const double* B, int k, i64 ld, double* sv, int* order,
+                                        int* flag) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int j = warp; j < k; j += TTB_WARPS) {
+    double s = 0.0;
+    for (int i = lane; i < k; i += 32) s = fma(B[i + j * ld], B[i + j * ld], s);
+    s = warp_sum(s);
+    if (lane == 0) {
+      sv[j] = sqrt(s);
+      order[j] = j;
+    }
+  }
+  if (threadIdx.x == 0) *flag = 0;
+  __syncthreads();
+  for (int j = threadIdx.x; j < k; j += TTB_THREADS) {
+    const double sj = sv[j];
+    int rank = 0;
+    for (int i = 0; i < k; ++i) {
+      const double si = sv[i];
+      rank += (si > sj) || (si == sj && i < j);
+    }
+    if (sj == sj) order[rank] = j;  // a NaN keeps the unsorted order
+    if (sj == 0.0) *flag = 1;       // benign race: every writer stores 1
+  }
+  __syncthreads();
+}
+
+// Column-pivoted QR of the upper-triangular k x k matrix in *F (column step
+// ld, zeros below), in place; ``other`` is a work area of the same size.
+// Beyond the registers the columns are sorted by norm once and factored
+// plainly: the factors are then in ``other``, and the two pointers change
+// places.
+static __device__ void cta_pivoted(double*& F, double*& other, int k, i64 ld, int* perm,
+                                   double* sv, double* tau2, double* red) {
+  if (k <= 32) {
+    hh_pivot<4, 1>(F, k, ld, perm, sv, tau2);
+  } else if (k <= 64) {
+    hh_pivot<8, 2>(F, k, ld, perm, sv, tau2);
+  } else if (k <= 96) {
+    hh_pivot<12, 3>(F, k, ld, perm, sv, tau2);
+  } else if (k <= kPivotMax) {
+    hh_pivot<16, 4>(F, k, ld, perm, sv, tau2);
+  } else {
+    for (int j = threadIdx.x; j < k; j += TTB_THREADS) {
+      double s = 0.0;
+      for (int i = 0; i <= j; ++i) s = fma(F[i + j * ld], F[i + j * ld], s);
+      sv[j] = s;
+      perm[j] = j;
+    }
+    __syncthreads();
+    for (int j = threadIdx.x; j < k; j += TTB_THREADS) {
+      int rank = 0;
+      for (int i = 0; i < k; ++i) rank += (sv[i] > sv[j]) || (sv[i] == sv[j] && i < j);
+      if (sv[j] == sv[j]) perm[rank] = j;
+    }
+    __syncthreads();
+    for (int e = threadIdx.x; e < k * k; e += TTB_THREADS)
+      other[e % k + (e / k) * ld] = F[e % k + perm[e / k] * ld];
+    __syncthreads();
+    if (k <= kHHRows)
+      cta_hh(other, ld, k, k, tau2);
+    else
+      cta_householder(other, k, k, ld, tau2, red);
+    double* t = F;
+    F = other;
+    other = t;
+  }
+}
+
+// X <- Q X for the k x k reflectors in F, X k x k (column step ld) or a view.
+static __device__ void cta_apply_square(const double* F, int k, i64 ld, const double* tau, Mat X,
+                                        int start) {
+  if (k <= kHHRows) {
+    cta_hh_apply(F, ld, k, k, tau, X, k, start);
+    return;
+  }
+  if (start == HH_IDENT)
+    for (int e = threadIdx.x; e < k * k; e += TTB_THREADS)
+      X(e % k, e / k) = e % k == e / k ? 1.0 : 0.0;
+  __syncthreads();
+  cta_apply_q(F, k, k, ld, tau, X, k);
+}
+
+// SVD of the upper-triangular k x k matrix R in Bsq (column major, column
+// step svd_step(k), zeros below the diagonal).  ``order`` has room for 2 k
+// ints (the second half keeps the pivot order), tau2 k doubles; S gets the
+// singular values, descending.
+//
+// Jacobi's sweeps depend on how near to orthogonal the columns start.  R's
+// own columns are far from it where the spectrum is steep, as it is in
+// rounding; those of L = R1^T, from the column-pivoted QR R P = Q2 R1, are
+// much nearer, and those of R2^T, from L = Q3 R2, nearer still (Drmac and
+// Veselic, "New fast and accurate Jacobi SVD algorithm", 2008): the 64-column
+// matrices of rounding a sum of rank-32 trains to 1e-6 take 15, 8 and 7
+// sweeps, a sampled field's 24, 9 and 7.  A 256 x 64 SVD took 4.3 ms with the
+// plain iteration and takes 0.69 ms, its left factor alone 0.63 and its right
+// one 0.47 ms.
+//
+// SQ_BOTH:  with L J = W S (J the rotations), R = (Q2 J) S (P W)^T: Vh is
+//           written and the left factor left in V (Us: scratch, the top of
+//           the caller's U).
+// SQ_LEFT:  with R2^T J = W S, R = (Q2 W) S (...): the left factor in V; no
+//           rotations are accumulated.
+// SQ_RIGHT: with L J = W S, the right factor (P W)^T is written to Vh.
+// On return V is where the left factor's column of singular value r is
+// V's column order[r].
+enum { SQ_BOTH = 0, SQ_LEFT = 1, SQ_RIGHT = 2 };
+static __device__ __noinline__ int cta_svd_square(int want, int k, double* Bsq, double*& V,
+                                                  double* sv, int* order, double* tau2, int* flag,
+                                                  Mat Us, double* S, Mat Vh, double* red) {
+  int* perm = order + k;
+  const double tol = 2.0 * sqrt((double)k) * 2.220446049250313e-16;
+  const i64 ld = svd_step(k);
+  double *F = Bsq, *X = V;
+  cta_pivoted(F, X, k, ld, perm, sv, tau2, red);
+  if (want == SQ_BOTH) {
+    cta_apply_square(F, k, ld, tau2, Us, HH_IDENT);  // Q2, explicit
+    cta_transpose_upper(F, F, k, ld);                // L takes the factors' place
+    for (int e = threadIdx.x; e < k * k; e += TTB_THREADS) X[e % k + (e / k) * ld] = Us(e % k, e / k);
+    __syncthreads();
+    double* t = F;  // F: the accumulated rotations, X: the iterated matrix
+    F = X;
+    X = t;
+  } else {
+    cta_transpose_upper(F, X, k, ld);
+    if (want == SQ_LEFT) {
+      // (sv is free until the columns are sorted: the second QR's scalars)
+      if (k <= kHHRows)
+        cta_hh(X, ld, k, k, sv);
+      else
+        cta_householder(X, k, k, ld, sv, red);
+      cta_transpose_upper(X, X, k, ld);
+    }
+  }
+  int status;
+  if (k > kJacobiMax) {
+    if (want != SQ_BOTH) {  // the rotations accumulated there go nowhere: F's are kept apart
+      status = cta_jacobi(X, k, ld, nullptr, 0, 60, tol, flag);
+    } else {
+      status = cta_jacobi(X, k, ld, F, ld, 60, tol, flag);
+    }
+  } else if (want == SQ_BOTH) {
+    status = cta_jacobi_blocks<true>(X, k, ld, F, 60, tol, flag);
+  } else {
+    status = cta_jacobi_blocks<false>(X, k, ld, nullptr, 60, tol, flag);
+  }
+  cta_sort_columns(X, k, ld, sv, order, flag);
+  for (int r = threadIdx.x; r < k; r += TTB_THREADS) S[r] = sv[order[r]];
+  if (want == SQ_LEFT) {
+    // W's columns in place, those of zero singular values completed
+    for (int e = threadIdx.x; e < k * k; e += TTB_THREADS) {
+      const int j = e / k, i = e % k;
+      if (sv[j] != 0.0) X[i + j * ld] /= sv[j];
+    }
+    __syncthreads();
+    if (*flag) cta_complete_rows(k, sv, order, order, Mat{X, ld, 1}, red);
+    cta_apply_square(F, k, ld, tau2, Mat{X, 1, ld}, HH_X);
+    V = X;
+    return status;
+  }
+  for (int e = threadIdx.x; e < k * k; e += TTB_THREADS) {
+    const int r = e / k, c = e % k, j = order[r];
+    Vh(r, perm[c]) = sv[j] == 0.0 ? 0.0 : X[c + j * ld] / sv[j];
+  }
+  __syncthreads();
+  if (*flag) cta_complete_rows(k, sv, nullptr, order, Vh, red);
+  V = F;
+  return status;
+}
+
+// The SVD of R by the plain iteration on R's own columns (R V = B): S and Vh
+// written, B's columns S times the left factor.
+static __device__ __noinline__ int cta_svd_plain(int k, double* B, double* V, double* sv,
+                                                 int* order, int* flag, double* S, Mat Vh) {
+  const i64 ld = svd_step(k);
+  const double tol = 4.0 * k * 2.220446049250313e-16;
+  for (int e = threadIdx.x; e < k * k; e += TTB_THREADS) {
+    const int i = e % k, j = e / k;
+    V[i + j * ld] = (i == j) ? 1.0 : 0.0;
+  }
+  const int status = cta_jacobi(B, k, ld, V, ld, 60, tol, flag);
+  for (int j = threadIdx.x; j < k; j += TTB_THREADS) {
+    double s = 0.0;
+    for (int i = 0; i < k; ++i) s = fma(B[i + j * ld], B[i + j * ld], s);
+    sv[j] = sqrt(s);
+    order[j] = j;
+  }
+  __syncthreads();
+  for (int j = threadIdx.x; j < k; j += TTB_THREADS) {
+    const double sj = sv[j];
+    int rank = 0;
+    for (int i = 0; i < k; ++i) {
+      const double si = sv[i];
+      rank += (si > sj) || (si == sj && i < j);
+    }
+    if (sj == sj) order[rank] = j;  // a NaN keeps the unsorted order
+  }
+  __syncthreads();
+  for (int r = threadIdx.x; r < k; r += TTB_THREADS) S[r] = sv[order[r]];
+  for (int e = threadIdx.x; e < k * k; e += TTB_THREADS) {
+    const int r = e % k, c = e / k;
+    Vh(r, c) = V[c + order[r] * ld];
+  }
+  __syncthreads();
+  return status;
+}
+
+// U <- [B(:, order) / S; 0] after cta_svd_plain.
+static __device__ void cta_top_u(int k, int m, const double* B, const double* sv,
+                                 const int* order, Mat U) {
+  const i64 ld = svd_step(k);
+  for (int e = threadIdx.x; e < m * k; e += TTB_THREADS) {
+    const int i = e % m, r = e / m, j = order[r];
+    double v = 0.0;
+    if (i < k) v = (sv[j] > 0.0) ? B[i + j * ld] / sv[j] : (i == r ? 1.0 : 0.0);
+    U(i, r) = v;
+  }
+  __syncthreads();
+}
+
+// Thin SVD of the m x k matrix A (any strides), m >= k required, as
+// A = U diag(S) Vh with S descending: Householder QR A = Q R, the SVD of R
+// (cta_svd_square), U = Q [U_R; 0].  A caller that needs one orthonormal
+// factor only (the other times S is its product with A) passes the other as
+// NULL and saves the accumulation of the rotations.  Work areas (shared or global): W (m x k,
+// column major, column step ldw), tau (k), Bsq and V (k columns of svd_step(k) each), sv (k),
+// order (2 k ints), flag (1 int), tau2 (k).  U (m x k), S (k) and Vh (k x k)
+// are strided outputs.  Returns the Jacobi sweeps used, or -1 if the sweep
+// cap was hit.
+__device__ __noinline__ int cta_svd_tall(CMat A, int m, int k, double* W, i64 ldw, double* tau,
+                                   double* Bsq, double* V, double* sv, int* order, int* flag,
+                                   double* tau2, Mat U, double* S, Mat Vh, double* red,
+                                   bool tiled) {
+  cta_load(A, W, ldw, m, k);
+  __syncthreads();
+  const bool tiles = tiled && m <= kHHRows;
+  if (tiles)
+    cta_hh(W, ldw, m, k, tau);
+  else
+    cta_householder(W, m, k, ldw, tau, red);
+  const i64 ld = svd_step(k);
+  for (int e = threadIdx.x; e < k * k; e += TTB_THREADS) {
+    int i = e % k, j = e / k;
+    Bsq[i + j * ld] = (i <= j) ? W[i + j * ldw] : 0.0;
+  }
+  __syncthreads();
+  const int want = !Vh.p ? SQ_LEFT : !U.p ? SQ_RIGHT : SQ_BOTH;
+  const int status =
+      tiled ? cta_svd_square(want, k, Bsq, V, sv, order, tau2, flag, U, S, Vh, red)
+            : cta_svd_plain(k, Bsq, V, sv, order, flag, S, Vh);
+  if (!U.p) return status;
+  if (!tiled) {
+    cta_top_u(k, m, Bsq, sv, order, U);
+    cta_apply_q(W, m, k, ldw, tau, U, k);
+    return status;
+  }
+  if (tiles) {
+    cta_hh_apply(W, ldw, m, k, tau, U, k, HH_TOP, V, k, ld, order);
+  } else {
+    for (int e = threadIdx.x; e < m * k; e += TTB_THREADS) {
+      int i = e % m, r = e / m;
+      U(i, r) = i < k ? V[i + order[r] * ld] : 0.0;
+    }
+    __syncthreads();
+    cta_apply_q(W, m, k, ldw, tau, U, k);
+  }
+  return status;
+}
+
+// Gaussian elimination with partial pivoting on [W | b] (LAPACK getrf/getrs
+// semantics: largest |pivot|, first index on ties), W column major with
+// leading dimension ld, then back substitution.  b is overwritten with the
+// solution and W with the factors.  Returns 0, or the 1-based index of the
+// first exactly-zero pivot (the solve then stops, like gesv's info > 0).
+__device__ __noinline__ int cta_gepp_solve(double* W, i64 ld, double* b, int n, double* redv, int* redi) {
+  for (int j = 0; j < n; ++j) {
+    double best = -1.0;
+    int bi = -1;
+    for (int i = j + threadIdx.x; i < n; i += TTB_THREADS) {
+      double a = fabs(W[i + j * ld]);
+      if (a > best) { best = a; bi = i; }
+    }
+    int piv = block_argmax_abs(best, bi, redv, redi);
+    if (piv != j) {
+      for (int c = j + threadIdx.x; c < n; c += TTB_THREADS) {
+        double t = W[j + c * ld];
+        W[j + c * ld] = W[piv + c * ld];
+        W[piv + c * ld] = t;
+      }
+      if (threadIdx.x == 0) {
+        double t = b[j];
+        b[j] = b[piv];
+        b[piv] = t;
+      }
+    }
+    __syncthreads();
+    const double d = W[j + j * ld];
+    if (d == 0.0) return j + 1;
+    const double rd = 1.0 / d;
+    for (int i = j + 1 + threadIdx.x; i < n; i += TTB_THREADS) W[i + j * ld] *= rd;
+    __syncthreads();
+    const int rows = n - j - 1;
+    const int total = rows * rows;
+    for (int e = threadIdx.x; e < total; e += TTB_THREADS) {
+      int i = j + 1 + e % rows, c = j + 1 + e / rows;
+      W[i + c * ld] = fma(-W[i + j * ld], W[j + c * ld], W[i + c * ld]);
+    }
+    const double bj = b[j];
+    for (int i = j + 1 + threadIdx.x; i < n; i += TTB_THREADS) b[i] = fma(-W[i + j * ld], bj, b[i]);
+    __syncthreads();
+  }
+  for (int j = n - 1; j >= 0; --j) {
+    if (threadIdx.x == 0) b[j] = b[j] / W[j + j * ld];
+    __syncthreads();
+    const double xj = b[j];
+    for (int i = threadIdx.x; i < j; i += TTB_THREADS) b[i] = fma(-W[i + j * ld], xj, b[i]);
+    __syncthreads();
+  }
+  return 0;
+}
+
+// ---------------------------------------------------------------------------
+// blocked factorisations for matrices that do not fit in shared memory
+// ---------------------------------------------------------------------------
+
+// Rows up to which the register tiles alone factor a matrix in global memory
+// (four columns a warp and step); taller ones take LNB-column panels with
+// the trailing updates as GEMMs.
+constexpr int kHHTall = 512;
+
+// A panel's reflectors: in registers, or row by row beyond their reach.
+static __device__ __forceinline__ void cta_hh_any(double* W, int m, int k, i64 ld, double* tau,
+                                                  double* red, bool tiled) {
+  if (tiled && m <= kHHRows)
+    cta_hh(W, ld, m, k, tau);
+  else
+    cta_householder(W, m, k, ld, tau, red);
+}
+
+
+// Blocked Gaussian elimination with partial pivoting on [W | b] (W column
+// major, leading dimension ld), panels of LNB columns factored in ``panel``
+// (rows x LNB doubles, shared or global memory), trailing updates as GEMMs.
+// Same pivot rule and result as cta_gepp_solve; b becomes the solution.
+__device__ __noinline__ int cta_gepp_blocked(double* W, i64 ld, double* b, int n, double* panel, double* redv,
+                                int* redi, int* ipiv, GemmSmem& gsm, double* ring) {
+  const int tid = threadIdx.x;
+  for (int j0 = 0; j0 < n; j0 += LNB) {
+    const int jb = min(LNB, n - j0);
+    const int rows = n - j0;
+    double* P = panel;
+    for (int e = tid; e < rows * jb; e += TTB_THREADS) {
+      int i = e % rows, c = e / rows;
+      P[i + (i64)c * rows] = W[(j0 + i) + (i64)(j0 + c) * ld];
+    }
+    __syncthreads();
+    for (int c = 0; c < jb; ++c) {
+      double best = -1.0;
+      int bi = -1;
+      for (int i = c + tid; i < rows; i += TTB_THREADS) {
+        double a = fabs(P[i + (i64)c * rows]);
+        if (a > best) { best = a; bi = i; }
+      }
+      const int piv = block_argmax_abs(best, bi, redv, redi);
+      if (tid == 0) ipiv[c] = piv;
+      if (piv != c) {
+        for (int cc = tid; cc < jb; cc += TTB_THREADS) {
+          double t = P[c + (i64)cc * rows];
+          P[c + (i64)cc * rows] = P[piv + (i64)cc * rows];
+          P[piv + (i64)cc * rows] = t;
+        }
+      }
+      __syncthreads();
+      const double d = P[c + (i64)c * rows];
+      if (d == 0.0) return j0 + c + 1;
+      const double rd = 1.0 / d;
+      for (int i = c + 1 + tid; i < rows; i += TTB_THREADS) P[i + (i64)c * rows] *= rd;
+      __syncthreads();
+      const int rr = rows - c - 1, cw = jb - c - 1;
+      for (int e = tid; e < rr * cw; e += TTB_THREADS) {
+        int i = c + 1 + e % rr, cc = c + 1 + e / rr;
+        P[i + (i64)cc * rows] = fma(-P[i + (i64)c * rows], P[c + (i64)cc * rows],
+                                    P[i + (i64)cc * rows]);
+      }
+      __syncthreads();
+    }
+    for (int e = tid; e < rows * jb; e += TTB_THREADS) {
+      int i = e % rows, c = e / rows;
+      W[(j0 + i) + (i64)(j0 + c) * ld] = P[i + (i64)c * rows];
+    }
+    // row swaps and the unit-lower solve on the columns right of the panel
+    // and on b; each thread owns whole columns, so no synchronisation
+    const int ncols = n - j0 - jb;
+    for (int col = tid; col <= ncols; col += TTB_THREADS) {
+      double* x = (col < ncols) ? W + (i64)(j0 + jb + col) * ld + j0 : b + j0;
+      for (int c = 0; c < jb; ++c) {
+        const int piv = ipiv[c];
+        if (piv != c) {
+          double t = x[c];
+          x[c] = x[piv];
+          x[piv] = t;
+        }
+      }
+      for (int r = 1; r < jb; ++r) {
+        double acc = x[r];
+        for (int q = 0; q < r; ++q) acc = fma(-P[r + (i64)q * rows], x[q], acc);
+        x[r] = acc;
+      }
+    }
+    __syncthreads();
+    if (rows > jb) {
+      // A22 -= L21 U12 ; b2 -= L21 u_b
+      if (ncols > 0)
+        gemm_sel(CMat{P + jb, 1, rows}, CMat{W + j0 + (i64)(j0 + jb) * ld, 1, ld},
+                 Mat{W + (j0 + jb) + (i64)(j0 + jb) * ld, 1, ld}, rows - jb, ncols, jb, -1.0,
+                 1.0, gsm, ring);
+      for (int i = tid; i < rows - jb; i += TTB_THREADS) {
+        double acc = b[j0 + jb + i];
+        for (int q = 0; q < jb; ++q) acc = fma(-P[jb + i + (i64)q * rows], b[j0 + q], acc);
+        b[j0 + jb + i] = acc;
+      }
+    }
+    __syncthreads();
+  }
+  for (int j = n - 1; j >= 0; --j) {
+    if (tid == 0) b[j] = b[j] / W[j + (i64)j * ld];
+    __syncthreads();
+    const double xj = b[j];
+    for (int i = tid; i < j; i += TTB_THREADS) b[i] = fma(-W[i + (i64)j * ld], xj, b[i]);
+    __syncthreads();
+  }
+  return 0;
+}
+
+// T factor (jb x jb, upper triangular, column major in Tm) of the block
+// reflector H_0 ... H_{jb-1} = I - V T V^T, V the rows x jb explicit
+// reflector block (unit diagonal, zeros above) in Wp with leading dim ldw
+// (LAPACK dlarft, forward column-wise).  G is jb x jb scratch.
+static __device__ void cta_block_t(const double* Wp, i64 ldw, int rows, int jb, const double* tau,
+                            double* G, double* Tm, GemmSmem& gsm, double* ring) {
+  gemm_sel(CMat{Wp, ldw, 1}, CMat{Wp, 1, ldw}, Mat{G, 1, LNB}, jb, jb, rows, 1.0, 0.0, gsm, ring);
+  const int tid = threadIdx.x;
+  for (int e = tid; e < LNB * LNB; e += TTB_THREADS) Tm[e] = 0.0;
+  __syncthreads();
+  for (int i = 0; i < jb; ++i) {  // column i, a thread per entry
+    if (tid < i) {
+      double acc = 0.0;
+      for (int r = tid; r < i; ++r) acc = fma(Tm[tid + r * LNB], G[r + i * LNB], acc);
+      Tm[tid + i * LNB] = -tau[i] * acc;
+    }
+    if (tid == i) Tm[i + i * LNB] = tau[i];
+    __syncthreads();
+  }
+}
+
+// X (m x nx, strided) <- H_0 ... H_{p-1} X for the block reflectors left in
+// W by cta_qr_blocked (explicit reflector blocks, leading dimension m),
+// applied last block first; only rows >= the block's first row change.
+// Columns of X left of a block are untouched (as for an identity start).
+static __device__ void cta_apply_q_blocked(const double* W, int m, int p, const double* tau, Mat X,
+                                    int nx, double* Y, double* G, double* Tm, GemmSmem& gsm, double* ring) {
+  const int tid = threadIdx.x;
+  const int last = ((p - 1) / LNB) * LNB;
+  for (int j0 = last; j0 >= 0; j0 -= LNB) {
+    const int jb = min(LNB, p - j0);
+    const int rows = m - j0;
+    const double* Wp = W + j0 + (i64)j0 * m;
+    cta_block_t(Wp, m, rows, jb, tau + j0, G, Tm, gsm, ring);
+    for (int c0 = 0; c0 < nx; c0 += YCH) {
+      const int nc = min(YCH, nx - c0);
+      Mat Xs{X.p + j0 * X.rs + c0 * X.cs, X.rs, X.cs};
+      gemm_sel(CMat{Wp, m, 1}, CMat{Xs.p, Xs.rs, Xs.cs}, Mat{Y, 1, LNB}, jb, nc, rows, 1.0, 0.0,
+               gsm, ring);
+      for (int col = tid; col < nc; col += TTB_THREADS) {
+        double y[LNB];
+        for (int i = 0; i < jb; ++i) y[i] = Y[i + (i64)col * LNB];
+        for (int i = 0; i < jb; ++i) {
+          double acc = 0.0;
+          for (int q = i; q < jb; ++q) acc = fma(Tm[i + q * LNB], y[q], acc);
+          Y[i + (i64)col * LNB] = acc;
+        }
+      }
+      __syncthreads();
+      gemm_sel(CMat{Wp, 1, m}, CMat{Y, 1, LNB}, Xs, rows, nc, jb, -1.0, 1.0, gsm, ring);
+    }
+  }
+}
+
+// Blocked (compact WY) economic QR of the m x k matrix A into the m x k
+// column-major work area W (global), panels of LNB columns: Householder on
+// the panel (cta_householder), the T factor, then the trailing update
+// C -= V (T^T (V^T C)) as two GEMMs through Y (LNB x k, shared).  Q (m x p)
+// and R (p x k) as in cta_qr; either may be NULL.  Same reflectors and R as
+// the unblocked factorisation up to rounding.
+__device__ __noinline__ void cta_qr_blocked(CMat A, int m, int k, double* W, double* tau, Mat Q, Mat R,
+                               double* Y, double* G, double* Tm, double* red, GemmSmem& gsm, double* ring,
+                               bool tiled) {
+  if (tiled && m <= kHHTall) {
+    cta_qr(A, m, k, W, m, tau, Q, R, red, true);
+    return;
+  }
+  const int p = m < k ? m : k;
+  const int tid = threadIdx.x;
+  cta_load(A, W, m, m, k);
+  __syncthreads();
+  for (int j0 = 0; j0 < p; j0 += LNB) {
+    const int jb = min(LNB, p - j0);
+    const int rows = m - j0;
+    double* Wp = W + j0 + (i64)j0 * m;
+    cta_hh_any(Wp, rows, jb, m, tau + j0, red, tiled);
+    // R's diagonal block, then the explicit reflector form in its place
+    for (int e = tid; e < jb * jb; e += TTB_THREADS) {
+      int r = e % jb, c = e / jb;
+      if (r <= c) {
+        if (R.p) R(j0 + r, j0 + c) = Wp[r + (i64)c * m];
+        Wp[r + (i64)c * m] = (r == c) ? 1.0 : 0.0;
+      }
+    }
+    __syncthreads();
+    const int nt = k - j0 - jb;
+    if (nt > 0) {
+      cta_block_t(Wp, m, rows, jb, tau + j0, G, Tm, gsm, ring);
+      for (int c0 = 0; c0 < nt; c0 += YCH) {
+        const int nc = min(YCH, nt - c0);
+        double* C = W + j0 + (i64)(j0 + jb + c0) * m;
+        // Y = V^T C (jb x nc), then Y = T^T Y, then C -= V Y
+        gemm_sel(CMat{Wp, m, 1}, CMat{C, 1, m}, Mat{Y, 1, LNB}, jb, nc, rows, 1.0, 0.0, gsm, ring);
+        for (int col = tid; col < nc; col += TTB_THREADS) {
+          double y[LNB];
+          for (int i = 0; i < jb; ++i) y[i] = Y[i + (i64)col * LNB];
+          for (int i = jb - 1; i >= 0; --i) {
+            double acc = 0.0;
+            for (int q = 0; q <= i; ++q) acc = fma(Tm[q + i * LNB], y[q], acc);
+            Y[i + (i64)col * LNB] = acc;
+          }
+        }
+        __syncthreads();
+        gemm_sel(CMat{Wp, 1, m}, CMat{Y, 1, LNB}, Mat{C, 1, m}, rows, nc, jb, -1.0, 1.0, gsm, ring);
+      }
+    }
+  }
+  if (R.p) {
+    for (int e = tid; e < p * k; e += TTB_THREADS) {
+      int i = e % p, j = e / p;
+      int jp = (i / LNB) * LNB;  // panel of row i
+      bool in_diag_block = (j >= jp && j < jp + LNB && j < p);
+      if (i > j) R(i, j) = 0.0;
+      else if (!in_diag_block) R(i, j) = W[i + (i64)j * m];
+    }
+  }
+  if (Q.p) {
+    for (int e = tid; e < m * p; e += TTB_THREADS) {
+      int i = e % m, j = e / m;
+      Q(i, j) = (i == j) ? 1.0 : 0.0;
+    }
+    __syncthreads();
+    cta_apply_q_blocked(W, m, p, tau, Q, p, Y, G, Tm, gsm, ring);
+  }
+  __syncthreads();
+}
+
+// R factor only of the economic QR of the m x k view A, two-level blocked
+// for tall operands: outer panels of LNB2 columns are factorised by the
+// LNB-blocked Householder code (trailing updates inside the panel only),
+// then the panel's LNB2 reflectors update the rest of the matrix as one
+// compact-WY block, C -= V (T^T (V^T C)), whose products have 64-wide tiles
+// and long K.  Same reflectors as cta_qr_blocked.  W (m x k column major)
+// and tau (min(m, k)) are global work; ``pool`` (shared) holds
+// 2 LNB2^2 + LNB2^2 + LNB * LNB2 + 2 LNB^2 doubles.
+__device__ __noinline__ void cta_qr_r_blocked2(CMat A, int m, int k, double* W, double* tau,
+                                                      Mat R, double* pool, double* red,
+                                                      double* ring) {
+  const int p = m < k ? m : k;
+  const int tid = threadIdx.x;
+  double* G2 = pool;                      // LNB2 x LNB2: V^T V, later T^T Y
+  double* T2 = G2 + LNB2 * LNB2;          // LNB2 x LNB2 upper triangular
+  double* Yo = T2 + LNB2 * LNB2;          // LNB2 x LNB2 chunk of V^T C
+  double* Yi = Yo + LNB2 * LNB2;          // LNB x LNB2 (inner updates)
+  double* Gi = Yi + LNB * LNB2;
+  double* Ti = Gi + LNB * LNB;
+  cta_load(A, W, m, m, k);
+  __syncthreads();
+  for (int o0 = 0; o0 < p; o0 += LNB2) {
+    const int ob = min(LNB2, p - o0);
+    const int orows = m - o0;
+    double* Wo = W + o0 + (i64)o0 * m;
+    // inner LNB-blocked factorisation of the panel's ob columns
+    for (int j0 = o0; j0 < o0 + ob; j0 += LNB) {
+      const int jb = min(LNB, o0 + ob - j0);
+      const int rows = m - j0;
+      double* Wp = W + j0 + (i64)j0 * m;
+      cta_householder(Wp, rows, jb, m, tau + j0, red);
+      for (int e = tid; e < jb * jb; e += TTB_THREADS) {
+        int r = e % jb, c = e / jb;
+        if (r <= c) {
+          R(j0 + r, j0 + c) = Wp[r + (i64)c * m];
+          Wp[r + (i64)c * m] = (r == c) ? 1.0 : 0.0;
+        }
+      }
+      __syncthreads();
+      const int nt = o0 + ob - j0 - jb;
+      if (nt > 0) {
+        // T of the block (as cta_block_t), column by column over the block
+        cta_gemm_pipe(CMat{Wp, m, 1}, CMat{Wp, 1, m}, Mat{Gi, 1, LNB}, jb, jb, rows, 1.0, 0.0,
+                      ring);
+        for (int e = tid; e < LNB * LNB; e += TTB_THREADS) Ti[e] = 0.0;
+        __syncthreads();
+        for (int i = 0; i < jb; ++i) {
+          if (tid < i) {
+            double acc = 0.0;
+            for (int r = tid; r < i; ++r) acc = fma(Ti[tid + r * LNB], Gi[r + i * LNB], acc);
+            Ti[tid + i * LNB] = -tau[j0 + i] * acc;
+          }
+          if (tid == 0) Ti[i + i * LNB] = tau[j0 + i];
+          __syncthreads();
+        }
+        double* C = W + j0 + (i64)(j0 + jb) * m;
+        cta_gemm_pipe(CMat{Wp, m, 1}, CMat{C, 1, m}, Mat{Yi, 1, LNB}, jb, nt, rows, 1.0, 0.0,
+                      ring);
+        for (int col = tid; col < nt; col += TTB_THREADS) {
+          double y[LNB];
+          for (int i = 0; i < jb; ++i) y[i] = Yi[i + (i64)col * LNB];
+          for (int i = jb - 1; i >= 0; --i) {
+            double acc = 0.0;
+            for (int q = 0; q <= i; ++q) acc = fma(Ti[q + i * LNB], y[q], acc);
+            Yi[i + (i64)col * LNB] = acc;
+          }
+        }
+        __syncthreads();
+        cta_gemm_pipe(CMat{Wp, 1, m}, CMat{Yi, 1, LNB}, Mat{C, 1, m}, rows, nt, jb, -1.0, 1.0,
+                      ring);
+      }
+    }
+    // R entries above the inner diagonal blocks move out; V gets zeros there
+    for (int e = tid; e < ob * ob; e += TTB_THREADS) {
+      int r = e % ob, c = e / ob;
+      if (r < c && (r / LNB) != (c / LNB)) {
+        R(o0 + r, o0 + c) = Wo[r + (i64)c * m];
+        Wo[r + (i64)c * m] = 0.0;
+      }
+    }
+    __syncthreads();
+    const int nt = k - o0 - ob;
+    if (nt <= 0) continue;
+    // T of the panel: T[i, i] = tau_i, T[0:i, i] = -tau_i T[0:i, 0:i] (V^T V)[0:i, i]
+    cta_gemm_pipe(CMat{Wo, m, 1}, CMat{Wo, 1, m}, Mat{G2, 1, LNB2}, ob, ob, orows, 1.0, 0.0, ring);
+    for (int e = tid; e < LNB2 * LNB2; e += TTB_THREADS) T2[e] = 0.0;
+    __syncthreads();
+    for (int i = 0; i < ob; ++i) {
+      const double ti = tau[o0 + i];
+      for (int q = tid; q < i; q += TTB_THREADS) {
+        double acc = 0.0;
+        for (int r = q; r < i; ++r) acc = fma(T2[q + r * LNB2], G2[r + i * LNB2], acc);
+        T2[q + i * LNB2] = -ti * acc;
+      }
+      if (tid == 0) T2[i + i * LNB2] = ti;
+      __syncthreads();
+    }
+    for (int c0 = 0; c0 < nt; c0 += LNB2) {
+      const int nc = min(LNB2, nt - c0);
+      double* C = W + o0 + (i64)(o0 + ob + c0) * m;
+      // Yo = V^T C, G2 = T^T Yo, C -= V G2
+      cta_gemm_pipe(CMat{Wo, m, 1}, CMat{C, 1, m}, Mat{Yo, 1, LNB2}, ob, nc, orows, 1.0, 0.0, ring);
+      cta_gemm_pipe(CMat{T2, LNB2, 1}, CMat{Yo, 1, LNB2}, Mat{G2, 1, LNB2}, ob, nc, ob, 1.0, 0.0,
+                    ring);
+      cta_gemm_pipe(CMat{Wo, 1, m}, CMat{G2, 1, LNB2}, Mat{C, 1, m}, orows, nc, ob, -1.0, 1.0,
+                    ring);
+    }
+  }
+  // the rest of R: below the diagonal zero, right of each outer panel from W
+  for (int e = tid; e < p * k; e += TTB_THREADS) {
+    int i = e % p, j = e / p;
+    if (i > j) {
+      R(i, j) = 0.0;
+    } else if (j >= min((i / LNB2) * LNB2 + LNB2, p)) {
+      R(i, j) = W[i + (i64)j * m];
+    }
+  }
+  __syncthreads();
+}
+
+// cta_svd_tall for matrices that do not fit in shared memory: blocked QR
+// into the global work area W, the SVD of R in Bsq/V (global or shared), U
+// by the reflectors.  Y needs LNB * max(k, 1) doubles, G and Tm LNB * LNB
+// each (shared).
+__device__ __noinline__ int cta_svd_tall_blocked(CMat A, int m, int k, double* W, double* tau,
+                                           double* Bsq, double* V, double* sv, int* order,
+                                           int* flag, double* tau2, Mat U, double* S, Mat Vh,
+                                           double* Y, double* G, double* Tm, double* red,
+                                           GemmSmem& gsm, double* ring, bool tiled) {
+  const i64 ld = svd_step(k);
+  cta_qr_blocked(A, m, k, W, tau, Mat{nullptr, 0, 0}, Mat{Bsq, 1, ld}, Y, G, Tm, red, gsm, ring,
+                 tiled);
+  __syncthreads();
+  const int want = !Vh.p ? SQ_LEFT : !U.p ? SQ_RIGHT : SQ_BOTH;
+  const int status =
+      tiled ? cta_svd_square(want, k, Bsq, V, sv, order, tau2, flag, U, S, Vh, red)
+            : cta_svd_plain(k, Bsq, V, sv, order, flag, S, Vh);
+  if (!U.p) return status;
+  if (!tiled) {
+    cta_top_u(k, m, Bsq, sv, order, U);
+    cta_apply_q_blocked(W, m, k, tau, U, k, Y, G, Tm, gsm, ring);
+    return status;
+  }
+  if (m <= kHHTall) {
+    cta_hh_apply(W, m, m, k, tau, U, k, HH_TOP, V, k, ld, order);
+    return status;
+  }
+  for (int e = threadIdx.x; e < m * k; e += TTB_THREADS) {
+    int i = e % m, r = e / m;
+    U(i, r) = i < k ? V[i + order[r] * ld] : 0.0;
+  }
+  __syncthreads();
+  cta_apply_q_blocked(W, m, k, tau, U, k, Y, G, Tm, gsm, ring);
+  return status;
+}
+
+}  // namespace ttb

@@ -35,7 +35,7 @@ constexpr int kMaxDevices = 64;
 int smem_limit_once(const void* func, int bytes, int* done);
 }
 
-namespace {
+namespace ttb_tensor {
 
 typedef long long i64;
 
@@ -283,7 +283,8 @@ __global__ void __launch_bounds__(THREADS, 1) k_gemm_3xtf32(const __grid_constan
   }
 }
 
-}  // namespace
+}  // namespace ttb_tensor
+using namespace ttb_tensor;
 
 extern "C" {
 

@@ -365,17 +365,21 @@ def qr(a: torch.Tensor, want_q=True, want_r=True, q_out=None, r_out=None):
     return q, r
 
 
-def svd(a: torch.Tensor, status: Optional[torch.Tensor] = None):
-    """Thin SVD of a 2-D (strided) view: (U (m, p), S (p,), Vh (p, k))."""
+def svd(a: torch.Tensor, status: Optional[torch.Tensor] = None, want_u=True, want_vh=True):
+    """Thin SVD of a 2-D (strided) view: (U (m, p), S (p,), Vh (p, k)).  One
+    of the factors may be left out (None), which is about twice as fast; the
+    other times S is then its product with ``a``."""
     m, k = a.shape
     p = min(m, k)
-    u, s, vh = empty(m, p), empty(p), empty(p, k)
+    s = empty(p)
+    u = empty(m, p) if want_u else None
+    vh = empty(p, k) if want_vh else None
     L = lib()
     ar = arena()
     with ar.scope():
         work = ar.take(L.ttb_svd_work_doubles(m, k))
-        d = _lib.SVD(ptr(a), a.stride(0), a.stride(1), ptr(u), u.stride(0), u.stride(1), ptr(s),
-                     ptr(vh), vh.stride(0), vh.stride(1), ptr(work), ptr(status), m, k)
+        d = _lib.SVD(ptr(a), a.stride(0), a.stride(1), ptr(u), p, 1, ptr(s), ptr(vh), k, 1,
+                     ptr(work), ptr(status), m, k)
         arr = (_lib.SVD * 1)(d)
         check(L.ttb_svd(arr, 1, stream()), "ttb_svd")
     return u, s, vh

@@ -481,7 +481,7 @@ class TensorTrain:
         out: List[torch.Tensor] = []
 
         def split(matrix: torch.Tensor, lb: int):
-            u, sv, _ = K.svd(matrix)
+            u, sv, _ = K.svd(matrix, want_vh=False)
             nb = _svd_rank(sv, delta, max_rank)
             piece = K.empty(matrix.shape[0], nb)
             K.copy_(piece, u[:, :nb])
@@ -785,12 +785,12 @@ def left_svd_sweep(cores: List[torch.Tensor], error: float, max_rank=None) -> No
     delta = error / math.sqrt(len(cores) - 1) * float(nrm.item())
     for i in range(len(cores) - 1):
         s = cores[i].shape
-        u, sv, vh = K.svd(cores[i].reshape(s[0] * s[1] * s[2], s[3]))
+        matrix = cores[i].reshape(s[0] * s[1] * s[2], s[3])
+        u, sv, _ = K.svd(matrix, want_vh=False)
         nb = _svd_rank(sv, delta, max_rank)
         core = K.empty(s[0], s[1], s[2], nb)
         K.copy_(core.view(-1, nb), u[:, :nb])
-        carry = K.empty(nb, s[3])
-        K.copy_(carry, vh[:nb], scale=sv, scale_axis=0)
+        carry = K.matmul(core.view(-1, nb).t(), matrix)  # S Vh
         cores[i] = core
         cores[i + 1] = _apply_left(carry, cores[i + 1])
 
@@ -803,12 +803,11 @@ def right_svd_sweep(cores: List[torch.Tensor], error: float, max_rank=None) -> N
     delta = error / math.sqrt(len(cores) - 1) * float(nrm.item())
     for i in range(len(cores) - 1, 0, -1):
         s = cores[i].shape
-        u, sv, vh = K.svd(cores[i].reshape(s[0], s[1] * s[2] * s[3]))
+        matrix = cores[i].reshape(s[0], s[1] * s[2] * s[3])
+        _, sv, vh = K.svd(matrix, want_u=False)
         nb = _svd_rank(sv, delta, max_rank)
-        core = K.empty(nb, s[1], s[2], s[3])
-        K.copy_(core.view(nb, -1), vh[:nb])
-        carry = K.empty(s[0], nb)
-        K.copy_(carry, u[:, :nb], scale=sv, scale_axis=1)
+        core = vh[:nb].view(nb, s[1], s[2], s[3])
+        carry = K.matmul(matrix, vh[:nb].t())  # U S
         cores[i] = core
         cores[i - 1] = _apply_right(cores[i - 1], carry)
 
@@ -861,7 +860,7 @@ def tt_svd(tensor, error: float = 1e-12, max_rank: Optional[int] = None,
     for i in range(len(phys) - 1):
         rows = bond * phys[i][0] * phys[i][1]
         matrix = cur.view(rows, -1)
-        u, sv, _ = K.svd(matrix)
+        u, sv, _ = K.svd(matrix, want_vh=False)
         nb = _svd_rank(sv, delta, max_rank)
         core = K.empty(rows, nb)
         K.copy_(core, u[:, :nb])
