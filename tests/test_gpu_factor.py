@@ -25,7 +25,7 @@ def K():
 
 
 def dev(a):
-    return torch.from_numpy(np.array(a, dtype=np.float64)).cuda()
+    return torch.from_numpy(np.ascontiguousarray(a, dtype=np.float64)).cuda()
 
 
 def orth(q):
@@ -75,3 +75,30 @@ def test_svd_one_factor(K, m, k, deficient):
         assert orth(factor) < 1e-12
     assert np.linalg.norm(ul @ (ul.T @ a) - a) < 1e-12 * scale
     assert np.linalg.norm((a @ vr.T) @ vr - a) < 1e-12 * scale
+
+
+@pytest.mark.parametrize("n", [2, 32, 33, 65, 97, 129, 160, 161, 177, 257, 530, 1024, 1025])
+def test_lu_tile_edges(K, n):
+    """Whole systems in registers up to 160 unknowns, 16-column panels with
+    128-column strips beyond, row by row past 1024: against LAPACK, with rows
+    that need swapping and exact ties in the pivot search."""
+    rng = np.random.default_rng(n)
+    a = rng.integers(-2, 3, (n, n)).astype(float) + n * 0.1 * np.eye(n)[rng.permutation(n)]
+    b = rng.standard_normal(n)
+    x = dev(b)
+    info = torch.zeros(1, dtype=torch.int32, device="cuda")
+    K.lu_solve_(dev(a.T), x, info)
+    assert info.item() == 0
+    want = np.linalg.solve(a, b)
+    bound = 1e-13 * max(1.0, np.linalg.cond(a))
+    assert np.linalg.norm(x.cpu().numpy() - want) < bound * np.linalg.norm(want)
+
+
+@pytest.mark.parametrize("n,at", [(40, 40), (150, 7), (300, 1), (300, 290), (600, 333)])
+def test_lu_zero_pivot(K, n, at):
+    """The first exactly-zero pivot is reported by its 1-based index."""
+    a = np.triu(np.ones((n, n)))
+    a[at - 1, at - 1] = 0.0
+    info = torch.zeros(1, dtype=torch.int32, device="cuda")
+    K.lu_solve_(dev(a.T), dev(np.ones(n)), info)
+    assert info.item() == at

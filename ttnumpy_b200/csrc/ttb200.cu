@@ -413,7 +413,7 @@ __global__ void __launch_bounds__(TTB_THREADS) k_svd(const __grid_constant__ SBa
 constexpr int kMaxL = 24;
 struct LBatch {
   int count;
-  int mode[kMaxL];  // 0: all in shared memory, 1: blocked, panel shared, 2: blocked, panel global
+  int mode[kMaxL];  // 0: all in registers, 1: blocked, panel shared, 2: blocked, panel global
   ttb_lu_t d[kMaxL];
 };
 
@@ -428,19 +428,8 @@ __global__ void __launch_bounds__(TTB_THREADS) k_lu(const __grid_constant__ LBat
   if (n <= 0) return;
   const int mode = lb.mode[blockIdx.x];
   int info;
-  if (mode == 0) {
-    double* W = dsm;
-    double* b = dsm + (i64)n * n;
-    for (i64 e = threadIdx.x; e < (i64)n * n; e += TTB_THREADS) {
-      i64 i = e % n, j = e / n;
-      W[e] = q.a[i + j * q.lda];
-    }
-    for (int i = threadIdx.x; i < n; i += TTB_THREADS) b[i] = q.b[i];
-    __syncthreads();
-    info = cta_gepp_solve(W, n, b, n, redv, redi);
-    __syncthreads();
-    if (info == 0)
-      for (int i = threadIdx.x; i < n; i += TTB_THREADS) q.b[i] = b[i];
+  if (mode == 0) {  // the whole system in registers
+    info = cta_gepp_solve(q.a, q.lda, q.b, n, dsm);
   } else {
     double* panel = mode == 1 ? dsm : q.work;
     info = cta_gepp_blocked(q.a, q.lda, q.b, n, panel, redv, redi, ipiv, gsm);
@@ -1627,10 +1616,10 @@ int ttb_lu_solve(const ttb_lu_t* ps, int count, void* stream) {
     for (int j = 0; j < lb.count; ++j) {
       lb.d[j] = ps[i0 + j];
       const i64 n = lb.d[j].n;
-      const i64 whole = (n * n + n) * 8, panel = n * LNB * 8;
-      if (whole <= kSmemCap) {
+      const i64 panel = lu_panel_doubles((int)n) * 8;
+      if (n <= kLuWhole) {
         lb.mode[j] = 0;
-        smem = std::max(smem, whole);
+        smem = std::max<i64>(smem, lu_buf_doubles((int)n) * 8);
       } else if (panel <= kSmemCap) {
         lb.mode[j] = 1;
         smem = std::max(smem, panel);

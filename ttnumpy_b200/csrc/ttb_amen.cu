@@ -36,6 +36,9 @@ constexpr i64 kPoolD = kPoolBytes / 8;
 // blocked factorisations' reflector chunk
 static_assert(kPoolD >= 3 * LNB2 * LNB2 + LNB * LNB2 + 2 * LNB * LNB, "pool too small");
 static_assert(kPoolD >= (i64)LNB * YCH + 2 * LNB * LNB, "pool too small");
+// direct solves held in the pool fit the registers, their multipliers the ring
+static_assert(kPoolD < (kLuWhole + 1) * (kLuWhole + 2), "pool beyond lu_whole");
+static_assert(lu_buf_doubles(kLuWhole) <= GSTAGES * GSTAGE_D, "ring too small");
 // ring + pool + the kernel's static shared memory (about 9 KB) within 227 KB
 static_assert(kRingBytes + kPoolBytes <= 216 * 1024, "dynamic shared memory over budget");
 constexpr int kMaxRestarts = 4;        // common.py:230
@@ -916,9 +919,8 @@ __device__ __noinline__ void project(Ctx& c, const double* left, int a, int i, c
 // Economic QR of the m x k view A: Q (m x p) and R (p x k) strided outputs.
 __device__ __noinline__ void qr(Ctx& c, CMat A, int m, int k, Mat Q, Mat R) {
   const int p = min(m, k);
-  const int ldw = odd_step(m);
-  if ((i64)ldw * k + p <= kPoolD) {
-    cta_qr(A, m, k, c.pool, ldw, c.pool + (i64)ldw * k, Q, R, c.sm->red, false);
+  if ((i64)m * k + p <= kPoolD) {
+    cta_qr(A, m, k, c.pool, m, c.pool + (i64)m * k, Q, R, c.sm->red, false);
     return;
   }
   const i64 mark = c.top;
@@ -963,8 +965,7 @@ __device__ __noinline__ void svd(Ctx& c, CMat A, int m, int k, Mat U, double* S,
   CMat At = tall ? A : CMat{A.p, A.cs, A.rs};
   Mat Ut = tall ? U : Mat{Vh.p, Vh.cs, Vh.rs};
   Mat Vt = tall ? Vh : Mat{U.p, U.cs, U.rs};
-  const int ldw = odd_step(M);
-  const i64 need = (i64)ldw * K + 2 * (i64)svd_step(K) * K + 4 * (i64)K + 6;
+  const i64 need = (i64)M * K + 2 * (i64)K * K + 3 * (i64)K + 2;
   const i64 mark = c.top;
   double* base;
   const bool in_pool = need <= kPoolD;
@@ -975,21 +976,20 @@ __device__ __noinline__ void svd(Ctx& c, CMat A, int m, int k, Mat U, double* S,
     if (c.status) return;
   }
   double* W = base;
-  double* tau = W + (i64)ldw * K;
-  double* Bsq = align2(tau + K);
-  double* V = Bsq + (i64)svd_step(K) * K;
-  double* sv = V + (i64)svd_step(K) * K;
+  double* tau = W + (i64)M * K;
+  double* Bsq = tau + K;
+  double* V = Bsq + (i64)K * K;
+  double* sv = V + (i64)K * K;
   int* order = reinterpret_cast<int*>(sv + K);
-  double* tau2 = sv + 2 * K;
-  int* flag = reinterpret_cast<int*>(sv + 3 * K);
+  int* flag = reinterpret_cast<int*>(sv + 2 * K);
   if (in_pool) {
-    cta_svd_tall(At, M, K, W, ldw, tau, Bsq, V, sv, order, flag, tau2, Ut, S, Vt, c.sm->red,
+    cta_svd_tall(At, M, K, W, M, tau, Bsq, V, sv, order, flag, nullptr, Ut, S, Vt, c.sm->red,
                  false);
   } else {
     double* Y = c.pool;
     double* G = Y + (i64)LNB * YCH;
     double* Tm = G + LNB * LNB;
-    cta_svd_tall_blocked(At, M, K, W, tau, Bsq, V, sv, order, flag, tau2, Ut, S, Vt, Y, G, Tm,
+    cta_svd_tall_blocked(At, M, K, W, tau, Bsq, V, sv, order, flag, nullptr, Ut, S, Vt, Y, G, Tm,
                          c.sm->red, *c.gsm, c.ring, false);
   }
   c.top = mark;
@@ -1006,54 +1006,60 @@ __device__ __noinline__ void direct_solve(Ctx& c, const LocalOp& L, const double
   Sm* s = c.sm;
   double* W;
   double* panel = c.pool;  // the blocked elimination's panel (N x LNB)
-  const bool small = N * N + N <= kPoolD;
+  const bool small = N * N + N <= kPoolD;  // in the pool and in registers
   if (small) {
     W = c.pool;
   } else {
     W = take(c, N * N);
-    if (N * LNB > kPoolD) panel = take(c, N * LNB);  // beyond the pool: in the slab
+    if (lu_panel_doubles((int)N) > kPoolD) panel = take(c, N * LNB);  // in the slab
     if (c.status) return;
   }
-  // explicit local matrix, column major: each thread owns rows (j, kr, nf)
-  // and walks the columns (i, l, mt) in order (no divisions per element)
+  // Explicit local matrix, column major.  An item is a row (j, kr, nf) and the
+  // part (l, mt) of a column: the operator core times the right environment
+  // gives one number per left operator bond, kept in registers while the
+  // item's lt columns (i, l, mt) are formed.  Consecutive threads take
+  // consecutive rows.  (A thread walking a whole row re-read core and
+  // environment for every entry and left the threads past N idle: as long as
+  // the elimination itself on the QTT systems.)
   const int Nn = (int)N;
-  for (int row = threadIdx.x; row < Nn; row += TTB_THREADS) {
+  constexpr int kRegs = 8;  // left operator bonds held in registers at a time
+  const int items = Nn * L.m * L.rt;
+  for (int e = threadIdx.x; e < items; e += TTB_THREADS) {
+    const int row = e % Nn, q = e / Nn, mt = q % L.rt, l = q / L.rt;
     const int nf = row % L.rf, kr = (row / L.rf) % L.n, j = row / (L.rf * L.n);
-    int mt = 0, l = 0, i = 0;
-    for (int col = 0; col < Nn; ++col) {
-      double acc = 0.0;
-      for (int a = 0; a < L.R; ++a) {
-        const double la = L.left[(i * L.R + a) * L.lf + j];
-        if (la == 0.0) continue;
-        const double* op = L.op + ((a * L.n + kr) * L.m + l) * L.R2;
-        double t = 0.0;
-        for (int bb = 0; bb < L.R2; ++bb) t = fma(op[bb], L.right[(mt * L.R2 + bb) * L.rf + nf], t);
-        acc = fma(la, t, acc);
+    for (int a0 = 0; a0 < L.R; a0 += kRegs) {
+      double t[kRegs];
+#pragma unroll
+      for (int a = 0; a < kRegs; ++a) {
+        t[a] = 0.0;
+        if (a0 + a >= L.R) continue;
+        const double* op = L.op + (((i64)(a0 + a) * L.n + kr) * L.m + l) * L.R2;
+        const double* right = L.right + (i64)mt * L.R2 * L.rf + nf;
+        for (int bb = 0; bb < L.R2; ++bb) t[a] = fma(op[bb], right[(i64)bb * L.rf], t[a]);
       }
-      W[row + (i64)col * Nn] = acc;
-      if (++mt == L.rt) {
-        mt = 0;
-        if (++l == L.m) {
-          l = 0;
-          ++i;
+      const double* left = L.left + (i64)a0 * L.lf + j;
+      double* w = W + row + ((i64)l * L.rt + mt) * Nn;
+      for (int i = 0; i < L.lt; ++i) {
+        double acc = a0 ? *w : 0.0;
+#pragma unroll
+        for (int a = 0; a < kRegs; ++a) {
+          if (a0 + a >= L.R) continue;
+          const double la = left[(i64)a * L.lf];
+          if (la != 0.0) acc = fma(la, t[a], acc);
         }
+        *w = acc;
+        left += (i64)L.R * L.lf;
+        w += (i64)L.m * L.rt * Nn;
       }
     }
   }
   vcopy(u, b, N);
   __syncthreads();
   int info;
-  if (small) {
-    // b goes to the pool too so the whole solve stays on chip
-    double* bb = c.pool + N * N;
-    vcopy(bb, u, N);
-    __syncthreads();
-    info = cta_gepp_solve(W, N, bb, (int)N, s->red, s->redi);
-    __syncthreads();
-    if (info == 0) vcopy(u, bb, N);
-  } else {
+  if (small)
+    info = cta_gepp_solve(W, N, u, (int)N, c.ring);
+  else
     info = cta_gepp_blocked(W, N, u, (int)N, panel, s->red, s->redi, s->ipiv, *c.gsm, c.ring);
-  }
   __syncthreads();
   if (info != 0) c.status = ST_SINGULAR;
   c.top = mark;
@@ -2534,7 +2540,7 @@ long long ttb_amen_slab_doubles(int d, const int* dims, int kickrank, int rmax,
   const long long iter = N + std::max(6 * N, (kRestart + 3) * (N + 32) + 2048) + apply;
   const long long rank = 4 * N + 2LL * kRankChunk * R * n * r + R * r * r + r * r + apply;
   const long long fact = r * n * r + r + r * n * r        // U S Vh
-                         + (r * n) * r + 2 * r * (r + 16) + 6 * r + 6  // svd work
+                         + (r * n) * r + 2 * r * r + 4 * r  // svd work
                          + (r * n) * cols + 2 * cols * n * r + r * r  // enriched, padded, svh
                          + r * n * cols + cols * cols + cols * n * r  // Q, R, next
                          + r * n * cols + cols + r * n * K;            // qr work, block

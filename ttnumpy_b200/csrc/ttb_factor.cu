@@ -273,6 +273,35 @@ static __device__ __forceinline__ double hh_make(double (&x)[RP], int j) {
   return tau;
 }
 
+// Producer and consumers of a step: the warp that makes the next step's
+// reflector or pivot arrives when it is in shared memory and goes on with its
+// own updates; the others wait there.  Two barriers take turns (a warp cannot
+// be a step ahead without all having passed the one before).
+static __device__ __forceinline__ void step_arrive(int j) {
+  asm volatile("bar.arrive %0, %1;" ::"r"(1 + (j & 1)), "n"(TTB_THREADS) : "memory");
+}
+static __device__ __forceinline__ void step_wait(int j) {
+  asm volatile("bar.sync %0, %1;" ::"r"(1 + (j & 1)), "n"(TTB_THREADS) : "memory");
+}
+
+// x[at] for a warp-uniform ``at``, by halves (an indexed register array would
+// go to local memory).
+template <int N, int RP>
+static __device__ __forceinline__ double pick_reg(const double (&x)[RP], int at, int base = 0) {
+  if constexpr (N == 1) {
+    return base < RP ? x[base < RP ? base : 0] : 0.0;
+  } else {
+    const double lo = pick_reg<N / 2, RP>(x, at, base);
+    const double hi = pick_reg<N / 2, RP>(x, at, base + N / 2);
+    return (at & (N / 2)) ? hi : lo;
+  }
+}
+__host__ __device__ constexpr int ceil_pow2(int n) {
+  int p = 1;
+  while (p < n) p *= 2;
+  return p;
+}
+
 // dst = x[at] for a warp-uniform ``at``: a chain of moves the compiler does
 // not turn into an indexed array (which would put x in local memory).
 template <int RP, int SL>
@@ -1142,7 +1171,7 @@ static __device__ __noinline__ int cta_svd_square(int want, int k, double* Bsq, 
 // written, B's columns S times the left factor.
 static __device__ __noinline__ int cta_svd_plain(int k, double* B, double* V, double* sv,
                                                  int* order, int* flag, double* S, Mat Vh) {
-  const i64 ld = svd_step(k);
+  const i64 ld = k;
   const double tol = 4.0 * k * 2.220446049250313e-16;
   for (int e = threadIdx.x; e < k * k; e += TTB_THREADS) {
     const int i = e % k, j = e / k;
@@ -1178,7 +1207,7 @@ static __device__ __noinline__ int cta_svd_plain(int k, double* B, double* V, do
 // U <- [B(:, order) / S; 0] after cta_svd_plain.
 static __device__ void cta_top_u(int k, int m, const double* B, const double* sv,
                                  const int* order, Mat U) {
-  const i64 ld = svd_step(k);
+  const i64 ld = k;
   for (int e = threadIdx.x; e < m * k; e += TTB_THREADS) {
     const int i = e % m, r = e / m, j = order[r];
     double v = 0.0;
@@ -1193,7 +1222,8 @@ static __device__ void cta_top_u(int k, int m, const double* B, const double* sv
 // (cta_svd_square), U = Q [U_R; 0].  A caller that needs one orthonormal
 // factor only (the other times S is its product with A) passes the other as
 // NULL and saves the accumulation of the rotations.  Work areas (shared or global): W (m x k,
-// column major, column step ldw), tau (k), Bsq and V (k columns of svd_step(k) each), sv (k),
+// column major, column step ldw), tau (k), Bsq and V (k columns of svd_step(k) each, 16-byte
+// aligned, or k x k when not tiled), sv (k),
 // order (2 k ints), flag (1 int), tau2 (k).  U (m x k), S (k) and Vh (k x k)
 // are strided outputs.  Returns the Jacobi sweeps used, or -1 if the sweep
 // cap was hit.
@@ -1208,7 +1238,7 @@ __device__ __noinline__ int cta_svd_tall(CMat A, int m, int k, double* W, i64 ld
     cta_hh(W, ldw, m, k, tau);
   else
     cta_householder(W, m, k, ldw, tau, red);
-  const i64 ld = svd_step(k);
+  const i64 ld = tiled ? svd_step(k) : k;
   for (int e = threadIdx.x; e < k * k; e += TTB_THREADS) {
     int i = e % k, j = e / k;
     Bsq[i + j * ld] = (i <= j) ? W[i + j * ldw] : 0.0;
@@ -1237,55 +1267,413 @@ __device__ __noinline__ int cta_svd_tall(CMat A, int m, int k, double* W, i64 ld
   return status;
 }
 
+// ---------------------------------------------------------------------------
+// register-tiled Gaussian elimination
+// ---------------------------------------------------------------------------
+
+// Steps 0 .. steps - 1 of Gaussian elimination with partial pivoting on a
+// panel of rows x cols held in registers, warp w the columns w, w +
+// TTB_WARPS, ..., lane l the rows l, l + 32, ....  Rows stay where they are:
+// ``pos`` follows the position each would have had if the rows were swapped
+// (the pivot of a step is the largest remaining entry, the one of lowest
+// position on ties, as cta_gepp_solve takes it), and a row that has been
+// pivot keeps its values.  Each step's multipliers go through ``lbuf`` (2 x
+// 32 RPL doubles, shared; zeros in the finished rows), its pivot row through
+// ``piv`` (2 ints, shared); ipiv[j], if given, gets the position swapped with
+// j.  Every entry sees the updates of cta_gepp_solve in the same order: the
+// same bits.  Returns 0 or the 1-based step whose pivot is exactly zero.
+// The warp of the next pivot column takes it first and publishes it before
+// its other updates, so that a step costs the chain of one column: a search,
+// a reciprocal, a barrier; updating in memory took four barriers.
+template <int RPL, int CPW>
+static __device__ __forceinline__ int lu_steps(double (&x)[CPW][RPL], int (&pos)[RPL], int rows,
+                                               int steps, double* lbuf, int* piv, int* ipiv) {
+  constexpr int PW = ceil_pow2(RPL);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+  for (int r = 0; r < RPL; ++r) pos[r] = lane + 32 * r;
+  __syncthreads();  // every warp has its columns, and lbuf and piv are free
+  for (int j = -1; j < steps; ++j) {
+    double l[RPL];
+    int slot = 0, from = 0;
+    if (j >= 0) {
+      if (warp != j % TTB_WARPS) step_wait(j);
+      const int pr = piv[j & 1];
+      if (pr < 0) return j + 1;
+      const double* lb = lbuf + (j & 1) * 32 * RPL;
+#pragma unroll
+      for (int r = 0; r < RPL; ++r) l[r] = lb[lane + 32 * r];
+      slot = pr >> 5;
+      from = pr & 31;
+      // the pivot row takes position j, the row that was there the pivot's
+      int pp = pos[0];
+#pragma unroll
+      for (int r = 1; r < RPL; ++r) pp = r == slot ? pos[r] : pp;
+      pp = __shfl_sync(0xffffffffu, pp, from);
+#pragma unroll
+      for (int r = 0; r < RPL; ++r) {
+        if (lane + 32 * r == pr) pos[r] = j;
+        else if (pos[r] == j) pos[r] = pp;
+      }
+      if (ipiv && threadIdx.x == 0) ipiv[j] = pp;
+    } else {
+#pragma unroll
+      for (int r = 0; r < RPL; ++r) l[r] = 0.0;
+    }
+    const int n = j + 1;  // the next pivot column
+    int mine = -1;
+    if (n < steps && warp == n % TTB_WARPS) {  // this warp's, and done first
+      mine = n / TTB_WARPS;
+      double col[RPL];
+      pick_slot<RPL, CPW>(x, mine, col);
+      if (j >= 0) {
+        const double u = __shfl_sync(0xffffffffu, pick_reg<PW, RPL>(col, slot), from);
+#pragma unroll
+        for (int r = 0; r < RPL; ++r) col[r] = fma(-l[r], u, col[r]);
+      }
+      // the largest entry, the lowest position on ties (a NaN is never
+      // larger): its high word, its low word, then position and row
+      double best = -1.0;
+      unsigned at = 0x7fffffffu;
+#pragma unroll
+      for (int r = 0; r < RPL; ++r) {
+        const int row = lane + 32 * r;
+        const double a = fabs(col[r]);
+        const unsigned id = ((unsigned)pos[r] << 16) | row;
+        const bool in = row < rows && pos[r] >= n;
+        if (in && (a > best || (!(a < best) && id < at))) {
+          best = a;
+          at = id;
+        }
+      }
+      const unsigned hi = at == 0x7fffffffu ? 0u : (unsigned)__double2hiint(best);
+      const unsigned top = __reduce_max_sync(0xffffffffu, hi);
+      const unsigned lo = hi == top ? (unsigned)__double2loint(best) : 0u;
+      const unsigned low = __reduce_max_sync(0xffffffffu, lo);
+      at = __reduce_min_sync(0xffffffffu, hi == top && lo == low ? at : 0x7fffffffu);
+      const int pr = (int)(at & 0xffff);
+      const double d = __shfl_sync(0xffffffffu, pick_reg<PW, RPL>(col, pr >> 5), pr & 31);
+      if (lane == 0) piv[n & 1] = d == 0.0 ? -1 : pr;
+      const double rd = 1.0 / d;
+      double* lb = lbuf + (n & 1) * 32 * RPL;
+#pragma unroll
+      for (int r = 0; r < RPL; ++r) {
+        const int row = lane + 32 * r;
+        const bool below = pos[r] >= n && row != pr;
+        const double q = col[r] * rd;
+        lb[row] = below ? q : 0.0;
+        col[r] = below ? q : col[r];
+      }
+      __syncwarp();
+      step_arrive(n);
+#pragma unroll
+      for (int s = 0; s < CPW; ++s)
+        if (s == mine) {
+#pragma unroll
+          for (int r = 0; r < RPL; ++r)
+            asm volatile("mov.f64 %0, %1;" : "=d"(x[s][r]) : "d"(col[r]));
+        }
+    }
+    if (j < 0) continue;
+#pragma unroll
+    for (int s = 0; s < CPW; ++s) {
+      if (warp + TTB_WARPS * s <= j || s == mine) continue;
+      const double u = __shfl_sync(0xffffffffu, pick_reg<PW, RPL>(x[s], slot), from);
+#pragma unroll
+      for (int r = 0; r < RPL; ++r) x[s][r] = fma(-l[r], u, x[s][r]);
+    }
+  }
+  return 0;
+}
+
+// Solves U x = b for the upper triangle of W (column step ld), x over b, by
+// blocks of 32 columns: one warp the diagonal block, every thread the rows
+// above it.  Each row sees the columns last to first, one fma each, as a
+// column-by-column substitution takes them.
+static __device__ __noinline__ void cta_back_substitute(const double* W, i64 ld, double* b,
+                                                        int n) {
+  const int lane = threadIdx.x & 31;
+  for (int j0 = ((n - 1) / 32) * 32; j0 >= 0; j0 -= 32) {
+    const int jn = min(32, n - j0);
+    if (threadIdx.x < 32) {
+      double x = lane < jn ? b[j0 + lane] : 0.0;
+      const double diag = lane < jn ? W[(j0 + lane) + (j0 + lane) * ld] : 1.0;
+      for (int j = jn - 1; j >= 0; --j) {
+        const double w = lane < j ? W[(j0 + lane) + (j0 + j) * ld] : 0.0;
+        if (lane == j) x = x / diag;
+        const double xj = __shfl_sync(0xffffffffu, x, j);
+        if (lane < j) x = fma(-w, xj, x);
+      }
+      if (lane < jn) b[j0 + lane] = x;
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < j0; i += TTB_THREADS) {
+      double acc = b[i];
+      const double* row = W + i + j0 * ld;
+#pragma unroll 8
+      for (int j = jn - 1; j >= 0; --j) acc = fma(-row[j * ld], b[j0 + j], acc);
+      b[i] = acc;
+    }
+    __syncthreads();
+  }
+}
+
+// The whole matrix and b in registers: n <= 32 RPL, n + 1 <= TTB_WARPS CPW.
+template <int RPL, int CPW>
+static __device__ __noinline__ int lu_whole(double* W, i64 ld, double* b, int n, double* lbuf,
+                                            int* piv) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  double x[CPW][RPL];
+  int pos[RPL];
+#pragma unroll
+  for (int s = 0; s < CPW; ++s) {
+    const int c = warp + TTB_WARPS * s;
+#pragma unroll
+    for (int r = 0; r < RPL; ++r) {
+      const int i = lane + 32 * r;
+      x[s][r] = (c <= n && i < n) ? (c < n ? W[i + c * ld] : b[i]) : 0.0;
+    }
+  }
+  const int info = lu_steps<RPL, CPW>(x, pos, n, n, lbuf, piv, nullptr);
+  if (info) return info;
+#pragma unroll
+  for (int s = 0; s < CPW; ++s) {
+    const int c = warp + TTB_WARPS * s;
+#pragma unroll
+    for (int r = 0; r < RPL; ++r) {
+      const int i = lane + 32 * r;
+      if (c > n || i >= n) continue;
+      if (c < n) W[pos[r] + c * ld] = x[s][r];
+      else b[pos[r]] = x[s][r];
+    }
+  }
+  __syncthreads();
+  cta_back_substitute(W, ld, b, n);
+  return 0;
+}
+
 // Gaussian elimination with partial pivoting on [W | b] (LAPACK getrf/getrs
 // semantics: largest |pivot|, first index on ties), W column major with
 // leading dimension ld, then back substitution.  b is overwritten with the
-// solution and W with the factors.  Returns 0, or the 1-based index of the
-// first exactly-zero pivot (the solve then stops, like gesv's info > 0).
-__device__ __noinline__ int cta_gepp_solve(double* W, i64 ld, double* b, int n, double* redv, int* redi) {
-  for (int j = 0; j < n; ++j) {
-    double best = -1.0;
-    int bi = -1;
-    for (int i = j + threadIdx.x; i < n; i += TTB_THREADS) {
-      double a = fabs(W[i + j * ld]);
-      if (a > best) { best = a; bi = i; }
+// solution and W with the factors.  ``lbuf`` (shared) holds
+// lu_buf_doubles(n).  Returns 0, or the 1-based index of the first exactly-zero pivot
+// (the solve then stops, like gesv's info > 0).  Bound by the chain of a
+// step (a pivot search, a reciprocal, one barrier): 128 unknowns took 522 us
+// with the matrix updated in shared memory and take 193 us.
+__device__ __noinline__ int cta_gepp_solve(double* W, i64 ld, double* b, int n, double* lbuf) {
+  __shared__ int piv[2];
+  int info;
+  if (n <= 32) info = lu_whole<1, 5>(W, ld, b, n, lbuf, piv);
+  else if (n <= 64) info = lu_whole<2, 9>(W, ld, b, n, lbuf, piv);
+  else if (n <= 96) info = lu_whole<3, 13>(W, ld, b, n, lbuf, piv);
+  else if (n <= 128) info = lu_whole<4, 17>(W, ld, b, n, lbuf, piv);
+  else info = lu_whole<5, 21>(W, ld, b, n, lbuf, piv);
+  __syncthreads();
+  return info;
+}
+
+// One LNB-column panel of the blocked elimination: columns j0 .. of W's rows
+// j0 .., factored in registers, written back in pivoted order and, transposed
+// for the products, to P (pitch ``pp``): P[c * pp + i] is row i of column c.
+template <int RPL>
+static __device__ __noinline__ int lu_panel(double* W, i64 ld, int rows, int jb, double* P,
+                                            int pp, double* lbuf, int* piv, int* ipiv) {
+  constexpr int CPW = 2;
+  static_assert(TTB_WARPS * CPW == LNB, "a panel fills the warps' columns");
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  double x[CPW][RPL];
+  int pos[RPL];
+#pragma unroll
+  for (int s = 0; s < CPW; ++s) {
+    const int c = warp + TTB_WARPS * s;
+#pragma unroll
+    for (int r = 0; r < RPL; ++r) {
+      const int i = lane + 32 * r;
+      x[s][r] = (c < jb && i < rows) ? W[i + c * ld] : 0.0;
     }
-    int piv = block_argmax_abs(best, bi, redv, redi);
-    if (piv != j) {
-      for (int c = j + threadIdx.x; c < n; c += TTB_THREADS) {
-        double t = W[j + c * ld];
-        W[j + c * ld] = W[piv + c * ld];
-        W[piv + c * ld] = t;
-      }
-      if (threadIdx.x == 0) {
-        double t = b[j];
-        b[j] = b[piv];
-        b[piv] = t;
-      }
-    }
-    __syncthreads();
-    const double d = W[j + j * ld];
-    if (d == 0.0) return j + 1;
-    const double rd = 1.0 / d;
-    for (int i = j + 1 + threadIdx.x; i < n; i += TTB_THREADS) W[i + j * ld] *= rd;
-    __syncthreads();
-    const int rows = n - j - 1;
-    const int total = rows * rows;
-    for (int e = threadIdx.x; e < total; e += TTB_THREADS) {
-      int i = j + 1 + e % rows, c = j + 1 + e / rows;
-      W[i + c * ld] = fma(-W[i + j * ld], W[j + c * ld], W[i + c * ld]);
-    }
-    const double bj = b[j];
-    for (int i = j + 1 + threadIdx.x; i < n; i += TTB_THREADS) b[i] = fma(-W[i + j * ld], bj, b[i]);
-    __syncthreads();
   }
-  for (int j = n - 1; j >= 0; --j) {
-    if (threadIdx.x == 0) b[j] = b[j] / W[j + j * ld];
-    __syncthreads();
-    const double xj = b[j];
-    for (int i = threadIdx.x; i < j; i += TTB_THREADS) b[i] = fma(-W[i + j * ld], xj, b[i]);
-    __syncthreads();
+  const int info = lu_steps<RPL, CPW>(x, pos, rows, jb, lbuf, piv, ipiv);
+  if (info) return info;
+  __syncthreads();  // lbuf may share P's memory
+#pragma unroll
+  for (int s = 0; s < CPW; ++s) {
+    const int c = warp + TTB_WARPS * s;
+#pragma unroll
+    for (int r = 0; r < RPL; ++r) {
+      const int i = lane + 32 * r;
+      if (c >= jb || i >= rows) continue;
+      W[pos[r] + c * ld] = x[s][r];
+      P[c * pp + pos[r]] = x[s][r];
+    }
   }
+  __syncthreads();
+  return 0;
+}
+
+// cta_gepp_solve for a matrix in global memory, kLuWhole < n <= kLuRows,
+// panels of LNB columns; ``pool`` (shared) holds lu_panel_doubles(n).  Per
+// panel: the panel in registers (lu_panel); then the trailing columns, a
+// strip at a time: row swaps as one permutation of the at most 32 rows they
+// touch, the unit-lower solve with a thread per column, both into shared
+// memory, and C -= L21 U12 on the FP64 tensor path with C loaded straight
+// into the accumulator fragments' lanes, 32 x 16 entries a warp.  Every entry
+// sees the products and roundings of the plain blocked form (cta_gepp_blocked)
+// in the same order.  The floor on one SM is 2 n^3 / 3 flops at 128 a cycle
+// (2.1 ms for 928 unknowns); 928 unknowns took 27.4 ms with one synchronised
+// tile at a time and take 10.7 ms, half of it waiting for C.
+static __device__ __noinline__ int cta_gepp_strips(double* W, i64 ld, double* b, int n,
+                                                   double* pool) {
+  __shared__ int piv[2], ipiv[LNB], nmove, src[2 * LNB], dst[2 * LNB];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int g = lane >> 2, t = lane & 3;
+  double* lbuf = pool;                      // the panel's multipliers ...
+  double* P = pool;                         // ... then the panel, row pitch pp
+  double* Us = pool + LNB * lu_pitch(n);    // U12's strip, LNB x kLuStripPitch
+  for (int j0 = 0; j0 < n; j0 += LNB) {
+    const int jb = min(LNB, n - j0), rows = n - j0, pp = lu_pitch(rows);
+    double* Wp = W + j0 + j0 * ld;
+    int info;
+    if (rows <= 128) info = lu_panel<4>(Wp, ld, rows, jb, P, pp, lbuf, piv, ipiv);
+    else if (rows <= 256) info = lu_panel<8>(Wp, ld, rows, jb, P, pp, lbuf, piv, ipiv);
+    else if (rows <= 512) info = lu_panel<16>(Wp, ld, rows, jb, P, pp, lbuf, piv, ipiv);
+    else info = lu_panel<32>(Wp, ld, rows, jb, P, pp, lbuf, piv, ipiv);
+    if (info) return j0 + info;
+    // the swaps as moves: position dst[e] gets the row that was at src[e]
+    if (tid == 0) {
+      int cnt = 0;
+      for (int c = 0; c < jb; ++c) {
+        const int q = ipiv[c];
+        int ec = -1, eq = -1;
+        for (int e = 0; e < cnt; ++e) {
+          if (dst[e] == c) ec = e;
+          if (dst[e] == q) eq = e;
+        }
+        if (ec < 0) { ec = cnt++; dst[ec] = src[ec] = c; }
+        if (q == c) continue;
+        if (eq < 0) { eq = cnt++; dst[eq] = src[eq] = q; }
+        const int v = src[ec];
+        src[ec] = src[eq];
+        src[eq] = v;
+      }
+      nmove = cnt;
+    }
+    // zero rows below the panel, so that the products need no row test
+    for (int e = tid; e < LNB * (pp - rows); e += TTB_THREADS) {
+      const int c = e / (pp - rows), i = rows + e % (pp - rows);
+      P[c * pp + i] = 0.0;
+    }
+    if (jb < LNB)
+      for (int e = tid; e < (LNB - jb) * pp; e += TTB_THREADS) P[jb * pp + e] = 0.0;
+    __syncthreads();
+    const int cnt = nmove;
+    const int ncols = n - j0 - jb;  // trailing columns; b comes after them
+    for (int s0 = 0; s0 <= ncols; s0 += kLuStrip) {
+      const int sn = min(kLuStrip, ncols + 1 - s0);
+      // swaps: four columns of a warp in flight
+      for (int c4 = 4 * warp; c4 < sn; c4 += 4 * TTB_WARPS) {
+        double v[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const int c = s0 + c4 + u;
+          const double* col = c < ncols ? Wp + (jb + c) * ld : b + j0;
+          v[u] = (c4 + u < sn && lane < cnt) ? col[src[lane]] : 0.0;
+        }
+        __syncwarp();
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const int c = s0 + c4 + u;
+          double* col = c < ncols ? Wp + (jb + c) * ld : b + j0;
+          if (c4 + u >= sn || lane >= cnt) continue;
+          const int to = dst[lane];
+          if (to < jb) Us[to * kLuStripPitch + c4 + u] = v[u];
+          else col[to] = v[u];
+        }
+      }
+      if (jb < LNB)
+        for (int e = tid; e < (LNB - jb) * sn; e += TTB_THREADS)
+          Us[(jb + e / sn) * kLuStripPitch + e % sn] = 0.0;
+      __syncthreads();
+      // the unit-lower solve, a thread per column
+      for (int c = tid; c < sn; c += TTB_THREADS) {
+        double y[LNB];
+#pragma unroll
+        for (int r = 0; r < LNB; ++r) {
+          y[r] = Us[r * kLuStripPitch + c];
+          double acc = y[r];
+#pragma unroll
+          for (int q = 0; q < r; ++q) acc = fma(-P[q * pp + r], y[q], acc);
+          y[r] = r < jb ? acc : 0.0;
+          Us[r * kLuStripPitch + c] = y[r];
+        }
+      }
+      __syncthreads();
+      for (int e = tid; e < sn * LNB; e += TTB_THREADS) {
+        const int r = e % LNB, c = e / LNB;
+        double* col = s0 + c < ncols ? Wp + (jb + s0 + c) * ld : b + j0;
+        if (r < jb) col[r] = Us[r * kLuStripPitch + c];
+      }
+      // C -= L21 U12, b2 -= L21 u_b
+      const int below = rows - jb, wide = min(sn, ncols - s0);
+      const int tm = (below + 31) / 32, tn = (wide + 15) / 16;
+      if (below > 0 && wide > 0) {
+        for (int tile = warp; tile < tm * tn; tile += TTB_WARPS) {
+          const int m0 = jb + (tile % tm) * 32, n0 = (tile / tm) * 16;
+          double c0[4][2][2], acc[4][2][2];
+          double* cp[2][2];
+#pragma unroll
+          for (int j = 0; j < 2; ++j)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+              const int cc = n0 + 8 * j + 2 * t + h;
+              cp[j][h] = cc < wide ? Wp + (jb + s0 + cc) * ld : nullptr;
+#pragma unroll
+              for (int i = 0; i < 4; ++i) {
+                const int r = m0 + 8 * i + g;
+                acc[i][j][h] = 0.0;
+                c0[i][j][h] = (cp[j][h] && r < rows) ? cp[j][h][r] : 0.0;
+              }
+            }
+#pragma unroll
+          for (int kk = 0; kk < LNB; kk += 4) {
+            if (kk >= jb) break;
+            double av[4], bv[2];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              const int r = m0 + 8 * i + g;
+              av[i] = r < pp ? P[(kk + t) * pp + r] : 0.0;
+            }
+#pragma unroll
+            for (int j = 0; j < 2; ++j) bv[j] = Us[(kk + t) * kLuStripPitch + n0 + 8 * j + g];
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+              for (int j = 0; j < 2; ++j) dmma_8x8x4(acc[i][j][0], acc[i][j][1], av[i], bv[j]);
+          }
+#pragma unroll
+          for (int j = 0; j < 2; ++j)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+              if (!cp[j][h]) continue;
+#pragma unroll
+              for (int i = 0; i < 4; ++i) {
+                const int r = m0 + 8 * i + g;
+                if (r < rows) cp[j][h][r] = fma(1.0, c0[i][j][h], -1.0 * acc[i][j][h]);
+              }
+            }
+        }
+      }
+      if (s0 + sn > ncols) {  // this strip holds b, in its last column
+        for (int i = tid; i < below; i += TTB_THREADS) {
+          double acc = b[j0 + jb + i];
+          for (int q = 0; q < jb; ++q)
+            acc = fma(-P[q * pp + jb + i], Us[q * kLuStripPitch + sn - 1], acc);
+          b[j0 + jb + i] = acc;
+        }
+      }
+      __syncthreads();  // the strip's reads are done
+    }
+  }
+  cta_back_substitute(W, ld, b, n);
   return 0;
 }
 
@@ -1314,6 +1702,7 @@ static __device__ __forceinline__ void cta_hh_any(double* W, int m, int k, i64 l
 // Same pivot rule and result as cta_gepp_solve; b becomes the solution.
 __device__ __noinline__ int cta_gepp_blocked(double* W, i64 ld, double* b, int n, double* panel, double* redv,
                                 int* redi, int* ipiv, GemmSmem& gsm, double* ring) {
+  if (n <= kLuRows && __isShared(panel)) return cta_gepp_strips(W, ld, b, n, panel);
   const int tid = threadIdx.x;
   for (int j0 = 0; j0 < n; j0 += LNB) {
     const int jb = min(LNB, n - j0);
@@ -1392,13 +1781,7 @@ __device__ __noinline__ int cta_gepp_blocked(double* W, i64 ld, double* b, int n
     }
     __syncthreads();
   }
-  for (int j = n - 1; j >= 0; --j) {
-    if (tid == 0) b[j] = b[j] / W[j + (i64)j * ld];
-    __syncthreads();
-    const double xj = b[j];
-    for (int i = tid; i < j; i += TTB_THREADS) b[i] = fma(-W[i + (i64)j * ld], xj, b[i]);
-    __syncthreads();
-  }
+  cta_back_substitute(W, ld, b, n);
   return 0;
 }
 
@@ -1658,7 +2041,7 @@ __device__ __noinline__ int cta_svd_tall_blocked(CMat A, int m, int k, double* W
                                            int* flag, double* tau2, Mat U, double* S, Mat Vh,
                                            double* Y, double* G, double* Tm, double* red,
                                            GemmSmem& gsm, double* ring, bool tiled) {
-  const i64 ld = svd_step(k);
+  const i64 ld = tiled ? svd_step(k) : k;
   cta_qr_blocked(A, m, k, W, tau, Mat{nullptr, 0, 0}, Mat{Bsq, 1, ld}, Y, G, Tm, red, gsm, ring,
                  tiled);
   __syncthreads();

@@ -33,8 +33,21 @@ __device__ int cta_svd_tall_blocked(CMat A, int m, int k, double* W, double* tau
                                     Mat U, double* S, Mat Vh, double* Y, double* G, double* Tm,
                                     double* red, GemmSmem& gsm, double* ring = nullptr,
                                     bool tiled = true);
-__device__ int cta_gepp_solve(double* W, i64 ld, double* b, int n, double* redv, int* redi);
+__device__ int cta_gepp_solve(double* W, i64 ld, double* b, int n, double* lbuf);
 __device__ int cta_gepp_blocked(double* W, i64 ld, double* b, int n, double* panel, double* redv,
                                 int* redi, int* ipiv, GemmSmem& gsm, double* ring = nullptr);
+
+// Largest system cta_gepp_solve takes, and the doubles of its ``lbuf``.
+constexpr int kLuWhole = 160;
+__host__ __device__ constexpr int lu_buf_doubles(int n) { return 2 * ((n + 31) & ~31); }
+
+// Doubles of the shared ``panel`` that cta_gepp_blocked needs for n unknowns
+// (n <= kLuRows; beyond, LNB columns of n rows, in any memory): the panel at
+// a pitch that spreads a fragment over the banks, and a strip of U12.
+constexpr int kLuRows = 1024, kLuStrip = 128, kLuStripPitch = kLuStrip + 4;
+__host__ __device__ constexpr int lu_pitch(int rows) { return ((rows + 15) & ~15) + 4; }
+__host__ __device__ constexpr long long lu_panel_doubles(int n) {
+  return n <= kLuRows ? LNB * (lu_pitch(n) + kLuStripPitch) : (long long)n * LNB;
+}
 
 }  // namespace ttb
