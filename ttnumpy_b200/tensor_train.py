@@ -320,7 +320,7 @@ class TensorTrain:
         if self.col_modes != other.row_modes:
             raise DimensionMismatch("Tensor trains must have the same last and first physical "
                                     "dimensions respectively")
-        cores = [K.kron(a, x) for a, x in zip(self.cores, other.cores)]
+        cores = K.kron_many(list(zip(self.cores, other.cores)))
         return _round_result(TensorTrain._wrap(cores), truncate, error, max_rank, method, seed,
                              options)
 
