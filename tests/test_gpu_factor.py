@@ -102,3 +102,34 @@ def test_lu_zero_pivot(K, n, at):
     info = torch.zeros(1, dtype=torch.int32, device="cuda")
     K.lu_solve_(dev(a.T), dev(np.ones(n)), info)
     assert info.item() == at
+
+
+@pytest.mark.parametrize("m,k", [(511, 30), (512, 96), (513, 97), (600, 128), (769, 2), (1025, 64),
+                                 (2305, 33), (5000, 128), (20000, 5)])
+def test_tall_trees(K, m, k):
+    """Tall matrices go as trees of row blocks (from 512 rows, up to 128
+    columns; short last nodes, odd heights): LAPACK's R with its signs, with
+    and without Q, from row- and column-major storage, and several in one
+    call."""
+    rng = np.random.default_rng(m + k)
+    a = rng.standard_normal((m, k)) * np.logspace(0, -6, k)
+    r_ref = sla.qr(a, mode="r")[0][:k]
+    x = dev(a)
+    both = K.qr_many([(x, True, True, None, None), (dev(a.T).t(), True, True, None, None),
+                      (x, False, True, None, None), (x[:40], True, True, None, None)])
+    for q, r in both[:3]:
+        r = r.cpu().numpy()
+        assert np.linalg.norm(r - r_ref) < 1e-11 * np.linalg.norm(r_ref)
+        if q is not None:
+            q = q.cpu().numpy()
+            assert np.linalg.norm(q @ r - a) < 1e-13 * np.linalg.norm(a)
+            assert orth(q) < 1e-13
+    u, s, vh = (t.cpu().numpy() for t in K.svd(x.t()))
+    assert np.abs(s - sla.svdvals(a)).max() <= 1e-13 * s[0]
+    assert np.linalg.norm((u * s) @ vh - a.T) < 1e-13 * np.linalg.norm(a)
+    assert orth(u) < 1e-12 and orth(vh.T) < 1e-12
+    for want in ({"want_u": False}, {"want_vh": False}):
+        u, s1, vh = K.svd(x, **want)
+        factor = (u if u is not None else vh.t()).cpu().numpy()
+        assert orth(factor) < 1e-12
+        assert np.abs(s1.cpu().numpy() - s).max() <= 1e-13 * s[0]

@@ -504,6 +504,266 @@ __global__ void __launch_bounds__(TTB_THREADS) k_lu(const __grid_constant__ LBat
   if (q.info && threadIdx.x == 0) *q.info = info;
 }
 
+// ---------------------------------------------------------------------------
+// tall factorisations as trees of blocks
+// ---------------------------------------------------------------------------
+
+// A tall matrix is cut into row blocks that are factorised side by side, one
+// thread block each; their R factors are stacked, at most kTreeFan at a time,
+// and factorised again, up to one R (the TSQR of Demmel, Grigori, Hoemmen and
+// Langou, "Communication-optimal parallel and sequential QR and LU
+// factorizations", 2012).  Q comes back down the tree: each node applies its
+// reflectors to the k x k block its parent gives it.  One thread block alone
+// is bound by its own column chain and memory traffic over all rows (3072 x
+// 96 with Q: 13.9 ms); a tree's chain is one node of a few hundred rows per
+// level.
+constexpr int kTreeLevels = 24;  // 2^23 row blocks, halved at least at every level
+struct Tree {
+  const double* a;       // M x K view (K <= kTreeCols)
+  i64 a_rs, a_cs;
+  double* q;             // M x K view or NULL
+  i64 q_rs, q_cs;
+  double* r;             // QR: K x K view or NULL
+  i64 r_rs, r_cs;
+  double* s;             // SVD: singular values, NULL for a QR
+  double* vh;            // SVD: K x K view or NULL
+  i64 vh_rs, vh_cs;
+  int* status;
+  int M, K, levels, fan, svd;
+  int cnt[kTreeLevels];  // nodes of a level (level 0: row blocks)
+  // a level's reflectors, scalars and Q blocks in ``work``
+  i64 w[kTreeLevels], tau[kTreeLevels], o[kTreeLevels];
+  i64 root, sgn, first, sq, us;
+  double* work;
+
+  __host__ __device__ i64 row0(int i) const { return (i64)M * i / cnt[0]; }
+  __host__ __device__ int rows(int l, int i) const {
+    if (l == 0) return (int)(row0(i + 1) - row0(i));
+    const int left = cnt[l - 1] - i * fan;
+    return (left < fan ? left : fan) * K;
+  }
+  __host__ __device__ i64 at(int l, int i) const {  // first entry of a node's block
+    return l == 0 ? (row0(i) + 2 * i) * K : (i64)i * (fan * K + 1) * K;
+  }
+  __host__ __device__ static i64 step(int rows) { return (rows + 1) & ~1; }
+};
+
+constexpr int kTreeCols = 128, kTreeRows = 512, kTreeGroup = 8;
+// Problems of one call up to which the trees are used: more fill the chip
+// with a block each.
+constexpr int kTreeProblems = 16;
+
+// Tall enough that two levels of blocks beat one block: 512 x 96 takes 0.69 ms
+// in one block, 256 x 64 (where one block's tile ends) 0.21 ms.
+int tree_block(int K) { return K <= 96 ? 256 : 512; }
+bool tree_shape(int M, int K) {
+  return M >= kTreeRows && M > tree_block(K) && M < (1 << 28) && K >= 1 && K <= kTreeCols &&
+         M >= 3 * K;
+}
+
+// Row blocks and fan-in such that a node has at most 256 rows (512 above 96
+// columns: at least twice the columns), and the work areas of the tree.
+i64 tree_layout(Tree& t, int M, int K) {
+  t.M = M;
+  t.K = K;
+  const int high = tree_block(K);
+  t.fan = std::max(2, 256 / K);
+  t.cnt[0] = (M + high - 1) / high;
+  t.levels = 1;
+  while (t.cnt[t.levels - 1] > 1) {
+    t.cnt[t.levels] = (t.cnt[t.levels - 1] + t.fan - 1) / t.fan;
+    t.levels++;
+  }
+  i64 off = 0;
+  auto take = [&](i64 n) {
+    const i64 p = off;
+    off += (n + 1) & ~(i64)1;
+    return p;
+  };
+  for (int l = 0; l < t.levels; ++l) {
+    const i64 block = l == 0 ? ((i64)M + 2 * t.cnt[0]) * K : (i64)t.cnt[l] * (t.fan * K + 1) * K;
+    t.w[l] = take(block);
+    t.tau[l] = take((i64)t.cnt[l] * K);
+    t.o[l] = l == 0 ? 0 : take(block);
+  }
+  t.root = take((i64)K * K);
+  t.sgn = take(K);
+  t.first = take((i64)(t.rows(0, 0) + 1) * K);
+  t.sq = take(triangle_svd_doubles(K));
+  t.us = take((i64)K * K);
+  return off;
+}
+
+struct TreeBatch {
+  int count;
+  Tree d[kTreeGroup];
+};
+
+__device__ __forceinline__ double* node_shared(double* dsm, int rows, int k) {
+  return node_smem(rows, k) * 8 <= kSmemCap ? dsm : nullptr;
+}
+
+// Level l's nodes: factorised, R into the parent's stack (or the root).
+__global__ void __launch_bounds__(TTB_THREADS) k_tree_up(const __grid_constant__ TreeBatch tb,
+                                                         int l) {
+  extern __shared__ __align__(16) double dsm[];
+  const Tree& t = tb.d[blockIdx.y];
+  const int i = blockIdx.x, K = t.K;
+  if (l >= t.levels || i >= t.cnt[l]) return;
+  const int rows = t.rows(l, i);
+  double* W = t.work + t.w[l] + t.at(l, i);
+  const i64 ld = Tree::step(rows);
+  const CMat A = l == 0 ? CMat{t.a + t.row0(i) * t.a_rs, t.a_rs, t.a_cs} : CMat{W, 1, ld};
+  Mat R{t.work + t.root, 1, K};
+  if (l + 1 < t.levels) {
+    const int up = i / t.fan;
+    R = Mat{t.work + t.w[l + 1] + t.at(l + 1, up) + (i64)(i % t.fan) * K, 1,
+            Tree::step(t.rows(l + 1, up))};
+  }
+  cta_node_factor(A, rows, K, W, ld, t.work + t.tau[l] + (i64)i * K, node_shared(dsm, rows, K), R);
+}
+
+// The SVD of a tree's root: singular values, right factor, and the left one
+// into the root's place.
+__global__ void __launch_bounds__(TTB_THREADS) k_tree_svd(const __grid_constant__ TreeBatch tb) {
+  extern __shared__ __align__(16) double dsm[];
+  __shared__ double red[TTB_WARPS];
+  const Tree& t = tb.d[blockIdx.x];
+  const int K = t.K;
+  double* work = triangle_svd_doubles(K) * 8 <= kSmemCap ? dsm : t.work + t.sq;
+  const int st = cta_triangle_svd(t.work + t.root, K, work, Mat{t.work + t.us, 1, K}, t.s,
+                                  Mat{t.vh, t.vh_rs, t.vh_cs}, t.q ? t.work + t.root : nullptr,
+                                  red);
+  if (t.status && threadIdx.x == 0) *t.status = st;
+}
+
+// Level l's nodes from the top down: the node's Q times its parent's block
+// (the root starts from the left factor of an SVD, or from the identity).
+// ``part`` 0: every node; 1: the first node only, a row block into
+// ``first``; 2: every node, the row blocks with their columns signed.
+__global__ void __launch_bounds__(TTB_THREADS) k_tree_down(const __grid_constant__ TreeBatch tb,
+                                                           int l, int part) {
+  extern __shared__ __align__(16) double dsm[];
+  const Tree& t = tb.d[blockIdx.y];
+  const int i = blockIdx.x, K = t.K;
+  if (l >= t.levels || i >= t.cnt[l]) return;
+  // without Q only its first rows are needed, for the signs
+  if (!t.q && (t.svd || part == 2 || i > 0)) return;
+  const int rows = t.rows(l, i);
+  double* top = t.svd ? t.work + t.root : nullptr;
+  i64 ktop = K;
+  if (l + 1 < t.levels) {
+    const int up = i / t.fan;
+    ktop = Tree::step(t.rows(l + 1, up));
+    top = t.work + t.o[l + 1] + t.at(l + 1, up) + (i64)(i % t.fan) * K;
+    if (part == 2) {
+      const double* sgn = t.work + t.sgn;
+      for (int e = threadIdx.x; e < K * K; e += TTB_THREADS) top[e % K + (e / K) * ktop] *= sgn[e / K];
+    }
+  }
+  const i64 ld = Tree::step(rows);
+  Mat X{t.work + t.o[l] + t.at(l, i), 1, ld};
+  if (l == 0) X = part == 1 ? Mat{t.work + t.first, 1, rows} : Mat{t.q + t.row0(i) * t.q_rs, t.q_rs, t.q_cs};
+  cta_node_apply(t.work + t.w[l] + t.at(l, i), ld, rows, K, t.work + t.tau[l] + (i64)i * K,
+                 node_shared(dsm, rows, K), top, ktop, X);
+}
+
+// LAPACK's signs for a tree's QR.  A Householder factorisation of the tree's
+// Q itself, whose R is a sign matrix D, has the reflectors of the whole
+// matrix, so Q D and D R are what dgeqrf and dorgqr give; D is found on Q's
+// first K rows alone by eliminating with d_j = -sign(q_jj) at each step
+// (Ballard et al., "Reconstructing Householder vectors from tall-skinny QR",
+// 2014, section IV).
+__global__ void __launch_bounds__(TTB_THREADS) k_tree_signs(const __grid_constant__ TreeBatch tb) {
+  extern __shared__ __align__(16) double dsm[];
+  const Tree& t = tb.d[blockIdx.x];
+  const int K = t.K, ld = odd_step(K), rows = t.rows(0, 0);
+  const double* Q = t.work + t.first;
+  for (int e = threadIdx.x; e < K * K; e += TTB_THREADS)
+    dsm[e % K + (e / K) * ld] = Q[e % K + (i64)(e / K) * rows];
+  double* sgn = t.work + t.sgn;
+  for (int j = 0; j < K; ++j) {
+    __syncthreads();
+    const double q = dsm[j + j * ld], d = q >= 0.0 ? -1.0 : 1.0, inv = 1.0 / (q - d);
+    if (threadIdx.x == 0) sgn[j] = d;
+    const int left = K - j - 1;
+    for (int e = threadIdx.x; e < left * left; e += TTB_THREADS) {
+      const int i = j + 1 + e % left, c = j + 1 + e / left;
+      dsm[i + c * ld] = fma(-dsm[i + j * ld] * inv, dsm[j + c * ld], dsm[i + c * ld]);
+    }
+  }
+  __syncthreads();
+  if (!t.r) return;
+  const double* R = t.work + t.root;
+  for (int e = threadIdx.x; e < K * K; e += TTB_THREADS) {
+    const int i = e / K, j = e % K;
+    t.r[i * t.r_rs + j * t.r_cs] = i <= j ? sgn[i] * R[i + (i64)j * K] : 0.0;
+  }
+}
+
+int g_smem_tree[4][kMaxDevices];
+
+int run_trees(const std::vector<Tree>& all, cudaStream_t s) {
+  const void* kernels[4] = {(const void*)k_tree_up, (const void*)k_tree_svd,
+                            (const void*)k_tree_down, (const void*)k_tree_signs};
+  for (int i = 0; i < 4; ++i)
+    if (int e = smem_limit_once(kernels[i], kSmemCap, g_smem_tree[i])) return e;
+  for (size_t i0 = 0; i0 < all.size(); i0 += kTreeGroup) {
+    TreeBatch tb;
+    tb.count = (int)std::min<size_t>(kTreeGroup, all.size() - i0);
+    int levels = 0, most[kTreeLevels] = {};
+    i64 smem[kTreeLevels] = {}, square = 0, signs = 0;
+    bool any_q = false, any_svd = false, any_qr = false;
+    for (int j = 0; j < tb.count; ++j) {
+      const Tree& t = tb.d[j] = all[i0 + j];
+      levels = std::max(levels, t.levels);
+      for (int l = 0; l < t.levels; ++l) {
+        most[l] = std::max(most[l], t.cnt[l]);
+        // every node that fits is worked on in shared memory, also beside
+        // larger ones that do not (a stack's last node may be a short one)
+        for (int i = 0; i < t.cnt[l]; ++i) {
+          const i64 need = node_smem(t.rows(l, i), t.K) * 8;
+          if (need <= kSmemCap) smem[l] = std::max(smem[l], need);
+        }
+      }
+      if (triangle_svd_doubles(t.K) * 8 <= kSmemCap)
+        square = std::max<i64>(square, triangle_svd_doubles(t.K) * 8);
+      signs = std::max<i64>(signs, (i64)odd_step(t.K) * t.K * 8);
+      any_q = any_q || t.q;
+      any_svd = any_svd || t.svd;
+      any_qr = any_qr || !t.svd;
+    }
+    for (int l = 0; l < levels; ++l) {
+      k_tree_up<<<dim3(most[l], tb.count), TTB_THREADS, (size_t)smem[l], s>>>(tb, l);
+      counted();
+    }
+    if (any_svd) {
+      k_tree_svd<<<tb.count, TTB_THREADS, (size_t)square, s>>>(tb);
+      counted();
+      for (int l = levels - 1; any_q && l >= 0; --l) {
+        k_tree_down<<<dim3(most[l], tb.count), TTB_THREADS, (size_t)smem[l], s>>>(tb, l, 0);
+        counted();
+      }
+    } else if (any_qr) {
+      // without any Q, the signs still need its first rows
+      for (int l = levels - 1; l > 0; --l) {
+        k_tree_down<<<dim3(any_q ? most[l] : 1, tb.count), TTB_THREADS, (size_t)smem[l], s>>>(
+            tb, l, any_q ? 0 : 1);
+        counted();
+      }
+      k_tree_down<<<dim3(1, tb.count), TTB_THREADS, (size_t)smem[0], s>>>(tb, 0, 1);
+      counted();
+      k_tree_signs<<<tb.count, TTB_THREADS, (size_t)signs, s>>>(tb);
+      counted();
+      if (any_q) {
+        k_tree_down<<<dim3(most[0], tb.count), TTB_THREADS, (size_t)smem[0], s>>>(tb, 0, 2);
+        counted();
+      }
+    }
+  }
+  return last_error();
+}
+
 // the one-CTA factorisations' shared-memory limit on the current device
 int configure_smem() {
   int e = smem_limit_once((const void*)k_qr, kSmemCap, g_smem_qr);
@@ -1556,11 +1816,42 @@ int ttb_project(const ttb_project_t* ps, int count, void* stream) {
   return launch_gemms(s2, s);
 }
 
-long long ttb_qr_work_doubles(int m, int k) { return qr_need(m, k); }
+long long ttb_qr_work_doubles(int m, int k) {
+  Tree t;
+  return tree_shape(m, k) ? std::max(qr_need(m, k), tree_layout(t, m, k)) : qr_need(m, k);
+}
 
 int ttb_qr(const ttb_qr_t* ps, int count, void* stream) {
   if (int e = configure_smem()) return e;
   cudaStream_t s = as_stream(stream);
+  std::vector<ttb_qr_t> rest;
+  std::vector<Tree> trees;
+  for (int i = 0; i < count; ++i)
+    if (tree_shape(ps[i].m, ps[i].k)) trees.emplace_back();
+  if (!trees.empty() && (int)trees.size() <= kTreeProblems) {
+    trees.clear();
+    for (int i = 0; i < count; ++i) {
+      const ttb_qr_t& p = ps[i];
+      if (!tree_shape(p.m, p.k)) {
+        rest.push_back(p);
+        continue;
+      }
+      Tree t = {};
+      tree_layout(t, p.m, p.k);
+      t.a = p.a, t.a_rs = p.a_rs, t.a_cs = p.a_cs;
+      t.q = p.q, t.q_rs = p.q_rs, t.q_cs = p.q_cs;
+      t.r = p.r, t.r_rs = p.r_rs, t.r_cs = p.r_cs;
+      t.work = p.work;
+      trees.push_back(t);
+    }
+    double fl = 0.0;
+    for (const Tree& t : trees)
+      fl += (t.q ? 2.0 : 1.0) * (2.0 * t.M * t.K * (double)t.K - 2.0 / 3.0 * t.K * (double)t.K * t.K);
+    ProfScope prof(P_QR, s, fl, 0.0);
+    if (int e = run_trees(trees, s)) return e;
+    ps = rest.data();
+    count = (int)rest.size();
+  }
   for (int i0 = 0; i0 < count; i0 += kMaxQ) {
     QBatch qb;
     qb.count = std::min(kMaxQ, count - i0);
@@ -1635,19 +1926,57 @@ int ttb_qr_static(const ttb_qr_t* ps, int count, void* stream) {
 
 long long ttb_svd_work_doubles(int m, int k) {
   int M = std::max(m, k), K = std::min(m, k);
-  return svd_tall_need(M, K);
+  Tree t;
+  return tree_shape(M, K) ? std::max(svd_tall_need(M, K), tree_layout(t, M, K))
+                          : svd_tall_need(M, K);
 }
 
 int ttb_svd(const ttb_svd_t* ps, int count, void* stream) {
   if (int e = configure_smem()) return e;
   cudaStream_t s = as_stream(stream);
+  std::vector<ttb_svd_t> rest;
+  std::vector<Tree> trees;
+  auto tall = [](const ttb_svd_t& p) {
+    return tree_shape(std::max(p.m, p.k), std::min(p.m, p.k));
+  };
+  for (int i = 0; i < count; ++i)
+    if (tall(ps[i])) trees.emplace_back();
+  if (!trees.empty() && (int)trees.size() <= kTreeProblems) {
+    trees.clear();
+    double fl = 0.0;
+    for (int i = 0; i < count; ++i) {
+      const ttb_svd_t& p = ps[i];
+      if (!tall(p)) {
+        rest.push_back(p);
+        continue;
+      }
+      // a wide matrix by its transpose, as k_svd does
+      const bool up = p.m >= p.k;
+      Tree t = {};
+      tree_layout(t, std::max(p.m, p.k), std::min(p.m, p.k));
+      t.svd = 1;
+      t.a = p.a, t.a_rs = up ? p.a_rs : p.a_cs, t.a_cs = up ? p.a_cs : p.a_rs;
+      t.q = up ? p.u : p.vh, t.q_rs = up ? p.u_rs : p.vh_cs, t.q_cs = up ? p.u_cs : p.vh_rs;
+      t.vh = up ? p.vh : p.u, t.vh_rs = up ? p.vh_rs : p.u_cs, t.vh_cs = up ? p.vh_cs : p.u_rs;
+      t.s = p.s;
+      t.status = p.status;
+      t.work = p.work;
+      fl += 4.0 * t.M * t.K * (double)t.K - 4.0 / 3.0 * t.K * (double)t.K * t.K;
+      trees.push_back(t);
+    }
+    ProfScope prof(P_SVD, s, fl, 0.0);
+    if (int e = run_trees(trees, s)) return e;
+    ps = rest.data();
+    count = (int)rest.size();
+  }
   for (int i0 = 0; i0 < count; i0 += kMaxS) {
     SBatch sb;
     sb.count = std::min(kMaxS, count - i0);
     i64 smem = 0;
     for (int j = 0; j < sb.count; ++j) {
       sb.d[j] = ps[i0 + j];
-      const i64 whole = ttb_svd_work_doubles(sb.d[j].m, sb.d[j].k) * 8;
+      const i64 whole = svd_tall_need(std::max(sb.d[j].m, sb.d[j].k),
+                                      std::min(sb.d[j].m, sb.d[j].k)) * 8;
       const i64 blk = blocked_smem(std::min(sb.d[j].m, sb.d[j].k)) * 8;
       if (whole <= kSmemCap) {
         sb.mode[j] = 0;

@@ -16,23 +16,6 @@
 
 namespace ttb {
 
-// W (column major, column step ldw) <- the m x k view A, reading along A's
-// unit-stride direction.
-static __device__ __forceinline__ void cta_load(CMat A, double* W, i64 ldw, int m, int k) {
-  const int total = m * k;
-  if (A.cs == 1) {
-    for (int e = threadIdx.x; e < total; e += TTB_THREADS) {
-      const int i = e / k, j = e - i * k;
-      W[i + j * ldw] = A(i, j);
-    }
-  } else {
-    for (int e = threadIdx.x; e < total; e += TTB_THREADS) {
-      const int j = e / m, i = e - j * m;
-      W[i + j * ldw] = A(i, j);
-    }
-  }
-}
-
 // ---------------------------------------------------------------------------
 // Householder QR
 // ---------------------------------------------------------------------------
@@ -418,7 +401,7 @@ static __device__ __noinline__ void hh_columns(const double* W, i64 ld, int m, i
       const int c = g0 + tile_col<LPC>(s);
       if (start == HH_TOP) {
         const bool in = c < ncols;
-        tile_load<LPC, RP>(in ? top + order[c] * ktop : top, in ? kt : 0, x[s]);
+        tile_load<LPC, RP>(in ? top + (order ? order[c] : c) * ktop : top, in ? min(kt, m) : 0, x[s]);
       } else {
 #pragma unroll
         for (int r = 0; r < RP; ++r) {
@@ -495,7 +478,7 @@ static __device__ void cta_hh_apply(const double* W, i64 ld, int m, int p, const
     for (int e = threadIdx.x; e < m * ncols; e += TTB_THREADS) {
       const int i = e / ncols, c = e % ncols;
       X(i, c) = start == HH_IDENT ? (i == c ? 1.0 : 0.0)
-                                  : (i < kt ? top[i + order[c] * ktop] : 0.0);
+                                  : (i < kt ? top[i + (order ? order[c] : c) * ktop] : 0.0);
     }
     __syncthreads();
   }
@@ -2065,6 +2048,65 @@ __device__ __noinline__ int cta_svd_tall_blocked(CMat A, int m, int k, double* W
   }
   __syncthreads();
   cta_apply_q_blocked(W, m, k, tau, U, k, Y, G, Tm, gsm, ring);
+  return status;
+}
+
+// ---------------------------------------------------------------------------
+// nodes of a tree of factorisations (ttb200.cu)
+// ---------------------------------------------------------------------------
+
+__device__ __noinline__ void cta_node_factor(CMat A, int rows, int k, double* W, i64 ld,
+                                             double* tau, double* smem, Mat R) {
+  double* F = smem ? smem : W;
+  const i64 lf = smem ? ld + 2 : ld;
+  if (F != A.p) cta_load(A, F, lf, rows, k);
+  __syncthreads();
+  cta_hh(F, lf, rows, k, tau);
+  const int p = min(rows, k);
+  for (int e = threadIdx.x; e < k * k; e += TTB_THREADS) {
+    const int i = e % k, j = e / k;
+    R(i, j) = (i < p && i <= j) ? F[i + j * lf] : 0.0;
+  }
+  if (smem)
+    for (int e = threadIdx.x; e < rows * k; e += TTB_THREADS) {
+      const int i = e % rows, j = e / rows;
+      W[i + j * ld] = F[i + j * lf];
+    }
+}
+
+__device__ __noinline__ void cta_node_apply(const double* W, i64 ld, int rows, int k,
+                                            const double* tau, double* smem, const double* top,
+                                            i64 ktop, Mat X) {
+  const double* F = W;
+  i64 lf = ld;
+  if (smem) {
+    lf = ld + 2;
+    for (int e = threadIdx.x; e < rows * k; e += TTB_THREADS) {
+      const int i = e % rows, j = e / rows;
+      smem[i + j * lf] = W[i + j * ld];
+    }
+    F = smem;
+  }
+  __syncthreads();
+  cta_hh_apply(F, lf, rows, min(rows, k), tau, X, k, top ? HH_TOP : HH_IDENT, top, k, ktop);
+}
+
+__device__ __noinline__ int cta_triangle_svd(const double* R, int k, double* work, Mat Us,
+                                             double* S, Mat Vh, double* top, double* red) {
+  const i64 ld = svd_step(k);
+  double* B = align2(work);
+  double* V = B + ld * k;
+  double* sv = V + ld * k;
+  int* order = reinterpret_cast<int*>(sv + k);
+  double* tau2 = sv + 2 * k;
+  int* flag = reinterpret_cast<int*>(sv + 3 * k);
+  for (int e = threadIdx.x; e < k * k; e += TTB_THREADS) B[e % k + (e / k) * ld] = R[e];
+  __syncthreads();
+  const int want = !Vh.p ? SQ_LEFT : !top ? SQ_RIGHT : SQ_BOTH;
+  const int status = cta_svd_square(want, k, B, V, sv, order, tau2, flag, Us, S, Vh, red);
+  if (top)
+    for (int e = threadIdx.x; e < k * k; e += TTB_THREADS)
+      top[e] = V[e % k + order[e / k] * ld];
   return status;
 }
 

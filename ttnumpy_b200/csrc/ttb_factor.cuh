@@ -18,6 +18,23 @@ constexpr int LNB = 16;   // panel width of the blocked factorisations
 constexpr int YCH = 512;  // columns per chunk of the blocked trailing updates
 constexpr int LNB2 = 64;  // outer panel width of the two-level R-only QR
 
+// W (column major, column step ldw) <- the m x k view A, reading along A's
+// unit-stride direction.
+static __device__ __forceinline__ void cta_load(CMat A, double* W, i64 ldw, int m, int k) {
+  const int total = m * k;
+  if (A.cs == 1) {
+    for (int e = threadIdx.x; e < total; e += TTB_THREADS) {
+      const int i = e / k, j = e - i * k;
+      W[i + j * ldw] = A(i, j);
+    }
+  } else {
+    for (int e = threadIdx.x; e < total; e += TTB_THREADS) {
+      const int j = e / m, i = e - j * m;
+      W[i + j * ldw] = A(i, j);
+    }
+  }
+}
+
 __device__ void cta_qr(CMat A, int m, int k, double* W, i64 ldw, double* tau, Mat Q, Mat R,
                        double* red, bool tiled = true);
 __device__ void cta_qr_blocked(CMat A, int m, int k, double* W, double* tau, Mat Q, Mat R,
@@ -49,5 +66,29 @@ __host__ __device__ constexpr int lu_pitch(int rows) { return ((rows + 15) & ~15
 __host__ __device__ constexpr long long lu_panel_doubles(int n) {
   return n <= kLuRows ? LNB * (lu_pitch(n) + kLuStripPitch) : (long long)n * LNB;
 }
+
+// Nodes of a tree of factorisations.  ``smem`` (may be NULL) holds node_smem
+// doubles and is where the node's columns live meanwhile.
+// cta_node_factor: Householder QR of the rows x k view A (rows <= 2048): the
+// reflectors to W (column step ld, even) and tau, R (k x k, zero rows past
+// ``rows``).  A may be W itself.
+// cta_node_apply: X (rows x k) = the node's Q times [top; 0] (k x k, column
+// step ktop), or times [I; 0] without top.
+// cta_triangle_svd: SVD of the k x k upper-triangular R (column step k);
+// ``work`` (triangle_svd_doubles) in any memory, Us a k x k scratch view for
+// the case that both factors are wanted.  Vh may be NULL; ``top`` gets the
+// left factor (column step k) unless it is NULL.
+__host__ __device__ constexpr long long node_smem(int rows, int k) {
+  return ((long long)((rows + 1) & ~1) + 2) * k;
+}
+__host__ __device__ constexpr long long triangle_svd_doubles(int k) {
+  return 2LL * svd_step(k) * k + 3LL * k + 4;
+}
+__device__ void cta_node_factor(CMat A, int rows, int k, double* W, i64 ld, double* tau,
+                                double* smem, Mat R);
+__device__ void cta_node_apply(const double* W, i64 ld, int rows, int k, const double* tau,
+                               double* smem, const double* top, i64 ktop, Mat X);
+__device__ int cta_triangle_svd(const double* R, int k, double* work, Mat Us, double* S, Mat Vh,
+                                double* top, double* red);
 
 }  // namespace ttb
