@@ -415,19 +415,21 @@ __global__ void __launch_bounds__(TTB_THREADS) k_qr(const __grid_constant__ QBat
     double* W = dsm;
     const int ldw = odd_step(m);
     double* tau = W + (i64)ldw * k;
-    cta_qr(CMat{q.a, q.a_rs, q.a_cs}, m, k, W, ldw, tau, Mat{q.q, q.q_rs, q.q_cs},
+    cta_qr<true>(CMat{q.a, q.a_rs, q.a_cs}, m, k, W, ldw, tau, Mat{q.q, q.q_rs, q.q_cs},
            Mat{q.r, q.r_rs, q.r_cs}, red);
   } else {
     double* Y = dsm;
     double* G = Y + (i64)LNB * min(k, YCH);
     double* Tm = G + LNB * LNB;
-    cta_qr_blocked(CMat{q.a, q.a_rs, q.a_cs}, m, k, q.work, q.work + (i64)m * k,
+    cta_qr_blocked<true>(CMat{q.a, q.a_rs, q.a_cs}, m, k, q.work, q.work + (i64)m * k,
                    Mat{q.q, q.q_rs, q.q_cs}, Mat{q.r, q.r_rs, q.r_cs}, Y, G, Tm, red, gsm);
   }
 }
 
 i64 qr_need(int m, int k) { return (i64)odd_step(m) * k + std::min(m, k); }
-i64 blocked_smem(int k) { return (i64)LNB * std::min(std::max(k, 1), YCH) + 2 * LNB * LNB; }
+__host__ __device__ inline i64 blocked_smem(int k) {
+  return (i64)LNB * (k < 1 ? 1 : k < YCH ? k : YCH) + 2 * LNB * LNB;
+}
 
 constexpr int kMaxS = 16;
 struct SBatch {
@@ -441,6 +443,11 @@ i64 svd_tall_need(int M, int K) {
   return (i64)odd_step(M) * K + 2 * (i64)svd_step(K) * K + 4 * (i64)K + 6;
 }
 
+// shared doubles of a blocked SVD with its square matrices in shared memory
+__host__ __device__ inline i64 svd_square_smem(int K) {
+  return blocked_smem(K) + 2 * (i64)svd_step(K) * K + 3 * (i64)K + 6;
+}
+
 __global__ void __launch_bounds__(TTB_THREADS) k_svd(const __grid_constant__ SBatch sb) {
   extern __shared__ double dsm[];
   __shared__ double red[TTB_WARPS];
@@ -450,11 +457,13 @@ __global__ void __launch_bounds__(TTB_THREADS) k_svd(const __grid_constant__ SBa
   const bool tall = q.m >= q.k;
   const int M = tall ? q.m : q.k, K = tall ? q.k : q.m;
   const int mode = sb.mode[blockIdx.x];
-  double* base = mode == 0 ? dsm : q.work;
-  double* W = base;
+  double* W = mode == 0 ? dsm : q.work;
   const int ldw = odd_step(M);
   double* tau = W + (i64)ldw * K;
-  double* Bsq = align2(tau + K);
+  // a large W in global memory, the square matrices still shared if they fit
+  double* square = tau + K;
+  if (mode != 0 && svd_square_smem(K) * 8 <= kSmemCap) square = dsm + blocked_smem(K);
+  double* Bsq = align2(square);
   double* V = Bsq + (i64)svd_step(K) * K;
   double* sv = V + (i64)svd_step(K) * K;
   int* order = reinterpret_cast<int*>(sv + K);
@@ -466,12 +475,12 @@ __global__ void __launch_bounds__(TTB_THREADS) k_svd(const __grid_constant__ SBa
   Mat Vh = tall ? Mat{q.vh, q.vh_rs, q.vh_cs} : Mat{q.u, q.u_cs, q.u_rs};
   int st;
   if (mode == 0) {
-    st = cta_svd_tall(A, M, K, W, ldw, tau, Bsq, V, sv, order, flag, tau2, U, q.s, Vh, red);
+    st = cta_svd_tall<true>(A, M, K, W, ldw, tau, Bsq, V, sv, order, flag, tau2, U, q.s, Vh, red);
   } else {
     double* Y = dsm;
     double* G = Y + (i64)LNB * min(K, YCH);
     double* Tm = G + LNB * LNB;
-    st = cta_svd_tall_blocked(A, M, K, W, tau, Bsq, V, sv, order, flag, tau2, U, q.s, Vh, Y, G,
+    st = cta_svd_tall_blocked<true>(A, M, K, W, tau, Bsq, V, sv, order, flag, tau2, U, q.s, Vh, Y, G,
                               Tm, red, gsm);
   }
   if (q.status && threadIdx.x == 0) *q.status = st;
@@ -549,6 +558,7 @@ struct Tree {
 };
 
 constexpr int kTreeCols = 128, kTreeRows = 512, kTreeGroup = 8;
+constexpr int kTreeSlice = 32;  // columns of Q a block takes on the way down
 // Problems of one call up to which the trees are used: more fill the chip
 // with a block each.
 constexpr int kTreeProblems = 16;
@@ -638,15 +648,17 @@ __global__ void __launch_bounds__(TTB_THREADS) k_tree_svd(const __grid_constant_
 }
 
 // Level l's nodes from the top down: the node's Q times its parent's block
-// (the root starts from the left factor of an SVD, or from the identity).
+// (the root starts from the left factor of an SVD, or from the identity), a
+// block per kTreeSlice of its columns.
 // ``part`` 0: every node; 1: the first node only, a row block into
 // ``first``; 2: every node, the row blocks with their columns signed.
 __global__ void __launch_bounds__(TTB_THREADS) k_tree_down(const __grid_constant__ TreeBatch tb,
                                                            int l, int part) {
   extern __shared__ __align__(16) double dsm[];
   const Tree& t = tb.d[blockIdx.y];
-  const int i = blockIdx.x, K = t.K;
-  if (l >= t.levels || i >= t.cnt[l]) return;
+  const int i = blockIdx.x, K = t.K, c0 = blockIdx.z * kTreeSlice;
+  if (l >= t.levels || i >= t.cnt[l] || c0 >= K) return;
+  const int nc = min(kTreeSlice, K - c0);
   // without Q only its first rows are needed, for the signs
   if (!t.q && (t.svd || part == 2 || i > 0)) return;
   const int rows = t.rows(l, i);
@@ -658,14 +670,15 @@ __global__ void __launch_bounds__(TTB_THREADS) k_tree_down(const __grid_constant
     top = t.work + t.o[l + 1] + t.at(l + 1, up) + (i64)(i % t.fan) * K;
     if (part == 2) {
       const double* sgn = t.work + t.sgn;
-      for (int e = threadIdx.x; e < K * K; e += TTB_THREADS) top[e % K + (e / K) * ktop] *= sgn[e / K];
+      for (int e = threadIdx.x; e < K * nc; e += TTB_THREADS)
+        top[e % K + (c0 + e / K) * ktop] *= sgn[c0 + e / K];
     }
   }
   const i64 ld = Tree::step(rows);
   Mat X{t.work + t.o[l] + t.at(l, i), 1, ld};
   if (l == 0) X = part == 1 ? Mat{t.work + t.first, 1, rows} : Mat{t.q + t.row0(i) * t.q_rs, t.q_rs, t.q_cs};
   cta_node_apply(t.work + t.w[l] + t.at(l, i), ld, rows, K, t.work + t.tau[l] + (i64)i * K,
-                 node_shared(dsm, rows, K), top, ktop, X);
+                 node_shared(dsm, rows, K), top, ktop, X, c0, nc);
 }
 
 // LAPACK's signs for a tree's QR.  A Householder factorisation of the tree's
@@ -682,14 +695,15 @@ __global__ void __launch_bounds__(TTB_THREADS) k_tree_signs(const __grid_constan
   for (int e = threadIdx.x; e < K * K; e += TTB_THREADS)
     dsm[e % K + (e / K) * ld] = Q[e % K + (i64)(e / K) * rows];
   double* sgn = t.work + t.sgn;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   for (int j = 0; j < K; ++j) {
     __syncthreads();
     const double q = dsm[j + j * ld], d = q >= 0.0 ? -1.0 : 1.0, inv = 1.0 / (q - d);
     if (threadIdx.x == 0) sgn[j] = d;
-    const int left = K - j - 1;
-    for (int e = threadIdx.x; e < left * left; e += TTB_THREADS) {
-      const int i = j + 1 + e % left, c = j + 1 + e / left;
-      dsm[i + c * ld] = fma(-dsm[i + j * ld] * inv, dsm[j + c * ld], dsm[i + c * ld]);
+    for (int c = j + 1 + warp; c < K; c += TTB_WARPS) {
+      const double f = dsm[j + c * ld] * inv;
+      for (int i = j + 1 + lane; i < K; i += 32)
+        dsm[i + c * ld] = fma(-dsm[i + j * ld], f, dsm[i + c * ld]);
     }
   }
   __syncthreads();
@@ -713,6 +727,7 @@ int run_trees(const std::vector<Tree>& all, cudaStream_t s) {
     tb.count = (int)std::min<size_t>(kTreeGroup, all.size() - i0);
     int levels = 0, most[kTreeLevels] = {};
     i64 smem[kTreeLevels] = {}, square = 0, signs = 0;
+    int slices = 1;
     bool any_q = false, any_svd = false, any_qr = false;
     for (int j = 0; j < tb.count; ++j) {
       const Tree& t = tb.d[j] = all[i0 + j];
@@ -728,6 +743,7 @@ int run_trees(const std::vector<Tree>& all, cudaStream_t s) {
       }
       if (triangle_svd_doubles(t.K) * 8 <= kSmemCap)
         square = std::max<i64>(square, triangle_svd_doubles(t.K) * 8);
+      slices = std::max(slices, cdiv(t.K, kTreeSlice));
       signs = std::max<i64>(signs, (i64)odd_step(t.K) * t.K * 8);
       any_q = any_q || t.q;
       any_svd = any_svd || t.svd;
@@ -741,22 +757,22 @@ int run_trees(const std::vector<Tree>& all, cudaStream_t s) {
       k_tree_svd<<<tb.count, TTB_THREADS, (size_t)square, s>>>(tb);
       counted();
       for (int l = levels - 1; any_q && l >= 0; --l) {
-        k_tree_down<<<dim3(most[l], tb.count), TTB_THREADS, (size_t)smem[l], s>>>(tb, l, 0);
+        k_tree_down<<<dim3(most[l], tb.count, slices), TTB_THREADS, (size_t)smem[l], s>>>(tb, l, 0);
         counted();
       }
     } else if (any_qr) {
       // without any Q, the signs still need its first rows
       for (int l = levels - 1; l > 0; --l) {
-        k_tree_down<<<dim3(any_q ? most[l] : 1, tb.count), TTB_THREADS, (size_t)smem[l], s>>>(
-            tb, l, any_q ? 0 : 1);
+        k_tree_down<<<dim3(any_q ? most[l] : 1, tb.count, slices), TTB_THREADS, (size_t)smem[l],
+                      s>>>(tb, l, any_q ? 0 : 1);
         counted();
       }
-      k_tree_down<<<dim3(1, tb.count), TTB_THREADS, (size_t)smem[0], s>>>(tb, 0, 1);
+      k_tree_down<<<dim3(1, tb.count, slices), TTB_THREADS, (size_t)smem[0], s>>>(tb, 0, 1);
       counted();
       k_tree_signs<<<tb.count, TTB_THREADS, (size_t)signs, s>>>(tb);
       counted();
       if (any_q) {
-        k_tree_down<<<dim3(most[0], tb.count), TTB_THREADS, (size_t)smem[0], s>>>(tb, 0, 2);
+        k_tree_down<<<dim3(most[0], tb.count, slices), TTB_THREADS, (size_t)smem[0], s>>>(tb, 0, 2);
         counted();
       }
     }
@@ -1501,7 +1517,8 @@ __global__ void __launch_bounds__(TTB_THREADS) k_round(const __grid_constant__ t
                                                        i64 slot, i64 qslot) {
   extern __shared__ double dsm[];
   __shared__ double red[TTB_WARPS];
-  __shared__ GemmSmem gsm;
+  // the products run between the factorisations, in their area
+  GemmSmem& gsm = *reinterpret_cast<GemmSmem*>(dsm);
   __shared__ int rows_of[kRoundMaxD];
   __shared__ int nb_sh;
   const int pair = blockIdx.x;
@@ -1566,7 +1583,7 @@ __global__ void __launch_bounds__(TTB_THREADS) k_round(const __grid_constant__ t
     rows_of[k] = rl;  // rows of core k before its factorisation
     if (k == d - 1) break;
     const int pq = m < r_out ? m : r_out;
-    cta_qr(CMat{X, r_out, 1}, m, r_out, W, odd_step(m), tau,
+    cta_qr<true>(CMat{X, r_out, 1}, m, r_out, W, odd_step(m), tau,
            Mat{qcores + (i64)k * qslot, pq, 1}, Mat{Rm, RS, 1}, red);
     rl = pq;
   }
@@ -1590,10 +1607,10 @@ __global__ void __launch_bounds__(TTB_THREADS) k_round(const __grid_constant__ t
     int st;
     // the right factor only: U S is the matrix times its rows
     if (r >= c) {
-      st = cta_svd_tall(CMat{X, c, 1}, r, c, W, odd_step(r), tau, Bsq, V, sv, order, flag, tau2,
+      st = cta_svd_tall<true>(CMat{X, c, 1}, r, c, W, odd_step(r), tau, Bsq, V, sv, order, flag, tau2,
                         Mat{nullptr, 0, 0}, Sv, Mat{Vh, c, 1}, red);
     } else {
-      st = cta_svd_tall(CMat{X, 1, c}, c, r, W, odd_step(c), tau, Bsq, V, sv, order, flag, tau2,
+      st = cta_svd_tall<true>(CMat{X, 1, c}, c, r, W, odd_step(c), tau, Bsq, V, sv, order, flag, tau2,
                         Mat{Vh, 1, c}, Sv, Mat{nullptr, 0, 0}, red);
     }
     if (st < 0) status = -1;
@@ -1984,7 +2001,8 @@ int ttb_svd(const ttb_svd_t* ps, int count, void* stream) {
       } else {
         if (blk > kSmemCap) return (int)cudaErrorInvalidValue;
         sb.mode[j] = 1;
-        smem = std::max(smem, blk);
+        const i64 square = svd_square_smem(std::min(sb.d[j].m, sb.d[j].k)) * 8;
+        smem = std::max(smem, square <= kSmemCap ? square : blk);
       }
     }
     double fl = 0.0;

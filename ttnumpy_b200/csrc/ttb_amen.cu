@@ -920,7 +920,7 @@ __device__ __noinline__ void project(Ctx& c, const double* left, int a, int i, c
 __device__ __noinline__ void qr(Ctx& c, CMat A, int m, int k, Mat Q, Mat R) {
   const int p = min(m, k);
   if ((i64)m * k + p <= kPoolD) {
-    cta_qr(A, m, k, c.pool, m, c.pool + (i64)m * k, Q, R, c.sm->red, false);
+    cta_qr<false>(A, m, k, c.pool, m, c.pool + (i64)m * k, Q, R, c.sm->red);
     return;
   }
   const i64 mark = c.top;
@@ -933,9 +933,9 @@ __device__ __noinline__ void qr(Ctx& c, CMat A, int m, int k, Mat Q, Mat R) {
       // the one-level blocked factorisation of the same matrix, compared
       double* R1 = take(c, (i64)p * k);
       if (c.status) return;
-      cta_qr_blocked(A, m, k, W, W + (i64)m * k, Mat{nullptr, 0, 0}, Mat{R1, k, 1}, c.pool,
+      cta_qr_blocked<false>(A, m, k, W, W + (i64)m * k, Mat{nullptr, 0, 0}, Mat{R1, k, 1}, c.pool,
                      c.pool + (i64)LNB * YCH, c.pool + (i64)LNB * YCH + LNB * LNB, c.sm->red,
-                     *c.gsm, nullptr, false);
+                     *c.gsm, nullptr);
       double dsq = 0.0, rsq = 0.0;
       for (i64 e = threadIdx.x; e < (i64)p * k; e += TTB_THREADS) {
         const int i = (int)(e / k), j = (int)(e % k);
@@ -954,7 +954,8 @@ __device__ __noinline__ void qr(Ctx& c, CMat A, int m, int k, Mat Q, Mat R) {
   double* Y = c.pool;
   double* G = Y + (i64)LNB * YCH;
   double* Tm = G + LNB * LNB;
-  cta_qr_blocked(A, m, k, W, W + (i64)m * k, Q, R, Y, G, Tm, c.sm->red, *c.gsm, c.ring, false);
+  cta_qr_blocked<false>(A, m, k, W, W + (i64)m * k, Q, R, Y, G, Tm, c.sm->red, *c.gsm,
+                        c.ring);
   c.top = mark;
 }
 
@@ -983,14 +984,13 @@ __device__ __noinline__ void svd(Ctx& c, CMat A, int m, int k, Mat U, double* S,
   int* order = reinterpret_cast<int*>(sv + K);
   int* flag = reinterpret_cast<int*>(sv + 2 * K);
   if (in_pool) {
-    cta_svd_tall(At, M, K, W, M, tau, Bsq, V, sv, order, flag, nullptr, Ut, S, Vt, c.sm->red,
-                 false);
+    cta_svd_tall<false>(At, M, K, W, M, tau, Bsq, V, sv, order, flag, nullptr, Ut, S, Vt, c.sm->red);
   } else {
     double* Y = c.pool;
     double* G = Y + (i64)LNB * YCH;
     double* Tm = G + LNB * LNB;
-    cta_svd_tall_blocked(At, M, K, W, tau, Bsq, V, sv, order, flag, nullptr, Ut, S, Vt, Y, G, Tm,
-                         c.sm->red, *c.gsm, c.ring, false);
+    cta_svd_tall_blocked<false>(At, M, K, W, tau, Bsq, V, sv, order, flag, nullptr, Ut, S, Vt, Y, G, Tm,
+                         c.sm->red, *c.gsm, c.ring);
   }
   c.top = mark;
 }

@@ -317,6 +317,139 @@ static __device__ __forceinline__ void hh_reflect(double (&x)[SL][RP], const dou
   }
 }
 
+// x -= t (v . x) v for one slot, v's row pairs read from shared memory (twice:
+// held in registers they would crowd out the columns).
+template <int RP>
+static __device__ __forceinline__ void reflect_slot(double (&x)[RP], const double2* v, double t) {
+  double a[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+  for (int r = 0; r < RP; r += 2) {
+    const double2 p = v[4 * r];
+    a[r & 2] = fma(p.x, x[r], a[r & 2]);
+    a[(r & 2) + 1] = fma(p.y, x[r + 1], a[(r & 2) + 1]);
+  }
+  const double w = -t * group_sum<8>((a[0] + a[2]) + (a[1] + a[3]));
+#pragma unroll
+  for (int r = 0; r < RP; r += 2) {
+    const double2 p = v[4 * r];
+    x[r] = fma(w, p.x, x[r]);
+    x[r + 1] = fma(w, p.y, x[r + 1]);
+  }
+}
+
+// Column n of a panel, in one lane group of slot x, becomes reflector n: v
+// (zeros above, 1 at row n) to ``vb`` and tau to ``tb``, the other warps are
+// let go, then W's column n and tau[n] are written.  Rows below m only.
+template <int RP>
+static __device__ __forceinline__ void publish_slot(double (&x)[RP], int n, bool mine, int m,
+                                                    double2* vb, double* tb, double* wc,
+                                                    double* tau) {
+  double a = 0.0, c[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+  for (int r = 0; r < RP; ++r) {
+    const int i = tile_row<8>(r);
+    double y = x[r];
+    if (16 * (r >> 1) < kPanelMax) {  // rows above the pivot end within the panel's width
+      if (i == n) a = y;
+      if (i <= n) y = 0.0;
+    }
+    c[r & 3] = fma(y, y, c[r & 3]);
+  }
+  a = __shfl_sync(0xffffffffu, a, (threadIdx.x & 24) + ((n >> 1) & 7));
+  const double sigma = group_sum<8>((c[0] + c[2]) + (c[1] + c[3]));
+  double beta, t, scale;
+  hh_scalars(a, sigma, beta, t, scale);
+  if (mine) {
+#pragma unroll
+    for (int r = 0; r < RP; r += 2) {
+      const int i = tile_row<8>(r);
+      double2 p = make_double2(x[r] * scale, x[r + 1] * scale);
+      if (16 * (r >> 1) < kPanelMax) {
+        p.x = i > n ? p.x : i == n ? 1.0 : 0.0;
+        p.y = i + 1 > n ? p.y : i + 1 == n ? 1.0 : 0.0;
+      }
+      vb[4 * r] = p;
+    }
+    if ((threadIdx.x & 7) == 0) *tb = t;
+  }
+  __syncwarp();
+  step_arrive(n);
+  if (mine) {
+    if ((threadIdx.x & 7) == 0) tau[n] = t;
+#pragma unroll
+    for (int r = 0; r < RP; ++r) {
+      const int i = tile_row<8>(r);
+      if (t != 0.0) {
+        if (i > n) x[r] *= scale;
+        if (i == n) x[r] = beta;
+      }
+      if (i < m) wc[i] = x[r];
+    }
+  }
+}
+
+// hh_panel (below) for eight lanes a column, m <= 8 RP <= 256: reflectors go
+// through shared memory, ready to use, and the warp of the next column
+// updates and publishes it before its other columns, so that a column step
+// costs the chain of one column.  Neighbouring columns belong to different
+// warps (slot s of warp w: columns 32 s + 8 group + w), so that a publisher
+// is never more than one barrier ahead; its own late reads of a reflector
+// are why three buffers take turns.
+template <int RP, int SL>
+static __device__ __noinline__ void hh_panel8(double* W, i64 ld, int m, int k, double* tau,
+                                              double2 (*vbuf)[128], double* tb) {
+  static_assert(RP <= 32 && SL == 2 && TTB_WARPS == 8, "128 row pairs, two slots of 32 columns");
+  const int warp = threadIdx.x >> 5, lane8 = threadIdx.x & 7, group = (threadIdx.x & 31) >> 3;
+  const int p = m < k ? m : k;
+  double x[SL][RP];
+#pragma unroll
+  for (int s = 0; s < SL; ++s) {
+    const int c = 32 * s + 8 * group + warp;
+    tile_load<8, RP>(W + c * ld, c < k ? m : 0, x[s]);
+  }
+  __syncthreads();  // every warp has its columns; the buffers are free
+  int at = 2, to = 0;  // the buffers of steps j and j + 1
+  for (int j = -1; j < p; ++j) {
+    double t = 0.0;
+    const double2* v = vbuf[at] + lane8;
+    if (j >= 0) {
+      if (warp != (j & 7)) step_wait(j);
+      t = tb[at];
+    }
+    const int n = j + 1;
+    int done = -1;
+    if (n < p && warp == (n & 7)) {
+      done = n >> 5;
+      const bool mine = group == ((n >> 3) & 3);
+      if (done == 0) {
+        if (t != 0.0) reflect_slot<RP>(x[0], v, t);
+        publish_slot<RP>(x[0], n, mine, m, vbuf[to] + lane8, tb + to, W + n * ld, tau);
+      } else {
+        if (t != 0.0) reflect_slot<RP>(x[1], v, t);
+        publish_slot<RP>(x[1], n, mine, m, vbuf[to] + lane8, tb + to, W + n * ld, tau);
+      }
+    }
+    if (t != 0.0) {
+#pragma unroll
+      for (int s = 0; s < SL; ++s)
+        if (s != done && 32 * s + 24 + warp > j) reflect_slot<RP>(x[s], v, t);
+    }
+    at = to;
+    to = to == 2 ? 0 : to + 1;
+  }
+#pragma unroll
+  for (int s = 0; s < SL; ++s) {
+    const int c = 32 * s + 8 * group + warp;
+    if (c < p || c >= k) continue;
+#pragma unroll
+    for (int r = 0; r < RP; ++r) {
+      const int i = tile_row<8>(r);
+      if (i < m) W[i + c * ld] = x[s][r];
+    }
+  }
+  __syncthreads();
+}
+
 // Householder QR of the m x k panel in W, m <= LPC RP, k <= 32 / LPC *
 // TTB_WARPS * SL <= 64, in place in LAPACK dgeqr2's layout (see
 // cta_householder).  The warp that owns column j + 1 makes the next reflector
@@ -463,7 +596,13 @@ static __device__ __noinline__ void cta_hh_panel_apply(const double* W, i64 ld, 
                                                        i64 ktop, const int* order) {
 #define TTB_HH_APPLY(L, R, S) \
   hh_columns<L, R, S, FWD>(W, ld, m, p, tau, X, ncols, start, top, kt, ktop, order)
-  TTB_HH_TILE(m, TTB_HH_APPLY)
+  if (ncols <= 32 && m > 32 && m <= 256) {  // one slot holds them all
+    if (m <= 64) TTB_HH_APPLY(8, 8, 1);
+    else if (m <= 128) TTB_HH_APPLY(8, 16, 1);
+    else TTB_HH_APPLY(8, 32, 1);
+  } else {
+    TTB_HH_TILE(m, TTB_HH_APPLY)
+  }
 #undef TTB_HH_APPLY
   __syncthreads();
 }
@@ -497,12 +636,18 @@ static __device__ void cta_hh_apply(const double* W, i64 ld, int m, int p, const
 static __device__ __noinline__ void cta_hh(double* W, i64 ld, int m, int k, double* tau) {
   const int p = m < k ? m : k;
   const int width = hh_width(m);
+  __shared__ double2 vb[3][128];  // hh_panel8's reflectors (here: one copy for its tiles)
+  __shared__ double tb[3];
   for (int j0 = 0; j0 < p; j0 += width) {
     const int cols = min(width, k - j0), rows = m - j0;
     double* P = W + j0 + j0 * ld;
-#define TTB_HH_PANEL(L, R, S) hh_panel<L, R, S>(P, ld, rows, cols, tau + j0)
-    TTB_HH_TILE(rows, TTB_HH_PANEL)
-#undef TTB_HH_PANEL
+    if (rows <= 32) hh_panel8<4, 2>(P, ld, rows, cols, tau + j0, vb, tb);
+    else if (rows <= 64) hh_panel8<8, 2>(P, ld, rows, cols, tau + j0, vb, tb);
+    else if (rows <= 128) hh_panel8<16, 2>(P, ld, rows, cols, tau + j0, vb, tb);
+    else if (rows <= 256) hh_panel8<32, 2>(P, ld, rows, cols, tau + j0, vb, tb);
+    else if (rows <= 512) hh_panel<16, 32, 2>(P, ld, rows, cols, tau + j0);
+    else if (rows <= 1024) hh_panel<32, 32, 2>(P, ld, rows, cols, tau + j0);
+    else hh_panel<32, 64, 1>(P, ld, rows, cols, tau + j0);
     const int rest = k - j0 - cols;
     if (rest > 0)
       cta_hh_panel_apply<true>(P, ld, rows, min(cols, rows), tau + j0,
@@ -510,21 +655,37 @@ static __device__ __noinline__ void cta_hh(double* W, i64 ld, int m, int k, doub
   }
 }
 
+// Rows up to which the register tiles alone factor a matrix in global memory
+// (four columns a warp and step); taller ones take LNB-column panels with
+// the trailing updates as GEMMs.
+constexpr int kHHTall = 512;
+
+// A panel's reflectors: in registers, or row by row beyond their reach.
+template <bool TILED>
+static __device__ __forceinline__ void cta_hh_any(double* W, int m, int k, i64 ld, double* tau,
+                                                  double* red) {
+  if constexpr (TILED) {
+    if (m <= kHHRows) {
+      cta_hh(W, ld, m, k, tau);
+      return;
+    }
+  }
+  cta_householder(W, m, k, ld, tau, red);
+}
+
 // Economic QR of the m x k matrix ``A`` (any strides): Q (m x p) and R
 // (p x k), p = min(m, k).  ``W`` is a column-major work area (unit row step,
 // column step ldw >= m; an odd one spreads a row over the shared-memory
 // banks), ``tau`` p doubles; both may be shared or global memory.  Q and R
 // may be NULL to skip them.
+template <bool TILED>
 __device__ __noinline__ void cta_qr(CMat A, int m, int k, double* W, i64 ldw, double* tau, Mat Q,
-                                    Mat R, double* red, bool tiled) {
+                                    Mat R, double* red) {
   const int p = m < k ? m : k;
   cta_load(A, W, ldw, m, k);
   __syncthreads();
-  const bool tiles = tiled && m <= kHHRows;
-  if (tiles)
-    cta_hh(W, ldw, m, k, tau);
-  else
-    cta_householder(W, m, k, ldw, tau, red);
+  const bool tiles = TILED && m <= kHHRows;
+  cta_hh_any<TILED>(W, m, k, ldw, tau, red);
   if (R.p) {
     for (int e = threadIdx.x; e < p * k; e += TTB_THREADS) {
       int i = e / k, j = e % k;
@@ -533,7 +694,7 @@ __device__ __noinline__ void cta_qr(CMat A, int m, int k, double* W, i64 ldw, do
   }
   if (Q.p) {
     if (tiles) {
-      cta_hh_apply(W, ldw, m, p, tau, Q, p, HH_IDENT);
+      if constexpr (TILED) cta_hh_apply(W, ldw, m, p, tau, Q, p, HH_IDENT);
     } else {
       for (int e = threadIdx.x; e < m * p; e += TTB_THREADS) {
         int i = e % m, j = e / m;
@@ -1210,35 +1371,34 @@ static __device__ void cta_top_u(int k, int m, const double* B, const double* sv
 // order (2 k ints), flag (1 int), tau2 (k).  U (m x k), S (k) and Vh (k x k)
 // are strided outputs.  Returns the Jacobi sweeps used, or -1 if the sweep
 // cap was hit.
+template <bool TILED>
 __device__ __noinline__ int cta_svd_tall(CMat A, int m, int k, double* W, i64 ldw, double* tau,
                                    double* Bsq, double* V, double* sv, int* order, int* flag,
-                                   double* tau2, Mat U, double* S, Mat Vh, double* red,
-                                   bool tiled) {
+                                   double* tau2, Mat U, double* S, Mat Vh, double* red) {
   cta_load(A, W, ldw, m, k);
   __syncthreads();
-  const bool tiles = tiled && m <= kHHRows;
-  if (tiles)
-    cta_hh(W, ldw, m, k, tau);
-  else
-    cta_householder(W, m, k, ldw, tau, red);
-  const i64 ld = tiled ? svd_step(k) : k;
+  const bool tiles = TILED && m <= kHHRows;
+  cta_hh_any<TILED>(W, m, k, ldw, tau, red);
+  const i64 ld = TILED ? svd_step(k) : k;
   for (int e = threadIdx.x; e < k * k; e += TTB_THREADS) {
     int i = e % k, j = e / k;
     Bsq[i + j * ld] = (i <= j) ? W[i + j * ldw] : 0.0;
   }
   __syncthreads();
   const int want = !Vh.p ? SQ_LEFT : !U.p ? SQ_RIGHT : SQ_BOTH;
-  const int status =
-      tiled ? cta_svd_square(want, k, Bsq, V, sv, order, tau2, flag, U, S, Vh, red)
-            : cta_svd_plain(k, Bsq, V, sv, order, flag, S, Vh);
+  int status;
+  if constexpr (TILED)
+    status = cta_svd_square(want, k, Bsq, V, sv, order, tau2, flag, U, S, Vh, red);
+  else
+    status = cta_svd_plain(k, Bsq, V, sv, order, flag, S, Vh);
   if (!U.p) return status;
-  if (!tiled) {
+  if constexpr (!TILED) {
     cta_top_u(k, m, Bsq, sv, order, U);
     cta_apply_q(W, m, k, ldw, tau, U, k);
     return status;
   }
   if (tiles) {
-    cta_hh_apply(W, ldw, m, k, tau, U, k, HH_TOP, V, k, ld, order);
+    if constexpr (TILED) cta_hh_apply(W, ldw, m, k, tau, U, k, HH_TOP, V, k, ld, order);
   } else {
     for (int e = threadIdx.x; e < m * k; e += TTB_THREADS) {
       int i = e % m, r = e / m;
@@ -1664,20 +1824,6 @@ static __device__ __noinline__ int cta_gepp_strips(double* W, i64 ld, double* b,
 // blocked factorisations for matrices that do not fit in shared memory
 // ---------------------------------------------------------------------------
 
-// Rows up to which the register tiles alone factor a matrix in global memory
-// (four columns a warp and step); taller ones take LNB-column panels with
-// the trailing updates as GEMMs.
-constexpr int kHHTall = 512;
-
-// A panel's reflectors: in registers, or row by row beyond their reach.
-static __device__ __forceinline__ void cta_hh_any(double* W, int m, int k, i64 ld, double* tau,
-                                                  double* red, bool tiled) {
-  if (tiled && m <= kHHRows)
-    cta_hh(W, ld, m, k, tau);
-  else
-    cta_householder(W, m, k, ld, tau, red);
-}
-
 
 // Blocked Gaussian elimination with partial pivoting on [W | b] (W column
 // major, leading dimension ld), panels of LNB columns factored in ``panel``
@@ -1828,12 +1974,14 @@ static __device__ void cta_apply_q_blocked(const double* W, int m, int p, const 
 // C -= V (T^T (V^T C)) as two GEMMs through Y (LNB x k, shared).  Q (m x p)
 // and R (p x k) as in cta_qr; either may be NULL.  Same reflectors and R as
 // the unblocked factorisation up to rounding.
+template <bool TILED>
 __device__ __noinline__ void cta_qr_blocked(CMat A, int m, int k, double* W, double* tau, Mat Q, Mat R,
-                               double* Y, double* G, double* Tm, double* red, GemmSmem& gsm, double* ring,
-                               bool tiled) {
-  if (tiled && m <= kHHTall) {
-    cta_qr(A, m, k, W, m, tau, Q, R, red, true);
-    return;
+                               double* Y, double* G, double* Tm, double* red, GemmSmem& gsm, double* ring) {
+  if constexpr (TILED) {
+    if (m <= kHHTall) {
+      cta_qr<true>(A, m, k, W, m, tau, Q, R, red);
+      return;
+    }
   }
   const int p = m < k ? m : k;
   const int tid = threadIdx.x;
@@ -1843,7 +1991,7 @@ __device__ __noinline__ void cta_qr_blocked(CMat A, int m, int k, double* W, dou
     const int jb = min(LNB, p - j0);
     const int rows = m - j0;
     double* Wp = W + j0 + (i64)j0 * m;
-    cta_hh_any(Wp, rows, jb, m, tau + j0, red, tiled);
+    cta_hh_any<TILED>(Wp, rows, jb, m, tau + j0, red);
     // R's diagonal block, then the explicit reflector form in its place
     for (int e = tid; e < jb * jb; e += TTB_THREADS) {
       int r = e % jb, c = e / jb;
@@ -2019,27 +2167,30 @@ __device__ __noinline__ void cta_qr_r_blocked2(CMat A, int m, int k, double* W, 
 // into the global work area W, the SVD of R in Bsq/V (global or shared), U
 // by the reflectors.  Y needs LNB * max(k, 1) doubles, G and Tm LNB * LNB
 // each (shared).
+template <bool TILED>
 __device__ __noinline__ int cta_svd_tall_blocked(CMat A, int m, int k, double* W, double* tau,
                                            double* Bsq, double* V, double* sv, int* order,
                                            int* flag, double* tau2, Mat U, double* S, Mat Vh,
                                            double* Y, double* G, double* Tm, double* red,
-                                           GemmSmem& gsm, double* ring, bool tiled) {
-  const i64 ld = tiled ? svd_step(k) : k;
-  cta_qr_blocked(A, m, k, W, tau, Mat{nullptr, 0, 0}, Mat{Bsq, 1, ld}, Y, G, Tm, red, gsm, ring,
-                 tiled);
+                                           GemmSmem& gsm, double* ring) {
+  const i64 ld = TILED ? svd_step(k) : k;
+  cta_qr_blocked<TILED>(A, m, k, W, tau, Mat{nullptr, 0, 0}, Mat{Bsq, 1, ld}, Y, G, Tm, red, gsm,
+                        ring);
   __syncthreads();
   const int want = !Vh.p ? SQ_LEFT : !U.p ? SQ_RIGHT : SQ_BOTH;
-  const int status =
-      tiled ? cta_svd_square(want, k, Bsq, V, sv, order, tau2, flag, U, S, Vh, red)
-            : cta_svd_plain(k, Bsq, V, sv, order, flag, S, Vh);
+  int status;
+  if constexpr (TILED)
+    status = cta_svd_square(want, k, Bsq, V, sv, order, tau2, flag, U, S, Vh, red);
+  else
+    status = cta_svd_plain(k, Bsq, V, sv, order, flag, S, Vh);
   if (!U.p) return status;
-  if (!tiled) {
+  if constexpr (!TILED) {
     cta_top_u(k, m, Bsq, sv, order, U);
     cta_apply_q_blocked(W, m, k, tau, U, k, Y, G, Tm, gsm, ring);
     return status;
   }
   if (m <= kHHTall) {
-    cta_hh_apply(W, m, m, k, tau, U, k, HH_TOP, V, k, ld, order);
+    if constexpr (TILED) cta_hh_apply(W, m, m, k, tau, U, k, HH_TOP, V, k, ld, order);
     return status;
   }
   for (int e = threadIdx.x; e < m * k; e += TTB_THREADS) {
@@ -2076,7 +2227,7 @@ __device__ __noinline__ void cta_node_factor(CMat A, int rows, int k, double* W,
 
 __device__ __noinline__ void cta_node_apply(const double* W, i64 ld, int rows, int k,
                                             const double* tau, double* smem, const double* top,
-                                            i64 ktop, Mat X) {
+                                            i64 ktop, Mat X, int c0, int nc) {
   const double* F = W;
   i64 lf = ld;
   if (smem) {
@@ -2088,7 +2239,17 @@ __device__ __noinline__ void cta_node_apply(const double* W, i64 ld, int rows, i
     F = smem;
   }
   __syncthreads();
-  cta_hh_apply(F, lf, rows, min(rows, k), tau, X, k, top ? HH_TOP : HH_IDENT, top, k, ktop);
+  const Mat Xc{X.p + c0 * X.cs, X.rs, X.cs};
+  if (top) {
+    cta_hh_apply(F, lf, rows, min(rows, k), tau, Xc, nc, HH_TOP, top + c0 * ktop, k, ktop);
+    return;
+  }
+  for (int e = threadIdx.x; e < rows * nc; e += TTB_THREADS) {
+    const int i = e % rows, c = e / rows;
+    Xc(i, c) = i == c0 + c ? 1.0 : 0.0;
+  }
+  __syncthreads();
+  cta_hh_apply(F, lf, rows, min(rows, k), tau, Xc, nc, HH_X);
 }
 
 __device__ __noinline__ int cta_triangle_svd(const double* R, int k, double* work, Mat Us,
@@ -2109,5 +2270,19 @@ __device__ __noinline__ int cta_triangle_svd(const double* R, int k, double* wor
       top[e] = V[e % k + order[e / k] * ld];
   return status;
 }
+
+#define TTB_FACTOR_INSTANCE(T)                                                                    \
+  template __device__ void cta_qr<T>(CMat, int, int, double*, i64, double*, Mat, Mat, double*);    \
+  template __device__ void cta_qr_blocked<T>(CMat, int, int, double*, double*, Mat, Mat, double*,  \
+                                             double*, double*, double*, GemmSmem&, double*);      \
+  template __device__ int cta_svd_tall<T>(CMat, int, int, double*, i64, double*, double*, double*, \
+                                          double*, int*, int*, double*, Mat, double*, Mat,        \
+                                          double*);                                              \
+  template __device__ int cta_svd_tall_blocked<T>(CMat, int, int, double*, double*, double*,      \
+                                                  double*, double*, int*, int*, double*, Mat,     \
+                                                  double*, Mat, double*, double*, double*,        \
+                                                  double*, GemmSmem&, double*);
+TTB_FACTOR_INSTANCE(true)
+TTB_FACTOR_INSTANCE(false)
 
 }  // namespace ttb

@@ -3,10 +3,10 @@
 // pivoting.  Every thread of the block calls them together; matrices may be
 // in shared or in global memory.
 //
-// ``tiled`` chooses the register-tiled Householder steps and the
+// TILED chooses the register-tiled Householder steps and the
 // preconditioned, register-blocked Jacobi iteration; false takes the
 // column-by-column steps and the plain iteration.  The whole-solve kernel
-// passes false: the rank decisions of its sweeps react to the last digits of
+// takes false: the rank decisions of its sweeps react to the last digits of
 // a factorisation, and its solves are held to recorded trajectories.
 #pragma once
 
@@ -35,21 +35,24 @@ static __device__ __forceinline__ void cta_load(CMat A, double* W, i64 ldw, int 
   }
 }
 
+template <bool TILED>
 __device__ void cta_qr(CMat A, int m, int k, double* W, i64 ldw, double* tau, Mat Q, Mat R,
-                       double* red, bool tiled = true);
+                       double* red);
+template <bool TILED>
 __device__ void cta_qr_blocked(CMat A, int m, int k, double* W, double* tau, Mat Q, Mat R,
                                double* Y, double* G, double* Tm, double* red, GemmSmem& gsm,
-                               double* ring = nullptr, bool tiled = true);
+                               double* ring = nullptr);
 __device__ void cta_qr_r_blocked2(CMat A, int m, int k, double* W, double* tau, Mat R,
                                   double* pool, double* red, double* ring);
+template <bool TILED>
 __device__ int cta_svd_tall(CMat A, int m, int k, double* W, i64 ldw, double* tau, double* Bsq,
                             double* V, double* sv, int* order, int* flag, double* tau2, Mat U,
-                            double* S, Mat Vh, double* red, bool tiled = true);
+                            double* S, Mat Vh, double* red);
+template <bool TILED>
 __device__ int cta_svd_tall_blocked(CMat A, int m, int k, double* W, double* tau, double* Bsq,
                                     double* V, double* sv, int* order, int* flag, double* tau2,
                                     Mat U, double* S, Mat Vh, double* Y, double* G, double* Tm,
-                                    double* red, GemmSmem& gsm, double* ring = nullptr,
-                                    bool tiled = true);
+                                    double* red, GemmSmem& gsm, double* ring = nullptr);
 __device__ int cta_gepp_solve(double* W, i64 ld, double* b, int n, double* lbuf);
 __device__ int cta_gepp_blocked(double* W, i64 ld, double* b, int n, double* panel, double* redv,
                                 int* redi, int* ipiv, GemmSmem& gsm, double* ring = nullptr);
@@ -72,8 +75,8 @@ __host__ __device__ constexpr long long lu_panel_doubles(int n) {
 // cta_node_factor: Householder QR of the rows x k view A (rows <= 2048): the
 // reflectors to W (column step ld, even) and tau, R (k x k, zero rows past
 // ``rows``).  A may be W itself.
-// cta_node_apply: X (rows x k) = the node's Q times [top; 0] (k x k, column
-// step ktop), or times [I; 0] without top.
+// cta_node_apply: columns c0 .. c0 + nc - 1 of X (rows x k) = the node's Q
+// times [top; 0] (k x k, column step ktop), or times [I; 0] without top.
 // cta_triangle_svd: SVD of the k x k upper-triangular R (column step k);
 // ``work`` (triangle_svd_doubles) in any memory, Us a k x k scratch view for
 // the case that both factors are wanted.  Vh may be NULL; ``top`` gets the
@@ -87,7 +90,7 @@ __host__ __device__ constexpr long long triangle_svd_doubles(int k) {
 __device__ void cta_node_factor(CMat A, int rows, int k, double* W, i64 ld, double* tau,
                                 double* smem, Mat R);
 __device__ void cta_node_apply(const double* W, i64 ld, int rows, int k, const double* tau,
-                               double* smem, const double* top, i64 ktop, Mat X);
+                               double* smem, const double* top, i64 ktop, Mat X, int c0, int nc);
 __device__ int cta_triangle_svd(const double* R, int k, double* work, Mat Us, double* S, Mat Vh,
                                 double* top, double* red);
 
