@@ -46,7 +46,8 @@ def test_qr_tile_edges(K, m, k):
 
 @pytest.mark.parametrize("m,k", [(1, 1), (9, 8), (16, 17), (33, 32), (64, 65), (97, 96),
                                  (130, 128), (129, 129), (40, 257), (260, 257), (600, 20),
-                                 (20, 3000)])
+                                 (20, 3000), (100, 300), (193, 200), (390, 385), (513, 512),
+                                 (520, 514)])
 @pytest.mark.parametrize("deficient", [False, True])
 def test_svd_one_factor(K, m, k, deficient):
     """Both factors, the left one alone and the right one alone agree with

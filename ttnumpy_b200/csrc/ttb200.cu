@@ -434,13 +434,13 @@ __host__ __device__ inline i64 blocked_smem(int k) {
 constexpr int kMaxS = 16;
 struct SBatch {
   int count;
-  int mode[kMaxS];  // 0: shared memory, 1: blocked with the work area in global memory
+  int mode[kMaxS];  // 0: shared memory, 1: blocked, W in global memory, 2: with a cluster
   ttb_svd_t d[kMaxS];
 };
 
 // doubles of the tall SVD work area for an M x K (M >= K) problem
 i64 svd_tall_need(int M, int K) {
-  return (i64)odd_step(M) * K + 2 * (i64)svd_step(K) * K + 4 * (i64)K + 6;
+  return (i64)odd_step(M) * K + 2 * (i64)svd_step(K) * K + 4 * (i64)K + 8;
 }
 
 // shared doubles of a blocked SVD with its square matrices in shared memory
@@ -448,7 +448,9 @@ __host__ __device__ inline i64 svd_square_smem(int K) {
   return blocked_smem(K) + 2 * (i64)svd_step(K) * K + 3 * (i64)K + 6;
 }
 
-__global__ void __launch_bounds__(TTB_THREADS) k_svd(const __grid_constant__ SBatch sb) {
+// phase 0: every problem, those of mode 2 up to the Jacobi iteration; 1: the
+// rest of those of mode 2.
+__global__ void __launch_bounds__(TTB_THREADS) k_svd(const __grid_constant__ SBatch sb, int phase) {
   extern __shared__ double dsm[];
   __shared__ double red[TTB_WARPS];
   __shared__ GemmSmem gsm;
@@ -457,12 +459,13 @@ __global__ void __launch_bounds__(TTB_THREADS) k_svd(const __grid_constant__ SBa
   const bool tall = q.m >= q.k;
   const int M = tall ? q.m : q.k, K = tall ? q.k : q.m;
   const int mode = sb.mode[blockIdx.x];
+  if (phase == 1 && mode != 2) return;
   double* W = mode == 0 ? dsm : q.work;
   const int ldw = odd_step(M);
   double* tau = W + (i64)ldw * K;
   // a large W in global memory, the square matrices still shared if they fit
   double* square = tau + K;
-  if (mode != 0 && svd_square_smem(K) * 8 <= kSmemCap) square = dsm + blocked_smem(K);
+  if (mode == 1 && svd_square_smem(K) * 8 <= kSmemCap) square = dsm + blocked_smem(K);
   double* Bsq = align2(square);
   double* V = Bsq + (i64)svd_step(K) * K;
   double* sv = V + (i64)svd_step(K) * K;
@@ -473,17 +476,43 @@ __global__ void __launch_bounds__(TTB_THREADS) k_svd(const __grid_constant__ SBa
   // a^T = U' S Vh'  =>  a = Vh'^T S U'^T : U' goes to vh^T, Vh' to u^T
   Mat U = tall ? Mat{q.u, q.u_rs, q.u_cs} : Mat{q.vh, q.vh_cs, q.vh_rs};
   Mat Vh = tall ? Mat{q.vh, q.vh_rs, q.vh_cs} : Mat{q.u, q.u_cs, q.u_rs};
-  int st;
   if (mode == 0) {
-    st = cta_svd_tall<true>(A, M, K, W, ldw, tau, Bsq, V, sv, order, flag, tau2, U, q.s, Vh, red);
-  } else {
-    double* Y = dsm;
-    double* G = Y + (i64)LNB * min(K, YCH);
-    double* Tm = G + LNB * LNB;
-    st = cta_svd_tall_blocked<true>(A, M, K, W, tau, Bsq, V, sv, order, flag, tau2, U, q.s, Vh, Y, G,
-                              Tm, red, gsm);
+    const int st = cta_svd_tall<true>(A, M, K, W, ldw, tau, Bsq, V, sv, order, flag, tau2, U, q.s,
+                                      Vh, red);
+    if (q.status && threadIdx.x == 0) *q.status = st;
+    return;
   }
-  if (q.status && threadIdx.x == 0) *q.status = st;
+  double* Y = dsm;
+  double* G = Y + (i64)LNB * min(K, YCH);
+  double* Tm = G + LNB * LNB;
+  if (mode == 1) {
+    const int st = cta_svd_tall_blocked<true>(A, M, K, W, tau, Bsq, V, sv, order, flag, tau2, U,
+                                              q.s, Vh, Y, G, Tm, red, gsm);
+    if (q.status && threadIdx.x == 0) *q.status = st;
+  } else if (phase == 0) {
+    cta_svd_before(A, M, K, W, tau, Bsq, V, sv, order, flag, tau2, U, Vh, Y, G, Tm, red, gsm);
+  } else {
+    cta_svd_after(M, K, W, tau, Bsq, V, sv, order, tau2, flag, U, q.s, Vh, Y, G, Tm, red, gsm);
+  }
+}
+
+// The Jacobi iterations of mode-2 problems between the phases of k_svd, a
+// cluster of blocks each.
+constexpr int kSvdCluster = 8;
+__global__ void __cluster_dims__(kSvdCluster, 1, 1) __launch_bounds__(TTB_THREADS, 1)
+    k_svd_cluster(const __grid_constant__ SBatch sb) {
+  const int at = blockIdx.x / kSvdCluster;
+  const ttb_svd_t& q = sb.d[at];
+  if (sb.mode[at] != 2) return;  // the whole cluster
+  const bool tall = q.m >= q.k;
+  const int M = tall ? q.m : q.k, K = tall ? q.k : q.m;
+  double* Bsq = align2(q.work + (i64)odd_step(M) * K + K);
+  double* V = Bsq + (i64)svd_step(K) * K;
+  double* sv = V + (i64)svd_step(K) * K;
+  int* flags = reinterpret_cast<int*>(sv + 3 * K);
+  const int st = cluster_svd_iterate(tall ? q.u != nullptr : q.vh != nullptr,
+                                     tall ? q.vh != nullptr : q.u != nullptr, K, Bsq, V, flags);
+  if (q.status && threadIdx.x == 0 && blockIdx.x % kSvdCluster == 0) *q.status = st;
 }
 
 constexpr int kMaxL = 24;
@@ -1990,6 +2019,7 @@ int ttb_svd(const ttb_svd_t* ps, int count, void* stream) {
     SBatch sb;
     sb.count = std::min(kMaxS, count - i0);
     i64 smem = 0;
+    bool clusters = false;
     for (int j = 0; j < sb.count; ++j) {
       sb.d[j] = ps[i0 + j];
       const i64 whole = svd_tall_need(std::max(sb.d[j].m, sb.d[j].k),
@@ -2000,7 +2030,9 @@ int ttb_svd(const ttb_svd_t* ps, int count, void* stream) {
         smem = std::max(smem, whole);
       } else {
         if (blk > kSmemCap) return (int)cudaErrorInvalidValue;
-        sb.mode[j] = 1;
+        const int k = std::min(sb.d[j].m, sb.d[j].k);
+        sb.mode[j] = k > kClusterMin && k <= kClusterMax ? 2 : 1;
+        clusters = clusters || sb.mode[j] == 2;
         const i64 square = svd_square_smem(std::min(sb.d[j].m, sb.d[j].k)) * 8;
         smem = std::max(smem, square <= kSmemCap ? square : blk);
       }
@@ -2012,8 +2044,14 @@ int ttb_svd(const ttb_svd_t* ps, int count, void* stream) {
       fl += 4.0 * M * k * k - 4.0 / 3.0 * k * k * k;
     }
     ProfScope ps(P_SVD, s, fl, 0.0);
-    k_svd<<<sb.count, TTB_THREADS, (size_t)smem, s>>>(sb);
+    k_svd<<<sb.count, TTB_THREADS, (size_t)smem, s>>>(sb, 0);
     counted();
+    if (clusters) {
+      k_svd_cluster<<<sb.count * kSvdCluster, TTB_THREADS, 0, s>>>(sb);
+      counted();
+      k_svd<<<sb.count, TTB_THREADS, (size_t)smem, s>>>(sb, 1);
+      counted();
+    }
   }
   return last_error();
 }

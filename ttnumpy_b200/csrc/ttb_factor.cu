@@ -12,6 +12,8 @@
 // They are compiled once, here, and called from the kernels of the other
 // files (relocatable device code): inlined into every kernel, ptxas spent
 // minutes on each.
+#include <cooperative_groups.h>
+
 #include "ttb_factor.cuh"
 
 namespace ttb {
@@ -174,16 +176,23 @@ static __device__ __forceinline__ double lane_dot(const double (&x)[RP], const d
 }
 
 // Column ``col`` of a matrix with unit row step, rows below m (zeros beyond).
-template <int LPC, int RP>
+// L2: past the first-level cache, for columns that other SMs write.
+template <int LPC, int RP, bool L2 = false>
 static __device__ __forceinline__ void tile_load(const double* col, int m, double (&x)[RP]) {
   const bool even = (reinterpret_cast<uintptr_t>(col) & 15) == 0;
 #pragma unroll
   for (int r = 0; r < RP; r += 2) {
     const int i = tile_row<LPC>(r);
     if (2 * LPC * (r >> 1) + 2 * LPC <= m && even) {
-      const double2 p = *reinterpret_cast<const double2*>(col + i);
+      const double2* from = reinterpret_cast<const double2*>(col + i);
+      double2 p;
+      if constexpr (L2) p = __ldcg(from);
+      else p = *from;
       x[r] = p.x;
       x[r + 1] = p.y;
+    } else if constexpr (L2) {
+      x[r] = i < m ? __ldcg(col + i) : 0.0;
+      x[r + 1] = i + 1 < m ? __ldcg(col + i + 1) : 0.0;
     } else {
       x[r] = i < m ? col[i] : 0.0;
       x[r + 1] = i + 1 < m ? col[i + 1] : 0.0;
@@ -911,15 +920,18 @@ static __device__ __forceinline__ bool jacobi_angle(double al, double be, double
   return true;
 }
 
-// Two column slots of a warp, x and y: four pairs, one per eight lanes.
-template <int RP>
+// Two column slots of a warp, x and y: G = 32 / LPC pairs, one per lane group.
+template <int LPC, int RP, bool L2>
 struct Pairs {
+  static constexpr int G = 32 / LPC;
   double x[RP], y[RP];
   double nx, ny;  // their squared norms
 
+  static __device__ __forceinline__ int group() { return (threadIdx.x & 31) / LPC; }
+
   __device__ __forceinline__ void norms() {
-    nx = group_sum<8>(lane_dot<RP>(x, x));
-    ny = group_sum<8>(lane_dot<RP>(y, y));
+    nx = group_sum<LPC>(lane_dot<RP>(x, x));
+    ny = group_sum<LPC>(lane_dot<RP>(y, y));
   }
 
   // x <- c x - s y, y <- s x + c y
@@ -932,59 +944,113 @@ struct Pairs {
     }
   }
 
-  // The next pairing.  all: the circle method on the eight columns (the
-  // first x fixed, the others moved round one place: seven steps meet all 28
-  // pairs); else the y columns move round the groups (four steps meet the 16
-  // pairs across).  Either way the last step returns every column to its
-  // place.
-  __device__ __forceinline__ void next(bool all) {
-    const int lane = threadIdx.x & 31, g = lane >> 3;
-    if (all) {
-#pragma unroll
-      for (int r = 0; r < RP; ++r) {
-        const double up = __shfl_sync(0xffffffffu, g == 0 ? y[r] : x[r], (lane + 24) & 31);
-        const double down = __shfl_sync(0xffffffffu, y[r], (lane + 8) & 31);
-        y[r] = g == 3 ? x[r] : down;
-        if (g != 0) x[r] = up;
-      }
-    } else {
-#pragma unroll
-      for (int r = 0; r < RP; ++r) y[r] = __shfl_sync(0xffffffffu, y[r], (lane + 8) & 31);
-    }
+  // The next pairing.  all: the circle method on the 2 G columns (the first x
+  // fixed, the others moved round one place: 2 G - 1 steps meet all pairs);
+  // else the y columns move round the groups (G steps meet the pairs
+  // across).  Either way the last step returns every column to its place.
+  static __device__ __forceinline__ void round_table(double& u, double& v) {
+    const int lane = threadIdx.x & 31, g = group();
+    const double up = __shfl_sync(0xffffffffu, g == 0 ? v : u, (lane + 32 - LPC) & 31);
+    const double down = __shfl_sync(0xffffffffu, v, (lane + LPC) & 31);
+    v = g == G - 1 ? u : down;
+    if (g != 0) u = up;
   }
-
-  __device__ __forceinline__ void next_norms(bool all) {
-    const int lane = threadIdx.x & 31, g = lane >> 3;
-    const double down = __shfl_sync(0xffffffffu, ny, (lane + 8) & 31);
+  __device__ __forceinline__ void next(bool all, bool with_norms) {
     if (all) {
-      const double up = __shfl_sync(0xffffffffu, g == 0 ? ny : nx, (lane + 24) & 31);
-      ny = g == 3 ? nx : down;
-      if (g != 0) nx = up;
+#pragma unroll
+      for (int r = 0; r < RP; ++r) round_table(x[r], y[r]);
+      if (with_norms) round_table(nx, ny);
     } else {
-      ny = down;
+      const int from = ((threadIdx.x & 31) + LPC) & 31;
+#pragma unroll
+      for (int r = 0; r < RP; ++r) y[r] = __shfl_sync(0xffffffffu, y[r], from);
+      if (with_norms) ny = __shfl_sync(0xffffffffu, ny, from);
     }
   }
 
   // Columns ca + group and cb + group of the k x k matrix M (column step
   // ld), zeros beyond it; and back.
   __device__ __forceinline__ void load(const double* M, i64 ld, int k, int ca, int cb) {
-    const int g = (threadIdx.x & 31) >> 3;
-    const int a = ca + g, b = cb + g;
-    tile_load<8, RP>(M + a * ld, a < k ? k : 0, x);
-    tile_load<8, RP>(M + b * ld, b < k ? k : 0, y);
+    const int a = ca + group(), b = cb + group();
+    tile_load<LPC, RP, L2>(M + a * ld, a < k ? k : 0, x);
+    tile_load<LPC, RP, L2>(M + b * ld, b < k ? k : 0, y);
   }
   __device__ __forceinline__ void store(double* M, i64 ld, int k, int ca, int cb) const {
-    const int g = (threadIdx.x & 31) >> 3;
-    const int a = ca + g, b = cb + g;
+    const int a = ca + group(), b = cb + group();
 #pragma unroll
     for (int r = 0; r < RP; ++r) {
-      const int i = tile_row<8>(r);
+      const int i = tile_row<LPC>(r);
       if (i >= k) continue;
-      if (a < k) M[i + a * ld] = x[r];
-      if (b < k) M[i + b * ld] = y[r];
+      if constexpr (L2) {
+        if (a < k) __stcg(M + i + a * ld, x[r]);
+        if (b < k) __stcg(M + i + b * ld, y[r]);
+      } else {
+        if (a < k) M[i + a * ld] = x[r];
+        if (b < k) M[i + b * ld] = y[r];
+      }
     }
   }
 };
+
+// One round of a Jacobi sweep over the block pairs first, first + step, ...:
+// true if any of this warp's pairs was rotated.  See jacobi_blocks.
+template <int LPC, int RP, bool VACC, bool L2>
+static __device__ __forceinline__ bool jacobi_round(double* B, int k, i64 ld, double* V,
+                                                    double tol, int nb, int round, int first,
+                                                    int step) {
+  constexpr bool kRide = VACC && RP <= 16, kReplay = VACC && !kRide;
+  constexpr int G = 32 / LPC;
+  const double tol2 = tol * tol;
+  const bool all = round == 0;
+  const int steps = all ? 2 * G - 1 : G;
+  bool rotated = false;
+  for (int pr = first; pr < nb / 2; pr += step) {
+    const int pa = (pr == 0) ? 0 : ((pr - 1 + round) % (nb - 1)) + 1;
+    const int pb = ((nb - 2 - pr + round) % (nb - 1)) + 1;
+    const int ca = G * min(pa, pb), cb = G * max(pa, pb);
+    Pairs<LPC, RP, L2> p;
+    Pairs<LPC, kRide ? RP : 2, L2> q;
+    double cs[kReplay ? 2 * G - 1 : 1], sn[kReplay ? 2 * G - 1 : 1];
+    p.load(B, ld, k, ca, cb);
+    if constexpr (kRide) q.load(V, ld, k, ca, cb);
+    p.norms();
+    bool turned = false;
+#pragma unroll 1
+    for (int t = 0; t < steps; ++t) {
+      const double ga = group_sum<LPC>(lane_dot<RP>(p.x, p.y));
+      double c, s;
+      const bool rot = jacobi_angle(p.nx, p.ny, ga, tol, tol2, c, s);
+      if (__any_sync(0xffffffffu, rot)) {
+        turned = true;
+        const double tg = ga * s * __drcp_rn(c);
+        p.nx -= tg;
+        p.ny += tg;
+        p.rotate(c, s);
+        if constexpr (kRide) q.rotate(c, s);
+      }
+      if constexpr (kReplay) {
+        cs[t] = c;
+        sn[t] = s;
+      }
+      p.next(all, true);
+      if constexpr (kRide) q.next(all, false);
+    }
+    if (!turned) continue;
+    rotated = true;
+    p.store(B, ld, k, ca, cb);
+    if constexpr (kRide) q.store(V, ld, k, ca, cb);
+    if constexpr (kReplay) {
+      p.load(V, ld, k, ca, cb);
+#pragma unroll 1
+      for (int t = 0; t < steps; ++t) {
+        p.rotate(cs[t], sn[t]);
+        p.next(all, false);
+      }
+      p.store(V, ld, k, ca, cb);
+    }
+  }
+  return rotated;
+}
 
 // Hestenes' one-sided Jacobi on the columns of the k x k matrix B (column
 // step ld; see cta_jacobi, which it replaces up to k = 256) and, with VACC,
@@ -999,70 +1065,21 @@ struct Pairs {
 // round-robin order, one block barrier per meeting: a sweep of 64 columns has
 // 15 barriers and moves the matrices through shared memory 15 times, where
 // pairing single columns took 63.  What bounds a step is its chain (sums,
-// two reciprocal square roots, rotation: about 500 cycles) and, with V, the
+// two reciprocal square roots, rotation: about 900 cycles) and, with V, the
 // issue of FP64 and shuffle instructions.  V rides along in registers up to
 // RP = 16 and is rotated afterwards beyond.
 template <int RP, bool VACC>
 static __device__ __noinline__ int jacobi_blocks(double* B, int k, i64 ld, double* V,
                                                  int max_sweeps, double tol, int* flag) {
-  constexpr bool kRide = VACC && RP <= 16, kReplay = VACC && !kRide;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int nb = ((k + 7) >> 3) << 1, half = nb / 2;
-  const double tol2 = tol * tol;
+  const int nb = ((k + 7) >> 3) << 1;
   for (int sweep = 0; sweep < max_sweeps; ++sweep) {
     __syncthreads();
     if (threadIdx.x == 0) *flag = 0;
     __syncthreads();
     bool rotated = false;
     for (int round = 0; round < nb - 1; ++round) {
-      const bool all = round == 0;
-      const int steps = all ? 7 : 4;
-      for (int pr = warp; pr < half; pr += TTB_WARPS) {
-        const int pa = (pr == 0) ? 0 : ((pr - 1 + round) % (nb - 1)) + 1;
-        const int pb = ((nb - 2 - pr + round) % (nb - 1)) + 1;
-        const int ca = 4 * min(pa, pb), cb = 4 * max(pa, pb);
-        Pairs<RP> p;
-        Pairs<kRide ? RP : 2> q;
-        double cs[kReplay ? 7 : 1], sn[kReplay ? 7 : 1];
-        p.load(B, ld, k, ca, cb);
-        if constexpr (kRide) q.load(V, ld, k, ca, cb);
-        p.norms();
-        bool turned = false;
-#pragma unroll 1
-        for (int t = 0; t < steps; ++t) {
-          const double ga = group_sum<8>(lane_dot<RP>(p.x, p.y));
-          double c, s;
-          const bool rot = jacobi_angle(p.nx, p.ny, ga, tol, tol2, c, s);
-          if (__any_sync(0xffffffffu, rot)) {
-            turned = true;
-            const double tg = ga * s * __drcp_rn(c);
-            p.nx -= tg;
-            p.ny += tg;
-            p.rotate(c, s);
-            if constexpr (kRide) q.rotate(c, s);
-          }
-          if constexpr (kReplay) {
-            cs[t] = c;
-            sn[t] = s;
-          }
-          p.next(all);
-          p.next_norms(all);
-          if constexpr (kRide) q.next(all);
-        }
-        if (!turned) continue;
-        rotated = true;
-        p.store(B, ld, k, ca, cb);
-        if constexpr (kRide) q.store(V, ld, k, ca, cb);
-        if constexpr (kReplay) {
-          p.load(V, ld, k, ca, cb);
-#pragma unroll 1
-          for (int t = 0; t < steps; ++t) {
-            p.rotate(cs[t], sn[t]);
-            p.next(all);
-          }
-          p.store(V, ld, k, ca, cb);
-        }
-      }
+      rotated |= jacobi_round<8, RP, VACC, false>(B, k, ld, V, tol, nb, round, warp, TTB_WARPS);
       __syncthreads();
     }
     if (rotated && lane == 0) *flag = 1;  // benign race: every writer stores 1
@@ -1070,6 +1087,53 @@ static __device__ __noinline__ int jacobi_blocks(double* B, int k, i64 ld, doubl
     if (!*flag) return sweep + 1;
   }
   return -1;
+}
+
+// The same iteration by a cluster of blocks on matrices in global memory: the
+// block pairs of a round are dealt out to the cluster's warps, which meet at
+// a cluster barrier after each round and read and write the columns past
+// their first-level caches.  flags: three ints in global memory, the first
+// zero.  A round of 192 columns is 24 pairs: one per warp of three blocks,
+// where one block had taken them in three turns.  192 x 192 (left factor)
+// took 12.2 ms in one block and takes 4.0 ms, 250 x 250 24.2 and 7.6 ms; up
+// to 96 columns, which shared memory holds, one block is as fast.
+template <int LPC, int RP, bool VACC>
+static __device__ __noinline__ int jacobi_cluster(double* B, int k, i64 ld, double* V,
+                                                  int max_sweeps, double tol, int* flags) {
+  namespace cg = cooperative_groups;
+  cg::cluster_group cl = cg::this_cluster();
+  constexpr int G = 32 / LPC;
+  const int lane = threadIdx.x & 31;
+  const int first = (int)cl.block_rank() * TTB_WARPS + (threadIdx.x >> 5);
+  const int step = (int)cl.num_blocks() * TTB_WARPS;
+  const int nb = 2 * ((k + 2 * G - 1) / (2 * G));
+  auto meet = [&]() {
+    __threadfence();
+    cl.sync();
+    asm volatile("fence.acq_rel.cluster;" ::: "memory");
+  };
+  for (int sweep = 0; sweep < max_sweeps; ++sweep) {
+    // the flag of the next sweep is cleared before this one's last barrier
+    if (cl.block_rank() == 0 && threadIdx.x == 0) __stcg(flags + (sweep + 1) % 3, 0);
+    bool rotated = false;
+    for (int round = 0; round < nb - 1; ++round) {
+      rotated |= jacobi_round<LPC, RP, VACC, true>(B, k, ld, V, tol, nb, round, first, step);
+      if (round == nb - 2 && rotated && lane == 0) __stcg(flags + sweep % 3, 1);
+      meet();
+    }
+    if (!__ldcg(flags + sweep % 3)) return sweep + 1;
+  }
+  return -1;
+}
+
+template <bool VACC>
+static __device__ __forceinline__ int cluster_iterate(double* B, int k, i64 ld, double* V,
+                                                      double tol, int* flags) {
+  if (k <= 128) return jacobi_cluster<8, 16, VACC>(B, k, ld, V, 60, tol, flags);
+  if (k <= 192) return jacobi_cluster<8, 24, VACC>(B, k, ld, V, 60, tol, flags);
+  if (k <= 256) return jacobi_cluster<8, 32, VACC>(B, k, ld, V, 60, tol, flags);
+  if (k <= 384) return jacobi_cluster<16, 24, VACC>(B, k, ld, V, 60, tol, flags);
+  return jacobi_cluster<16, 32, VACC>(B, k, ld, V, 60, tol, flags);
 }
 
 // Orthonormal rows for the singular values that are exactly zero (their rows
@@ -1245,48 +1309,63 @@ static __device__ void cta_apply_square(const double* F, int k, i64 ld, const do
 // SQ_LEFT:  with R2^T J = W S, R = (Q2 W) S (...): the left factor in V; no
 //           rotations are accumulated.
 // SQ_RIGHT: with L J = W S, the right factor (P W)^T is written to Vh.
-// On return V is where the left factor's column of singular value r is
-// V's column order[r].
+//
+// In three parts, so that the iteration can be a cluster's: the matrix X it
+// works on and the factors F (of Q2, or the accumulated rotations) are Bsq
+// and V in the order square_roles gives.  At the end the left factor's column
+// of singular value r is column order[r] of square_left.
 enum { SQ_BOTH = 0, SQ_LEFT = 1, SQ_RIGHT = 2 };
-static __device__ __noinline__ int cta_svd_square(int want, int k, double* Bsq, double*& V,
-                                                  double* sv, int* order, double* tau2, int* flag,
-                                                  Mat Us, double* S, Mat Vh, double* red) {
-  int* perm = order + k;
-  const double tol = 2.0 * sqrt((double)k) * 2.220446049250313e-16;
+static __device__ __forceinline__ void square_roles(int want, int k, double* Bsq, double* V,
+                                                    double*& F, double*& X) {
+  const bool first = (k <= kPivotMax) != (want == SQ_BOTH);
+  F = first ? Bsq : V;
+  X = first ? V : Bsq;
+}
+static __device__ __forceinline__ double square_tol(int k) {
+  return 2.0 * sqrt((double)k) * 2.220446049250313e-16;
+}
+
+static __device__ __noinline__ void square_prepare(int want, int k, double* Bsq, double* V,
+                                                   double* sv, int* order, double* tau2, Mat Us,
+                                                   double* red) {
   const i64 ld = svd_step(k);
   double *F = Bsq, *X = V;
-  cta_pivoted(F, X, k, ld, perm, sv, tau2, red);
+  cta_pivoted(F, X, k, ld, order + k, sv, tau2, red);
   if (want == SQ_BOTH) {
     cta_apply_square(F, k, ld, tau2, Us, HH_IDENT);  // Q2, explicit
     cta_transpose_upper(F, F, k, ld);                // L takes the factors' place
     for (int e = threadIdx.x; e < k * k; e += TTB_THREADS) X[e % k + (e / k) * ld] = Us(e % k, e / k);
     __syncthreads();
-    double* t = F;  // F: the accumulated rotations, X: the iterated matrix
-    F = X;
-    X = t;
-  } else {
-    cta_transpose_upper(F, X, k, ld);
-    if (want == SQ_LEFT) {
-      // (sv is free until the columns are sorted: the second QR's scalars)
-      if (k <= kHHRows)
-        cta_hh(X, ld, k, k, sv);
-      else
-        cta_householder(X, k, k, ld, sv, red);
-      cta_transpose_upper(X, X, k, ld);
-    }
+    return;
   }
-  int status;
-  if (k > kJacobiMax) {
-    if (want != SQ_BOTH) {  // the rotations accumulated there go nowhere: F's are kept apart
-      status = cta_jacobi(X, k, ld, nullptr, 0, 60, tol, flag);
-    } else {
-      status = cta_jacobi(X, k, ld, F, ld, 60, tol, flag);
-    }
-  } else if (want == SQ_BOTH) {
-    status = cta_jacobi_blocks<true>(X, k, ld, F, 60, tol, flag);
-  } else {
-    status = cta_jacobi_blocks<false>(X, k, ld, nullptr, 60, tol, flag);
-  }
+  cta_transpose_upper(F, X, k, ld);
+  if (want != SQ_LEFT) return;
+  // (sv is free until the columns are sorted: the second QR's scalars)
+  if (k <= kHHRows)
+    cta_hh(X, ld, k, k, sv);
+  else
+    cta_householder(X, k, k, ld, sv, red);
+  cta_transpose_upper(X, X, k, ld);
+}
+
+static __device__ __noinline__ int square_iterate(int want, int k, double* Bsq, double* V,
+                                                  int* flag) {
+  const i64 ld = svd_step(k);
+  double *F, *X;
+  square_roles(want, k, Bsq, V, F, X);
+  const double tol = square_tol(k);
+  if (k > kJacobiMax) return cta_jacobi(X, k, ld, want == SQ_BOTH ? F : nullptr, ld, 60, tol, flag);
+  if (want == SQ_BOTH) return cta_jacobi_blocks<true>(X, k, ld, F, 60, tol, flag);
+  return cta_jacobi_blocks<false>(X, k, ld, nullptr, 60, tol, flag);
+}
+
+static __device__ __noinline__ void square_finish(int want, int k, double* Bsq, double* V,
+                                                  double* sv, int* order, double* tau2, int* flag,
+                                                  double* S, Mat Vh, double* red) {
+  const i64 ld = svd_step(k);
+  const int* perm = order + k;
+  double *F, *X;
+  square_roles(want, k, Bsq, V, F, X);
   cta_sort_columns(X, k, ld, sv, order, flag);
   for (int r = threadIdx.x; r < k; r += TTB_THREADS) S[r] = sv[order[r]];
   if (want == SQ_LEFT) {
@@ -1298,8 +1377,7 @@ static __device__ __noinline__ int cta_svd_square(int want, int k, double* Bsq, 
     __syncthreads();
     if (*flag) cta_complete_rows(k, sv, order, order, Mat{X, ld, 1}, red);
     cta_apply_square(F, k, ld, tau2, Mat{X, 1, ld}, HH_X);
-    V = X;
-    return status;
+    return;
   }
   for (int e = threadIdx.x; e < k * k; e += TTB_THREADS) {
     const int r = e / k, c = e % k, j = order[r];
@@ -1307,7 +1385,21 @@ static __device__ __noinline__ int cta_svd_square(int want, int k, double* Bsq, 
   }
   __syncthreads();
   if (*flag) cta_complete_rows(k, sv, nullptr, order, Vh, red);
-  V = F;
+}
+
+static __device__ __forceinline__ double* square_left(int want, int k, double* Bsq, double* V) {
+  double *F, *X;
+  square_roles(want, k, Bsq, V, F, X);
+  return want == SQ_LEFT ? X : F;
+}
+
+static __device__ __noinline__ int cta_svd_square(int want, int k, double* Bsq, double*& V,
+                                                  double* sv, int* order, double* tau2, int* flag,
+                                                  Mat Us, double* S, Mat Vh, double* red) {
+  square_prepare(want, k, Bsq, V, sv, order, tau2, Us, red);
+  const int status = square_iterate(want, k, Bsq, V, flag);
+  square_finish(want, k, Bsq, V, sv, order, tau2, flag, S, Vh, red);
+  V = square_left(want, k, Bsq, V);
   return status;
 }
 
@@ -2200,6 +2292,52 @@ __device__ __noinline__ int cta_svd_tall_blocked(CMat A, int m, int k, double* W
   __syncthreads();
   cta_apply_q_blocked(W, m, k, tau, U, k, Y, G, Tm, gsm, ring);
   return status;
+}
+
+// cta_svd_tall_blocked with the iteration left to a cluster in between:
+// everything in global memory.
+__device__ __noinline__ void cta_svd_before(CMat A, int m, int k, double* W, double* tau,
+                                            double* Bsq, double* V, double* sv, int* order,
+                                            int* flags, double* tau2, Mat U, Mat Vh, double* Y,
+                                            double* G, double* Tm, double* red, GemmSmem& gsm) {
+  cta_qr_blocked<true>(A, m, k, W, tau, Mat{nullptr, 0, 0}, Mat{Bsq, 1, svd_step(k)}, Y, G, Tm,
+                       red, gsm, nullptr);
+  __syncthreads();
+  const int want = !Vh.p ? SQ_LEFT : !U.p ? SQ_RIGHT : SQ_BOTH;
+  square_prepare(want, k, Bsq, V, sv, order, tau2, U, red);
+  if (threadIdx.x == 0) flags[0] = 0;
+}
+
+__device__ __noinline__ int cluster_svd_iterate(bool left, bool right, int k, double* Bsq,
+                                                double* V, int* flags) {
+  const int want = !right ? SQ_LEFT : !left ? SQ_RIGHT : SQ_BOTH;
+  const i64 ld = svd_step(k);
+  double *F, *X;
+  square_roles(want, k, Bsq, V, F, X);
+  const double tol = square_tol(k);
+  return want == SQ_BOTH ? cluster_iterate<true>(X, k, ld, F, tol, flags)
+                         : cluster_iterate<false>(X, k, ld, nullptr, tol, flags);
+}
+
+__device__ __noinline__ void cta_svd_after(int m, int k, double* W, double* tau, double* Bsq,
+                                           double* V, double* sv, int* order, double* tau2,
+                                           int* flag, Mat U, double* S, Mat Vh, double* Y,
+                                           double* G, double* Tm, double* red, GemmSmem& gsm) {
+  const i64 ld = svd_step(k);
+  const int want = !Vh.p ? SQ_LEFT : !U.p ? SQ_RIGHT : SQ_BOTH;
+  square_finish(want, k, Bsq, V, sv, order, tau2, flag, S, Vh, red);
+  if (!U.p) return;
+  const double* top = square_left(want, k, Bsq, V);
+  if (m <= kHHTall) {
+    cta_hh_apply(W, m, m, k, tau, U, k, HH_TOP, top, k, ld, order);
+    return;
+  }
+  for (int e = threadIdx.x; e < m * k; e += TTB_THREADS) {
+    int i = e % m, r = e / m;
+    U(i, r) = i < k ? top[i + order[r] * ld] : 0.0;
+  }
+  __syncthreads();
+  cta_apply_q_blocked(W, m, k, tau, U, k, Y, G, Tm, gsm, nullptr);
 }
 
 // ---------------------------------------------------------------------------

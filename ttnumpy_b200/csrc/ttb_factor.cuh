@@ -53,6 +53,22 @@ __device__ int cta_svd_tall_blocked(CMat A, int m, int k, double* W, double* tau
                                     double* V, double* sv, int* order, int* flag, double* tau2,
                                     Mat U, double* S, Mat Vh, double* Y, double* G, double* Tm,
                                     double* red, GemmSmem& gsm, double* ring = nullptr);
+
+// cta_svd_tall_blocked in three kernels for large k (kClusterMin < k <=
+// kClusterMax): before the Jacobi iteration, the iteration by a cluster of
+// blocks (returns the sweeps, -1 at the cap), and after it; every matrix in
+// global memory, flags three ints there.
+constexpr int kClusterMin = 96, kClusterMax = 512;
+__device__ void cta_svd_before(CMat A, int m, int k, double* W, double* tau, double* Bsq,
+                               double* V, double* sv, int* order, int* flags, double* tau2, Mat U,
+                               Mat Vh, double* Y, double* G, double* Tm, double* red,
+                               GemmSmem& gsm);
+__device__ int cluster_svd_iterate(bool left, bool right, int k, double* Bsq, double* V,
+                                   int* flags);
+__device__ void cta_svd_after(int m, int k, double* W, double* tau, double* Bsq, double* V,
+                              double* sv, int* order, double* tau2, int* flag, Mat U, double* S,
+                              Mat Vh, double* Y, double* G, double* Tm, double* red,
+                              GemmSmem& gsm);
 __device__ int cta_gepp_solve(double* W, i64 ld, double* b, int n, double* lbuf);
 __device__ int cta_gepp_blocked(double* W, i64 ld, double* b, int n, double* panel, double* redv,
                                 int* redi, int* ipiv, GemmSmem& gsm, double* ring = nullptr);
