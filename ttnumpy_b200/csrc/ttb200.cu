@@ -596,7 +596,7 @@ constexpr int kTreeProblems = 16;
 // in one block, 256 x 64 (where one block's tile ends) 0.21 ms.
 int tree_block(int K) { return K <= 96 ? 256 : 512; }
 bool tree_shape(int M, int K) {
-  return M >= kTreeRows && M > tree_block(K) && M < (1 << 28) && K >= 1 && K <= kTreeCols &&
+  return M > kTreeRows && M > tree_block(K) && M < (1 << 28) && K >= 1 && K <= kTreeCols &&
          M >= 3 * K;
 }
 
