@@ -145,13 +145,14 @@ __device__ double vnorm_diff(const double* x, const double* y, i64 n, double* re
 // A solve may run on a cluster of blocks: block 0 (the leader) runs the
 // whole solve as a lone block would, and posts each product large enough
 // (a tiled GEMM of two or more output tiles, a sparse operator-core product)
-// as a command in its shared memory; the other blocks read it over
+// and the steps of an elimination (the local matrix, a panel's update) as a
+// command in its shared memory; the other blocks read it over
 // distributed shared memory and compute their share of the output tiles
 // (tiles rank, rank + csize, ...) or rows, each exactly as the lone block
 // computes it, so the solve's results do not depend on the cluster size.  A
 // command is bracketed by two cluster barriers (posted; done); the leader
 // ends every solve, normally or on an error, with the exit command.
-enum { CL_EXIT = 0, CL_GEMM = 1, CL_SPMM = 2, CL_VEC = 3 };
+enum { CL_EXIT = 0, CL_GEMM = 1, CL_SPMM = 2, CL_VEC = 3, CL_LOCAL = 4, CL_LU = 5 };
 
 // The element-wise passes of a MINRES iteration on long vectors run in
 // kVecChunks fixed chunks, each reduced by one block-wide sum; the chunk
@@ -290,6 +291,10 @@ __device__ __noinline__ double vpass_chunk(const VecArgs& q, int chunk, double* 
   return block_sum(acc, red);
 }
 
+struct LocalDims {  // of a local operator: bonds and modes
+  int lt, lf, R, R2, n, m, rt, rf;
+};
+
 struct ClusterCmd {
   int op;
   VecArgs vec;
@@ -306,7 +311,14 @@ struct ClusterCmd {
   const int* sp_col;
   const double* sp_val;
   int sp_rows, sp_nnz, sp_cols;
+  // CL_LOCAL: a, b, sp_val the left environment, core and right environment,
+  // c the matrix; CL_LU: c the matrix, rhs, M unknowns, the panel at K
+  LocalDims dim;
+  double* rhs;
+  int ipiv[LNB];
 };
+static_assert(sizeof(ClusterCmd) % 8 == 0 && sizeof(ClusterCmd) / 8 <= TTB_THREADS,
+              "a command is read in one step");
 
 __device__ __forceinline__ void cluster_barrier() {
   cooperative_groups::this_cluster().sync();  // arrive.release + wait.acquire
@@ -815,6 +827,8 @@ struct LocalOp {
   const double* rightP;  // right re-laid out as [b, p, q] (permute_op)
   SpOp sx, sp;           // op's sparse forms SP_X and SP_P (permute_op), if any
   int lt, lf, R, R2, n, m, rt, rf;
+
+  __device__ LocalDims dims() const { return LocalDims{lt, lf, R, R2, n, m, rt, rf}; }
 };
 
 __device__ LocalOp local_A(Ctx& c, int k) {
@@ -1000,31 +1014,20 @@ __device__ __noinline__ void svd(Ctx& c, CMat A, int m, int k, Mat U, double* S,
 // ---------------------------------------------------------------------------
 
 // Explicit local matrix (column major, n x n) and GEPP solve; u <- solution.
-__device__ __noinline__ void direct_solve(Ctx& c, const LocalOp& L, const double* b, double* u) {
-  const i64 N = (i64)L.lf * L.n * L.rf;
-  const i64 mark = c.top;
-  Sm* s = c.sm;
-  double* W;
-  double* panel = c.pool;  // the blocked elimination's panel (N x LNB)
-  const bool small = N * N + N <= kPoolD;  // in the pool and in registers
-  if (small) {
-    W = c.pool;
-  } else {
-    W = take(c, N * N);
-    if (lu_panel_doubles((int)N) > kPoolD) panel = take(c, N * LNB);  // in the slab
-    if (c.status) return;
-  }
-  // Explicit local matrix, column major.  An item is a row (j, kr, nf) and the
-  // part (l, mt) of a column: the operator core times the right environment
-  // gives one number per left operator bond, kept in registers while the
-  // item's lt columns (i, l, mt) are formed.  Consecutive threads take
-  // consecutive rows.  (A thread walking a whole row re-read core and
-  // environment for every entry and left the threads past N idle: as long as
-  // the elimination itself on the QTT systems.)
-  const int Nn = (int)N;
+// Explicit local matrix, column major: the items rank, rank + size, ... of
+// the blocks of a cluster.  An item is a row (j, kr, nf) and the part (l, mt)
+// of a column: the operator core times the right environment gives one number
+// per left operator bond, kept in registers while the item's lt columns (i, l,
+// mt) are formed.  Consecutive threads take consecutive rows.  (A thread
+// walking a whole row re-read core and environment for every entry and left
+// the threads past N idle: as long as the elimination itself on the QTT
+// systems.)
+__device__ __noinline__ void form_local(const double* lenv, const double* core, const double* renv,
+                                        const LocalDims& L, double* W, int rank, int size) {
+  const int Nn = L.lf * L.n * L.rf;
   constexpr int kRegs = 8;  // left operator bonds held in registers at a time
   const int items = Nn * L.m * L.rt;
-  for (int e = threadIdx.x; e < items; e += TTB_THREADS) {
+  for (int e = rank * TTB_THREADS + threadIdx.x; e < items; e += size * TTB_THREADS) {
     const int row = e % Nn, q = e / Nn, mt = q % L.rt, l = q / L.rt;
     const int nf = row % L.rf, kr = (row / L.rf) % L.n, j = row / (L.rf * L.n);
     for (int a0 = 0; a0 < L.R; a0 += kRegs) {
@@ -1033,11 +1036,11 @@ __device__ __noinline__ void direct_solve(Ctx& c, const LocalOp& L, const double
       for (int a = 0; a < kRegs; ++a) {
         t[a] = 0.0;
         if (a0 + a >= L.R) continue;
-        const double* op = L.op + (((i64)(a0 + a) * L.n + kr) * L.m + l) * L.R2;
-        const double* right = L.right + (i64)mt * L.R2 * L.rf + nf;
+        const double* op = core + (((i64)(a0 + a) * L.n + kr) * L.m + l) * L.R2;
+        const double* right = renv + (i64)mt * L.R2 * L.rf + nf;
         for (int bb = 0; bb < L.R2; ++bb) t[a] = fma(op[bb], right[(i64)bb * L.rf], t[a]);
       }
-      const double* left = L.left + (i64)a0 * L.lf + j;
+      const double* left = lenv + (i64)a0 * L.lf + j;
       double* w = W + row + ((i64)l * L.rt + mt) * Nn;
       for (int i = 0; i < L.lt; ++i) {
         double acc = a0 ? *w : 0.0;
@@ -1053,11 +1056,76 @@ __device__ __noinline__ void direct_solve(Ctx& c, const LocalOp& L, const double
       }
     }
   }
+}
+
+// Trailing columns from which a panel's update is worth two cluster barriers
+// and a read of the panel by every block.
+constexpr int kLuShare = 96;
+
+// cta_gepp_blocked with the strips of each panel's update shared out; W and b
+// in global memory, n <= kLuRows, every entry as a lone block computes it.
+__device__ __noinline__ int cluster_gepp(Ctx& c, double* W, double* b, int n) {
+  ClusterCmd& q = *c.cmd;
+  for (int j0 = 0; j0 < n; j0 += LNB) {
+    if (const int info = cta_gepp_panel(W, n, n, j0, c.pool, q.ipiv)) return info;
+    if (n - j0 - LNB < kLuShare) {
+      cta_gepp_update(W, n, b, n, j0, c.pool, q.ipiv, false, 0, 1);
+      continue;
+    }
+    if (threadIdx.x == 0) {
+      q.op = CL_LU;
+      q.c = W;
+      q.rhs = b;
+      q.M = n;
+      q.K = j0;
+    }
+    cluster_barrier();  // posted
+    cta_gepp_update(W, n, b, n, j0, c.pool, q.ipiv, false, 0, c.csize);
+    cluster_barrier();  // every strip is written
+  }
+  cta_back_substitute(W, n, b, n);
+  return 0;
+}
+
+__device__ __noinline__ void direct_solve(Ctx& c, const LocalOp& L, const double* b, double* u) {
+  const i64 N = (i64)L.lf * L.n * L.rf;
+  const i64 mark = c.top;
+  Sm* s = c.sm;
+  double* W;
+  double* panel = c.pool;  // the blocked elimination's panel (N x LNB)
+  const bool small = N * N + N <= kPoolD;  // in the pool and in registers
+  if (small) {
+    W = c.pool;
+  } else {
+    W = take(c, N * N);
+    if (lu_panel_doubles((int)N) > kPoolD) panel = take(c, N * LNB);  // in the slab
+    if (c.status) return;
+  }
+  // A cluster forms and eliminates the matrices of the slab together (a
+  // quarter of a mode-32 diffusion solve while the leader did it alone: eight
+  // such solves on eight blocks each 739 -> 626 ms).
+  const bool shared = c.csize > 1 && !small && N <= kLuRows && panel == c.pool;
+  if (shared) {
+    if (threadIdx.x == 0) {
+      ClusterCmd& q = *c.cmd;
+      q.op = CL_LOCAL;
+      q.a = L.left;
+      q.b = L.op;
+      q.sp_val = L.right;
+      q.c = W;
+      q.dim = L.dims();
+    }
+    cluster_barrier();
+  }
+  form_local(L.left, L.op, L.right, L.dims(), W, 0, shared ? c.csize : 1);
+  if (shared) cluster_barrier();
   vcopy(u, b, N);
   __syncthreads();
   int info;
   if (small)
     info = cta_gepp_solve(W, N, u, (int)N, c.ring);
+  else if (shared)
+    info = cluster_gepp(c, W, u, (int)N);
   else
     info = cta_gepp_blocked(W, N, u, (int)N, panel, s->red, s->redi, s->ipiv, *c.gsm, c.ring);
   __syncthreads();
@@ -2445,9 +2513,13 @@ __global__ void __launch_bounds__(TTB_THREADS, 1)
 // A cluster's worker block: run the leader's commands until the exit one.
 // ``lead`` is the leader's command slot (distributed shared memory).
 __device__ __noinline__ void cluster_worker(Ctx& c, const ClusterCmd* lead, int rank) {
+  __shared__ ClusterCmd q;
   for (;;) {
     cluster_barrier();  // a command is posted
-    ClusterCmd q = *lead;
+    if (threadIdx.x < sizeof(ClusterCmd) / 8)
+      reinterpret_cast<unsigned long long*>(&q)[threadIdx.x] =
+          reinterpret_cast<const unsigned long long*>(lead)[threadIdx.x];
+    __syncthreads();
     if (q.op == CL_EXIT) {
       cluster_barrier();  // the leader's shared memory stays until every block has read
       return;
@@ -2460,6 +2532,10 @@ __device__ __noinline__ void cluster_worker(Ctx& c, const ClusterCmd* lead, int 
         const double v = vpass_chunk(q.vec, k, c.sm->red);
         if (threadIdx.x == 0) c.vpart[k] = v;
       }
+    } else if (q.op == CL_LOCAL) {
+      form_local(q.a, q.b, q.sp_val, q.dim, q.c, rank, c.csize);
+    } else if (q.op == CL_LU) {
+      cta_gepp_update(q.c, q.M, q.rhs, q.M, q.K, c.pool, q.ipiv, true, rank, c.csize);
     } else {
       const int tw = q.b_cs == 1 ? spmm_tile(q.sp_rows, q.sp_nnz, q.sp_cols) : 0;
       if (tw > 0)

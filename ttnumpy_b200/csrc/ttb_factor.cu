@@ -1625,7 +1625,7 @@ static __device__ __forceinline__ int lu_steps(double (&x)[CPW][RPL], int (&pos)
 // blocks of 32 columns: one warp the diagonal block, every thread the rows
 // above it.  Each row sees the columns last to first, one fma each, as a
 // column-by-column substitution takes them.
-static __device__ __noinline__ void cta_back_substitute(const double* W, i64 ld, double* b,
+__device__ __noinline__ void cta_back_substitute(const double* W, i64 ld, double* b,
                                                         int n) {
   const int lane = threadIdx.x & 31;
   for (int j0 = ((n - 1) / 32) * 32; j0 >= 0; j0 -= 32) {
@@ -1747,166 +1747,194 @@ static __device__ __noinline__ int lu_panel(double* W, i64 ld, int rows, int jb,
 
 // cta_gepp_solve for a matrix in global memory, kLuWhole < n <= kLuRows,
 // panels of LNB columns; ``pool`` (shared) holds lu_panel_doubles(n).  Per
-// panel: the panel in registers (lu_panel); then the trailing columns, a
-// strip at a time: row swaps as one permutation of the at most 32 rows they
-// touch, the unit-lower solve with a thread per column, both into shared
-// memory, and C -= L21 U12 on the FP64 tensor path with C loaded straight
-// into the accumulator fragments' lanes, 32 x 16 entries a warp.  Every entry
-// sees the products and roundings of the plain blocked form (cta_gepp_blocked)
-// in the same order.  The floor on one SM is 2 n^3 / 3 flops at 128 a cycle
-// (2.1 ms for 928 unknowns); 928 unknowns took 27.4 ms with one synchronised
-// tile at a time and take 10.7 ms, half of it waiting for C.
-static __device__ __noinline__ int cta_gepp_strips(double* W, i64 ld, double* b, int n,
-                                                   double* pool) {
-  __shared__ int piv[2], ipiv[LNB], nmove, src[2 * LNB], dst[2 * LNB];
+// panel: the panel in registers (cta_gepp_panel); then the trailing columns, a
+// strip at a time (cta_gepp_update): row swaps as one permutation of the at
+// most 32 rows they touch, the unit-lower solve with a thread per column, both
+// into shared memory, and C -= L21 U12 on the FP64 tensor path with C loaded
+// straight into the accumulator fragments' lanes, 32 x 16 entries a warp.
+// Every entry sees the products and roundings of the plain blocked form
+// (cta_gepp_blocked) in the same order, whatever the strips.  The floor on one
+// SM is 2 n^3 / 3 flops at 128 a cycle (2.1 ms for 928 unknowns); 928 unknowns
+// took 27.4 ms with one synchronised tile at a time and take 10.7 ms, half of
+// it waiting for C, so a cluster deals out the strips.
+//
+// The panel at j0: factored in place, a copy in the pool for cta_gepp_update,
+// its row swaps in ``ipiv`` (shared, LNB).  Returns 0 or the first zero pivot.
+__device__ __noinline__ int cta_gepp_panel(double* W, i64 ld, int n, int j0, double* pool,
+                                           int* ipiv) {
+  __shared__ int piv[2];
+  const int jb = min(LNB, n - j0), rows = n - j0, pp = lu_pitch(rows);
+  double* Wp = W + j0 + j0 * ld;
+  int info;
+  if (rows <= 128) info = lu_panel<4>(Wp, ld, rows, jb, pool, pp, pool, piv, ipiv);
+  else if (rows <= 256) info = lu_panel<8>(Wp, ld, rows, jb, pool, pp, pool, piv, ipiv);
+  else if (rows <= 512) info = lu_panel<16>(Wp, ld, rows, jb, pool, pp, pool, piv, ipiv);
+  else info = lu_panel<32>(Wp, ld, rows, jb, pool, pp, pool, piv, ipiv);
+  return info ? j0 + info : 0;
+}
+
+// The trailing columns and b under the panel at j0: the strips rank, rank +
+// size, ...; ``fetch`` reads the panel from W first (a block that did not
+// factor it).
+__device__ __noinline__ void cta_gepp_update(double* W, i64 ld, double* b, int n, int j0,
+                                             double* pool, const int* ipiv, bool fetch, int rank,
+                                             int size) {
+  __shared__ int nmove, src[2 * LNB], dst[2 * LNB];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int g = lane >> 2, t = lane & 3;
-  double* lbuf = pool;                      // the panel's multipliers ...
-  double* P = pool;                         // ... then the panel, row pitch pp
-  double* Us = pool + LNB * lu_pitch(n);    // U12's strip, LNB x kLuStripPitch
-  for (int j0 = 0; j0 < n; j0 += LNB) {
-    const int jb = min(LNB, n - j0), rows = n - j0, pp = lu_pitch(rows);
-    double* Wp = W + j0 + j0 * ld;
-    int info;
-    if (rows <= 128) info = lu_panel<4>(Wp, ld, rows, jb, P, pp, lbuf, piv, ipiv);
-    else if (rows <= 256) info = lu_panel<8>(Wp, ld, rows, jb, P, pp, lbuf, piv, ipiv);
-    else if (rows <= 512) info = lu_panel<16>(Wp, ld, rows, jb, P, pp, lbuf, piv, ipiv);
-    else info = lu_panel<32>(Wp, ld, rows, jb, P, pp, lbuf, piv, ipiv);
-    if (info) return j0 + info;
-    // the swaps as moves: position dst[e] gets the row that was at src[e]
-    if (tid == 0) {
-      int cnt = 0;
-      for (int c = 0; c < jb; ++c) {
-        const int q = ipiv[c];
-        int ec = -1, eq = -1;
-        for (int e = 0; e < cnt; ++e) {
-          if (dst[e] == c) ec = e;
-          if (dst[e] == q) eq = e;
-        }
-        if (ec < 0) { ec = cnt++; dst[ec] = src[ec] = c; }
-        if (q == c) continue;
-        if (eq < 0) { eq = cnt++; dst[eq] = src[eq] = q; }
-        const int v = src[ec];
-        src[ec] = src[eq];
-        src[eq] = v;
-      }
-      nmove = cnt;
+  const int jb = min(LNB, n - j0), rows = n - j0, pp = lu_pitch(rows);
+  double* P = pool;                       // the panel, row pitch pp
+  double* Us = pool + LNB * lu_pitch(n);  // U12's strip, LNB x kLuStripPitch
+  double* Wp = W + j0 + j0 * ld;
+  const int ncols = n - j0 - jb;  // trailing columns; b comes after them
+  // a strip per block where there are that many columns, in tiles of 16
+  const int strip = min(kLuStrip, ((ncols + size) / size + 15) & ~15);
+  if (fetch)
+    for (int e = tid; e < jb * rows; e += TTB_THREADS) {
+      const int c = e / rows, i = e % rows;
+      P[c * pp + i] = Wp[i + c * ld];
     }
-    // zero rows below the panel, so that the products need no row test
-    for (int e = tid; e < LNB * (pp - rows); e += TTB_THREADS) {
-      const int c = e / (pp - rows), i = rows + e % (pp - rows);
-      P[c * pp + i] = 0.0;
+  // the swaps as moves: position dst[e] gets the row that was at src[e]
+  if (tid == 0) {
+    int cnt = 0;
+    for (int c = 0; c < jb; ++c) {
+      const int q = ipiv[c];
+      int ec = -1, eq = -1;
+      for (int e = 0; e < cnt; ++e) {
+        if (dst[e] == c) ec = e;
+        if (dst[e] == q) eq = e;
+      }
+      if (ec < 0) { ec = cnt++; dst[ec] = src[ec] = c; }
+      if (q == c) continue;
+      if (eq < 0) { eq = cnt++; dst[eq] = src[eq] = q; }
+      const int v = src[ec];
+      src[ec] = src[eq];
+      src[eq] = v;
+    }
+    nmove = cnt;
+  }
+  // zero rows below the panel, so that the products need no row test
+  for (int e = tid; e < LNB * (pp - rows); e += TTB_THREADS) {
+    const int c = e / (pp - rows), i = rows + e % (pp - rows);
+    P[c * pp + i] = 0.0;
+  }
+  if (jb < LNB)
+    for (int e = tid; e < (LNB - jb) * pp; e += TTB_THREADS) P[jb * pp + e] = 0.0;
+  __syncthreads();
+  const int cnt = nmove;
+  for (int s0 = rank * strip; s0 <= ncols; s0 += size * strip) {
+    const int sn = min(strip, ncols + 1 - s0);
+    // swaps: four columns of a warp in flight
+    for (int c4 = 4 * warp; c4 < sn; c4 += 4 * TTB_WARPS) {
+      double v[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int c = s0 + c4 + u;
+        const double* col = c < ncols ? Wp + (jb + c) * ld : b + j0;
+        v[u] = (c4 + u < sn && lane < cnt) ? col[src[lane]] : 0.0;
+      }
+      __syncwarp();
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int c = s0 + c4 + u;
+        double* col = c < ncols ? Wp + (jb + c) * ld : b + j0;
+        if (c4 + u >= sn || lane >= cnt) continue;
+        const int to = dst[lane];
+        if (to < jb) Us[to * kLuStripPitch + c4 + u] = v[u];
+        else col[to] = v[u];
+      }
     }
     if (jb < LNB)
-      for (int e = tid; e < (LNB - jb) * pp; e += TTB_THREADS) P[jb * pp + e] = 0.0;
+      for (int e = tid; e < (LNB - jb) * sn; e += TTB_THREADS)
+        Us[(jb + e / sn) * kLuStripPitch + e % sn] = 0.0;
     __syncthreads();
-    const int cnt = nmove;
-    const int ncols = n - j0 - jb;  // trailing columns; b comes after them
-    for (int s0 = 0; s0 <= ncols; s0 += kLuStrip) {
-      const int sn = min(kLuStrip, ncols + 1 - s0);
-      // swaps: four columns of a warp in flight
-      for (int c4 = 4 * warp; c4 < sn; c4 += 4 * TTB_WARPS) {
-        double v[4];
+    // the unit-lower solve, a thread per column
+    for (int c = tid; c < sn; c += TTB_THREADS) {
+      double y[LNB];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const int c = s0 + c4 + u;
-          const double* col = c < ncols ? Wp + (jb + c) * ld : b + j0;
-          v[u] = (c4 + u < sn && lane < cnt) ? col[src[lane]] : 0.0;
-        }
-        __syncwarp();
+      for (int r = 0; r < LNB; ++r) {
+        y[r] = Us[r * kLuStripPitch + c];
+        double acc = y[r];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const int c = s0 + c4 + u;
-          double* col = c < ncols ? Wp + (jb + c) * ld : b + j0;
-          if (c4 + u >= sn || lane >= cnt) continue;
-          const int to = dst[lane];
-          if (to < jb) Us[to * kLuStripPitch + c4 + u] = v[u];
-          else col[to] = v[u];
-        }
+        for (int q = 0; q < r; ++q) acc = fma(-P[q * pp + r], y[q], acc);
+        y[r] = r < jb ? acc : 0.0;
+        Us[r * kLuStripPitch + c] = y[r];
       }
-      if (jb < LNB)
-        for (int e = tid; e < (LNB - jb) * sn; e += TTB_THREADS)
-          Us[(jb + e / sn) * kLuStripPitch + e % sn] = 0.0;
-      __syncthreads();
-      // the unit-lower solve, a thread per column
-      for (int c = tid; c < sn; c += TTB_THREADS) {
-        double y[LNB];
+    }
+    __syncthreads();
+    for (int e = tid; e < sn * LNB; e += TTB_THREADS) {
+      const int r = e % LNB, c = e / LNB;
+      double* col = s0 + c < ncols ? Wp + (jb + s0 + c) * ld : b + j0;
+      if (r < jb) col[r] = Us[r * kLuStripPitch + c];
+    }
+    // C -= L21 U12, b2 -= L21 u_b
+    const int below = rows - jb, wide = min(sn, ncols - s0);
+    const int tm = (below + 31) / 32, tn = (wide + 15) / 16;
+    if (below > 0 && wide > 0) {
+      for (int tile = warp; tile < tm * tn; tile += TTB_WARPS) {
+        const int m0 = jb + (tile % tm) * 32, n0 = (tile / tm) * 16;
+        double c0[4][2][2], acc[4][2][2];
+        double* cp[2][2];
 #pragma unroll
-        for (int r = 0; r < LNB; ++r) {
-          y[r] = Us[r * kLuStripPitch + c];
-          double acc = y[r];
+        for (int j = 0; j < 2; ++j)
 #pragma unroll
-          for (int q = 0; q < r; ++q) acc = fma(-P[q * pp + r], y[q], acc);
-          y[r] = r < jb ? acc : 0.0;
-          Us[r * kLuStripPitch + c] = y[r];
-        }
-      }
-      __syncthreads();
-      for (int e = tid; e < sn * LNB; e += TTB_THREADS) {
-        const int r = e % LNB, c = e / LNB;
-        double* col = s0 + c < ncols ? Wp + (jb + s0 + c) * ld : b + j0;
-        if (r < jb) col[r] = Us[r * kLuStripPitch + c];
-      }
-      // C -= L21 U12, b2 -= L21 u_b
-      const int below = rows - jb, wide = min(sn, ncols - s0);
-      const int tm = (below + 31) / 32, tn = (wide + 15) / 16;
-      if (below > 0 && wide > 0) {
-        for (int tile = warp; tile < tm * tn; tile += TTB_WARPS) {
-          const int m0 = jb + (tile % tm) * 32, n0 = (tile / tm) * 16;
-          double c0[4][2][2], acc[4][2][2];
-          double* cp[2][2];
-#pragma unroll
-          for (int j = 0; j < 2; ++j)
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-              const int cc = n0 + 8 * j + 2 * t + h;
-              cp[j][h] = cc < wide ? Wp + (jb + s0 + cc) * ld : nullptr;
-#pragma unroll
-              for (int i = 0; i < 4; ++i) {
-                const int r = m0 + 8 * i + g;
-                acc[i][j][h] = 0.0;
-                c0[i][j][h] = (cp[j][h] && r < rows) ? cp[j][h][r] : 0.0;
-              }
-            }
-#pragma unroll
-          for (int kk = 0; kk < LNB; kk += 4) {
-            if (kk >= jb) break;
-            double av[4], bv[2];
+          for (int h = 0; h < 2; ++h) {
+            const int cc = n0 + 8 * j + 2 * t + h;
+            cp[j][h] = cc < wide ? Wp + (jb + s0 + cc) * ld : nullptr;
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
               const int r = m0 + 8 * i + g;
-              av[i] = r < pp ? P[(kk + t) * pp + r] : 0.0;
+              acc[i][j][h] = 0.0;
+              c0[i][j][h] = (cp[j][h] && r < rows) ? cp[j][h][r] : 0.0;
             }
-#pragma unroll
-            for (int j = 0; j < 2; ++j) bv[j] = Us[(kk + t) * kLuStripPitch + n0 + 8 * j + g];
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-              for (int j = 0; j < 2; ++j) dmma_8x8x4(acc[i][j][0], acc[i][j][1], av[i], bv[j]);
           }
 #pragma unroll
-          for (int j = 0; j < 2; ++j)
+        for (int kk = 0; kk < LNB; kk += 4) {
+          if (kk >= jb) break;
+          double av[4], bv[2];
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
-              if (!cp[j][h]) continue;
+          for (int i = 0; i < 4; ++i) {
+            const int r = m0 + 8 * i + g;
+            av[i] = r < pp ? P[(kk + t) * pp + r] : 0.0;
+          }
 #pragma unroll
-              for (int i = 0; i < 4; ++i) {
-                const int r = m0 + 8 * i + g;
-                if (r < rows) cp[j][h][r] = fma(1.0, c0[i][j][h], -1.0 * acc[i][j][h]);
-              }
+          for (int j = 0; j < 2; ++j) bv[j] = Us[(kk + t) * kLuStripPitch + n0 + 8 * j + g];
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < 2; ++j) dmma_8x8x4(acc[i][j][0], acc[i][j][1], av[i], bv[j]);
+        }
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            if (!cp[j][h]) continue;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              const int r = m0 + 8 * i + g;
+              if (r < rows) cp[j][h][r] = fma(1.0, c0[i][j][h], -1.0 * acc[i][j][h]);
             }
-        }
+          }
       }
-      if (s0 + sn > ncols) {  // this strip holds b, in its last column
-        for (int i = tid; i < below; i += TTB_THREADS) {
-          double acc = b[j0 + jb + i];
-          for (int q = 0; q < jb; ++q)
-            acc = fma(-P[q * pp + jb + i], Us[q * kLuStripPitch + sn - 1], acc);
-          b[j0 + jb + i] = acc;
-        }
-      }
-      __syncthreads();  // the strip's reads are done
     }
+    if (s0 + sn > ncols) {  // this strip holds b, in its last column
+      for (int i = tid; i < below; i += TTB_THREADS) {
+        double acc = b[j0 + jb + i];
+        for (int q = 0; q < jb; ++q)
+          acc = fma(-P[q * pp + jb + i], Us[q * kLuStripPitch + sn - 1], acc);
+        b[j0 + jb + i] = acc;
+      }
+    }
+    __syncthreads();  // the strip's reads are done
+  }
+}
+
+static __device__ __noinline__ int cta_gepp_strips(double* W, i64 ld, double* b, int n,
+                                                   double* pool) {
+  __shared__ int ipiv[LNB];
+  for (int j0 = 0; j0 < n; j0 += LNB) {
+    if (const int info = cta_gepp_panel(W, ld, n, j0, pool, ipiv)) return info;
+    cta_gepp_update(W, ld, b, n, j0, pool, ipiv, false, 0, 1);
   }
   cta_back_substitute(W, ld, b, n);
   return 0;

@@ -86,6 +86,14 @@ __host__ __device__ constexpr long long lu_panel_doubles(int n) {
   return n <= kLuRows ? LNB * (lu_pitch(n) + kLuStripPitch) : (long long)n * LNB;
 }
 
+// The steps of cta_gepp_blocked for n <= kLuRows (see there): for j0 = 0, LNB,
+// ...: the panel, then its update (every block of a cluster, ``fetch`` where
+// the panel was factored by another); at the end the back substitution.
+__device__ int cta_gepp_panel(double* W, i64 ld, int n, int j0, double* pool, int* ipiv);
+__device__ void cta_gepp_update(double* W, i64 ld, double* b, int n, int j0, double* pool,
+                                const int* ipiv, bool fetch, int rank, int size);
+__device__ void cta_back_substitute(const double* W, i64 ld, double* b, int n);
+
 // Nodes of a tree of factorisations.  ``smem`` (may be NULL) holds node_smem
 // doubles and is where the node's columns live meanwhile.
 // cta_node_factor: Householder QR of the rows x k view A (rows <= 2048): the

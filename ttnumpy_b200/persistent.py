@@ -405,6 +405,31 @@ def cluster_size(p: "_Prepared") -> int:
     return 4 if max(p.modes) >= 64 else 1
 
 
+# Largest cluster a batch is spread over by itself.
+SPREAD_MOST = 8
+
+
+def spread(count: int, sms: int) -> int:
+    """Thread blocks per solve of a batch of ``count`` that leaves
+    multiprocessors idle: the largest power of two up to ``SPREAD_MOST`` that
+    keeps the batch on half of the ``sms``, the other half staying free for
+    other streams.
+
+    A lone block is bound by one multiprocessor's FP64 and L2 rates; a
+    cluster shares out its products, eliminations and long vector passes,
+    each block computing its share as the lone block would, so results are
+    the same bits.  Eight 4-dimensional diffusion solves on 1 / 2 / 8 blocks
+    each: mode 32 960 / 766 / 626 ms, mode 16 186 / 163 / 140 ms; 5
+    dimensions of mode 8 123 / 103 / 85 ms; 32 Poisson systems on trains of
+    mode 2 68 / 61 ms on 1 / 2.  Past the multiprocessors clusters wait for
+    one another: 36 solves of mode 32 took 1156 ms alone, 992 ms in pairs
+    and 1213 ms in fours."""
+    size = 1
+    while size < SPREAD_MOST and 4 * size * count <= sms:
+        size *= 2
+    return size
+
+
 def _cost(p: "_Prepared") -> float:
     """Relative cost estimate of a solve for the launch order: the local
     apply grows like n^3 R^2 at the bonds such problems reach, times d."""
@@ -425,14 +450,17 @@ def amen_persistent(requests: Sequence, rmax: int = 64, max_rmax: int = 256,
     whose bonds outgrow ``rmax`` are re-run with twice the capacity.  With
     ``time_limit`` (seconds) a solve still running after that long on the
     device stops with status -6; with ``cluster`` > 1 every solve runs on a
-    cluster of that many thread blocks (same results)."""
+    cluster of that many thread blocks, and a batch that leaves the device
+    idle is spread over clusters by itself (``spread``; same results)."""
     K.device_ok()
     preps = prepare(requests)
+    sms = torch.cuda.get_device_properties("cuda").multi_processor_count
     results: List[Optional[Result]] = [None] * len(preps)
     todo = list(range(len(preps)))
     while todo:
-        out = PersistentBatch([preps[i] for i in todo], rmax, time_limit=time_limit,
-                              cluster=cluster).run(stream)
+        batch = [preps[i] for i in todo]
+        out = PersistentBatch(batch, rmax, time_limit=time_limit,
+                              cluster=cluster if cluster > 1 else spread(len(batch), sms)).run(stream)
         retry = []
         for i, res in zip(todo, out):
             if res.status == -4 and rmax < max_rmax:
