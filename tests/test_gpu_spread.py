@@ -14,16 +14,17 @@ def test_spread_keeps_half_of_the_device(count, size):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("direct", [150, 511, 1024])
-def test_spread_equals_lone_blocks(direct):
-    """Products, vector passes and eliminations shared out (also of the
-    smallest and largest systems that are) give the same bits."""
+@pytest.mark.parametrize("mode,direct", [(21, 150), (21, 511), (21, 1024), (32, 1000)])
+def test_spread_equals_lone_blocks(mode, direct):
+    """Products, vector passes, eliminations (also of the smallest and largest
+    systems that are shared) and the residual norm's tall factorisations give
+    the same bits on a cluster."""
     from ttnumpy_b200 import problems
 
     kw = dict(residual_tol=1e-8, symmetric=True, max_sweeps=5, seed=0, stagnation_factor=None,
               direct_solve_size=direct, kickrank=3)
     theta = np.array([0.3, -0.7, 0.5, 0.9])
-    probs = [problems.parametric_diffusion(4, 21, theta), problems.qtt_poisson_2d(7)]
+    probs = [problems.parametric_diffusion(4, mode, theta), problems.qtt_poisson_2d(7)]
     reqs = [(p.A, p.b, None, kw) for p in probs]
     lone = P.PersistentBatch(P.prepare(reqs), 64, cluster=1).run()
     for a, b in zip(lone, P.amen_persistent(reqs)):

@@ -152,7 +152,8 @@ __device__ double vnorm_diff(const double* x, const double* y, i64 n, double* re
 // computes it, so the solve's results do not depend on the cluster size.  A
 // command is bracketed by two cluster barriers (posted; done); the leader
 // ends every solve, normally or on an error, with the exit command.
-enum { CL_EXIT = 0, CL_GEMM = 1, CL_SPMM = 2, CL_VEC = 3, CL_LOCAL = 4, CL_LU = 5 };
+enum { CL_EXIT = 0, CL_GEMM = 1, CL_SPMM = 2, CL_VEC = 3, CL_LOCAL = 4, CL_LU = 5,
+       CL_QR = 6 };
 
 // The element-wise passes of a MINRES iteration on long vectors run in
 // kVecChunks fixed chunks, each reduced by one block-wide sum; the chunk
@@ -312,7 +313,8 @@ struct ClusterCmd {
   const double* sp_val;
   int sp_rows, sp_nnz, sp_cols;
   // CL_LOCAL: a, b, sp_val the left environment, core and right environment,
-  // c the matrix; CL_LU: c the matrix, rhs, M unknowns, the panel at K
+  // c the matrix; CL_LU: c the matrix, rhs, M unknowns, the panel at K; CL_QR:
+  // a the M x N matrix, c its work area, rhs the reflectors' scalars
   LocalDims dim;
   double* rhs;
   int ipiv[LNB];
@@ -931,6 +933,11 @@ __device__ __noinline__ void project(Ctx& c, const double* left, int a, int i, c
 // ---------------------------------------------------------------------------
 
 // Economic QR of the m x k view A: Q (m x p) and R (p x k) strided outputs.
+// Rows from which a cluster shares the residual norm's factorisations (eight
+// mode-32 diffusion solves on eight blocks each: 626 ms, shared 606 ms); below,
+// the two barriers a column cost as much as a lone block's pass over it.
+constexpr int kQrShare = 1024;
+
 __device__ __noinline__ void qr(Ctx& c, CMat A, int m, int k, Mat Q, Mat R) {
   const int p = min(m, k);
   if ((i64)m * k + p <= kPoolD) {
@@ -942,7 +949,24 @@ __device__ __noinline__ void qr(Ctx& c, CMat A, int m, int k, Mat Q, Mat R) {
   if (c.status) return;
   if (!Q.p && p > LNB2 && m >= 4 * k) {
     // R only of a tall matrix (the residual norm sweep): two-level blocking
-    cta_qr_r_blocked2(A, m, k, W, W + (i64)m * k, R, c.pool, c.sm->red, c.ring);
+    const bool shared = c.csize > 1 && m >= kQrShare && !__isShared(A.p);
+    if (shared) {
+      if (threadIdx.x == 0) {
+        ClusterCmd& q = *c.cmd;
+        q.op = CL_QR;
+        q.a = A.p;
+        q.a_rs = A.rs;
+        q.a_cs = A.cs;
+        q.M = m;
+        q.N = k;
+        q.c = W;
+        q.rhs = W + (i64)m * k;
+      }
+      cluster_barrier();
+    }
+    cta_qr_r_blocked2(A, m, k, W, W + (i64)m * k, R, c.pool, c.sm->red, c.ring, 0,
+                      shared ? c.csize : 1);
+    if (shared) cluster_barrier();
     if (c.T->debug & 1) {
       // the one-level blocked factorisation of the same matrix, compared
       double* R1 = take(c, (i64)p * k);
@@ -2536,6 +2560,9 @@ __device__ __noinline__ void cluster_worker(Ctx& c, const ClusterCmd* lead, int 
       form_local(q.a, q.b, q.sp_val, q.dim, q.c, rank, c.csize);
     } else if (q.op == CL_LU) {
       cta_gepp_update(q.c, q.M, q.rhs, q.M, q.K, c.pool, q.ipiv, true, rank, c.csize);
+    } else if (q.op == CL_QR) {
+      cta_qr_r_blocked2(CMat{q.a, q.a_rs, q.a_cs}, q.M, q.N, q.c, q.rhs, Mat{nullptr, 0, 0},
+                        c.pool, c.sm->red, c.ring, rank, c.csize);
     } else {
       const int tw = q.b_cs == 1 ? spmm_tile(q.sp_rows, q.sp_nnz, q.sp_cols) : 0;
       if (tw > 0)

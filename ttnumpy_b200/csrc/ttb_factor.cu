@@ -2163,6 +2163,133 @@ __device__ __noinline__ void cta_qr_blocked(CMat A, int m, int k, double* W, dou
   __syncthreads();
 }
 
+// Every block of a cluster of ``size`` at a point, its global writes visible
+// to the others; one block: its threads.
+static __device__ __forceinline__ void team_sync(int size) {
+  if (size > 1) {
+    cooperative_groups::this_cluster().sync();
+    asm volatile("fence.acq_rel.cluster;" ::: "memory");
+  } else {
+    __syncthreads();
+  }
+}
+
+// cta_householder of a panel (k <= LNB) by the blocks of a cluster, every
+// entry and sum as the lone block computes it: that block's warp ``vw`` takes
+// the rows j + 1 + 32 vw + lane + TTB_THREADS i of a step, so block ``rank``
+// takes the rows of the warps rank, rank + size, ..., its own warps two
+// columns each, and the warps' partial sums go to every block.  Two cluster
+// barriers a column.  A lone block reads and writes the panel through one
+// multiprocessor's path to L2: 6400 x 16 is 13 us a column there.
+static __device__ __noinline__ void team_householder(double* W, int m, int k, i64 ldw, double* tau,
+                                                     int rank, int size) {
+  static_assert(LNB <= 2 * TTB_WARPS, "two columns a warp");
+  constexpr int U = 8;  // rows of a lane in flight
+  __shared__ double hred[TTB_WARPS][LNB], nred[TTB_WARPS], hw[LNB];
+  cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  const int p = min(m, k);
+  for (int vw = rank; vw < TTB_WARPS; vw += size) {
+    if (wid != vw / size) continue;
+    double part = 0.0;
+#pragma unroll 8
+    for (int i = 1 + 32 * vw + lane; i < m; i += TTB_THREADS) part = fma(W[i], W[i], part);
+    part = warp_sum(part);
+    if (lane < size) *cl.map_shared_rank(&nred[vw], lane) = part;
+  }
+  team_sync(size);
+  for (int j = 0; j < p; ++j) {
+    double sigma = 0.0;
+    for (int w = 0; w < TTB_WARPS; ++w) sigma += nred[w];
+    double* col = W + j * ldw;
+    double* cb = col + ldw;
+    const int nc = k - j - 1;
+    const double alpha = col[j];
+    const double rowj = tid < nc ? cb[j + tid * ldw] : 0.0;
+    double t = 0.0, beta = alpha, scale = 0.0;
+    if (sigma != 0.0) {
+      const double nrm = sqrt(alpha * alpha + sigma);
+      beta = (alpha >= 0.0) ? -nrm : nrm;
+      t = (beta - alpha) / beta;
+      scale = 1.0 / (alpha - beta);
+      for (int vw = rank; vw < TTB_WARPS; vw += size)
+        for (int i = j + 1 + 32 * vw + lane + TTB_THREADS * wid; i < m;
+             i += TTB_THREADS * TTB_WARPS)
+          col[i] *= scale;
+    }
+    __syncthreads();
+    const int q0 = wid, q1 = wid + TTB_WARPS;  // this warp's columns
+    const double* c0 = cb + q0 * ldw;
+    const double* c1 = cb + q1 * ldw;
+    if (t != 0.0 && q0 < nc) {
+      for (int vw = rank; vw < TTB_WARPS; vw += size) {
+        double w0 = 0.0, w1 = 0.0;
+#pragma unroll 8
+        for (int i = j + 1 + 32 * vw + lane; i < m; i += TTB_THREADS) {
+          const double v = col[i];
+          w0 = fma(v, c0[i], w0);
+          if (q1 < nc) w1 = fma(v, c1[i], w1);
+        }
+        w0 = warp_sum(w0);
+        w1 = warp_sum(w1);
+        if (lane < size) {
+          double* to = cl.map_shared_rank(&hred[vw][0], lane);
+          to[q0] = w0;
+          if (q1 < nc) to[q1] = w1;
+        }
+      }
+    }
+    team_sync(size);  // the sums are in; alpha and row j are read
+    if (rank == 0 && tid == 0) {
+      col[j] = beta;
+      tau[j] = t;
+    }
+    if (t != 0.0) {
+      if (tid < nc) {
+        double sw = 0.0;
+        for (int w = 0; w < TTB_WARPS; ++w) sw += hred[w][tid];
+        const double wv = t * (sw + rowj);
+        hw[tid] = wv;
+        if (rank == 0) cb[j + tid * ldw] = rowj - wv;
+      }
+      __syncthreads();
+    }
+    for (int vw = rank; vw < TTB_WARPS; vw += size) {
+      double next = 0.0;  // of |column j + 1, rows > j + 1|^2, by warp 0
+      if (t != 0.0 && q0 < nc) {
+        const double h0 = -hw[q0], h1 = q1 < nc ? -hw[q1] : 0.0;
+        for (int i0 = j + 1 + 32 * vw + lane; i0 < m; i0 += U * TTB_THREADS) {
+          double v[U], x0[U], x1[U];
+#pragma unroll
+          for (int u = 0; u < U; ++u) {
+            const int i = i0 + u * TTB_THREADS;
+            v[u] = i < m ? col[i] : 0.0;
+            x0[u] = i < m ? c0[i] : 0.0;
+            x1[u] = (i < m && q1 < nc) ? c1[i] : 0.0;
+          }
+#pragma unroll
+          for (int u = 0; u < U; ++u) {
+            const int i = i0 + u * TTB_THREADS;
+            if (i >= m) continue;
+            const double x = fma(h0, v[u], x0[u]);
+            cb[i + q0 * ldw] = x;
+            if (q1 < nc) cb[i + q1 * ldw] = fma(h1, v[u], x1[u]);
+            if (q0 == 0 && i > j + 1) next = fma(x, x, next);
+          }
+        }
+      } else if (nc > 0 && wid == 0) {
+        for (int i = j + 2 + 32 * vw + lane; i < m; i += TTB_THREADS)
+          next = fma(cb[i], cb[i], next);
+      }
+      if (wid == 0) {
+        next = warp_sum(next);
+        if (lane < size) *cl.map_shared_rank(&nred[vw], lane) = next;
+      }
+    }
+    team_sync(size);  // the panel and the next norm are complete
+  }
+}
+
 // R factor only of the economic QR of the m x k view A, two-level blocked
 // for tall operands: outer panels of LNB2 columns are factorised by the
 // LNB-blocked Householder code (trailing updates inside the panel only),
@@ -2170,10 +2297,13 @@ __device__ __noinline__ void cta_qr_blocked(CMat A, int m, int k, double* W, dou
 // compact-WY block, C -= V (T^T (V^T C)), whose products have 64-wide tiles
 // and long K.  Same reflectors as cta_qr_blocked.  W (m x k column major)
 // and tau (min(m, k)) are global work; ``pool`` (shared) holds
-// 2 LNB2^2 + LNB2^2 + LNB * LNB2 + 2 LNB^2 doubles.
+// 2 LNB2^2 + LNB2^2 + LNB * LNB2 + 2 LNB^2 doubles.  The blocks of a cluster
+// may call it together (A, W, tau in global memory, R the leader's): they
+// share the inner panels' reflectors and take the outer updates a chunk of
+// LNB2 columns each, with the lone block's bits.
 __device__ __noinline__ void cta_qr_r_blocked2(CMat A, int m, int k, double* W, double* tau,
                                                       Mat R, double* pool, double* red,
-                                                      double* ring) {
+                                                      double* ring, int rank, int size) {
   const int p = m < k ? m : k;
   const int tid = threadIdx.x;
   double* G2 = pool;                      // LNB2 x LNB2: V^T V, later T^T Y
@@ -2182,8 +2312,11 @@ __device__ __noinline__ void cta_qr_r_blocked2(CMat A, int m, int k, double* W, 
   double* Yi = Yo + LNB2 * LNB2;          // LNB x LNB2 (inner updates)
   double* Gi = Yi + LNB * LNB2;
   double* Ti = Gi + LNB * LNB;
-  cta_load(A, W, m, m, k);
-  __syncthreads();
+  {
+    const int l0 = (int)((i64)k * rank / size), l1 = (int)((i64)k * (rank + 1) / size);
+    cta_load(CMat{A.p + l0 * A.cs, A.rs, A.cs}, W + (i64)l0 * m, m, m, l1 - l0);
+  }
+  team_sync(size);
   for (int o0 = 0; o0 < p; o0 += LNB2) {
     const int ob = min(LNB2, p - o0);
     const int orows = m - o0;
@@ -2193,7 +2326,15 @@ __device__ __noinline__ void cta_qr_r_blocked2(CMat A, int m, int k, double* W, 
       const int jb = min(LNB, o0 + ob - j0);
       const int rows = m - j0;
       double* Wp = W + j0 + (i64)j0 * m;
-      cta_householder(Wp, rows, jb, m, tau + j0, red);
+      if (size > 1) {
+        team_householder(Wp, rows, jb, m, tau + j0, rank, size);
+        if (rank > 0) {
+          team_sync(size);  // the leader updates the outer panel
+          continue;
+        }
+      } else {
+        cta_householder(Wp, rows, jb, m, tau + j0, red);
+      }
       for (int e = tid; e < jb * jb; e += TTB_THREADS) {
         int r = e % jb, c = e / jb;
         if (r <= c) {
@@ -2234,16 +2375,17 @@ __device__ __noinline__ void cta_qr_r_blocked2(CMat A, int m, int k, double* W, 
         cta_gemm_pipe(CMat{Wp, 1, m}, CMat{Yi, 1, LNB}, Mat{C, 1, m}, rows, nt, jb, -1.0, 1.0,
                       ring);
       }
+      if (size > 1) team_sync(size);
     }
     // R entries above the inner diagonal blocks move out; V gets zeros there
-    for (int e = tid; e < ob * ob; e += TTB_THREADS) {
+    for (int e = tid; rank == 0 && e < ob * ob; e += TTB_THREADS) {
       int r = e % ob, c = e / ob;
       if (r < c && (r / LNB) != (c / LNB)) {
         R(o0 + r, o0 + c) = Wo[r + (i64)c * m];
         Wo[r + (i64)c * m] = 0.0;
       }
     }
-    __syncthreads();
+    team_sync(size);
     const int nt = k - o0 - ob;
     if (nt <= 0) continue;
     // T of the panel: T[i, i] = tau_i, T[0:i, i] = -tau_i T[0:i, 0:i] (V^T V)[0:i, i]
@@ -2260,7 +2402,7 @@ __device__ __noinline__ void cta_qr_r_blocked2(CMat A, int m, int k, double* W, 
       if (tid == 0) T2[i + i * LNB2] = ti;
       __syncthreads();
     }
-    for (int c0 = 0; c0 < nt; c0 += LNB2) {
+    for (int c0 = rank * LNB2; c0 < nt; c0 += size * LNB2) {
       const int nc = min(LNB2, nt - c0);
       double* C = W + o0 + (i64)(o0 + ob + c0) * m;
       // Yo = V^T C, G2 = T^T Yo, C -= V G2
@@ -2270,9 +2412,10 @@ __device__ __noinline__ void cta_qr_r_blocked2(CMat A, int m, int k, double* W, 
       cta_gemm_pipe(CMat{Wo, 1, m}, CMat{G2, 1, LNB2}, Mat{C, 1, m}, orows, nc, ob, -1.0, 1.0,
                     ring);
     }
+    if (size > 1) team_sync(size);
   }
   // the rest of R: below the diagonal zero, right of each outer panel from W
-  for (int e = tid; e < p * k; e += TTB_THREADS) {
+  for (int e = tid; rank == 0 && e < p * k; e += TTB_THREADS) {
     int i = e % p, j = e / p;
     if (i > j) {
       R(i, j) = 0.0;

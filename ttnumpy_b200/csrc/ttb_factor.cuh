@@ -43,7 +43,8 @@ __device__ void cta_qr_blocked(CMat A, int m, int k, double* W, double* tau, Mat
                                double* Y, double* G, double* Tm, double* red, GemmSmem& gsm,
                                double* ring = nullptr);
 __device__ void cta_qr_r_blocked2(CMat A, int m, int k, double* W, double* tau, Mat R,
-                                  double* pool, double* red, double* ring);
+                                  double* pool, double* red, double* ring, int rank = 0,
+                                  int size = 1);
 template <bool TILED>
 __device__ int cta_svd_tall(CMat A, int m, int k, double* W, i64 ldw, double* tau, double* Bsq,
                             double* V, double* sv, int* order, int* flag, double* tau2, Mat U,
