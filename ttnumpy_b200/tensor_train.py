@@ -829,8 +829,8 @@ def round_in_one_launch(cores: List[torch.Tensor], error: float,
     launch: the left QR sweep and the right SVD sweep with every rank
     decision on the device, the bonds read back once.  Core by core the same
     sweeps are four to seven launches and a read-back per bond: 16 cores of
-    mode 2 and bond 10 take 3.2 ms that way and 1.6 ms in one launch, 8 cores
-    of mode 4 and bond 64 3.8 and 3.6 ms (the limit of what fits is also where
+    mode 2 and bond 10 take 2.8 ms that way and 1.5 ms in one launch, 8 cores
+    of mode 4 and bond 64 3.6 and 3.4 ms (the limit of what fits is also where
     the two meet).  None if the train does not fit, or if the iteration did
     not converge."""
     d = len(cores)
