@@ -554,7 +554,7 @@ __global__ void __launch_bounds__(TTB_THREADS) k_lu(const __grid_constant__ LBat
 // reflectors to the k x k block its parent gives it.  One thread block alone
 // is bound by its own column chain and memory traffic over all rows (3072 x
 // 96 with Q: 13.9 ms); a tree's chain is one node of a few hundred rows per
-// level.
+// level (1.9 ms).
 constexpr int kTreeLevels = 24;  // 2^23 row blocks, halved at least at every level
 struct Tree {
   const double* a;       // M x K view (K <= kTreeCols)
@@ -592,12 +592,12 @@ constexpr int kTreeSlice = 32;  // columns of Q a block takes on the way down
 // with a block each.
 constexpr int kTreeProblems = 16;
 
-// Tall enough that two levels of blocks beat one block: 512 x 96 takes 0.69 ms
-// in one block, 256 x 64 (where one block's tile ends) 0.21 ms.
+// Rows of a leaf; and tall enough that two levels of blocks beat one block's
+// register tiles: 1024 x 96 takes 1.24 ms as a tree and 3.8 ms in one block,
+// 512 x 96 0.95 and 0.69 ms, 512 x 32 0.25 and 0.13 ms.
 int tree_block(int K) { return K <= 96 ? 256 : 512; }
 bool tree_shape(int M, int K) {
-  return M > kTreeRows && M > tree_block(K) && M < (1 << 28) && K >= 1 && K <= kTreeCols &&
-         M >= 3 * K;
+  return M > kTreeRows && M < (1 << 28) && K >= 1 && K <= kTreeCols && M >= 3 * K;
 }
 
 // Row blocks and fan-in such that a node has at most 256 rows (512 above 96

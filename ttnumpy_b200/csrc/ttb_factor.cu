@@ -646,8 +646,9 @@ static __device__ __noinline__ void hh_panel8(double* W, i64 ld, int m, int k, d
 // one barrier.  Bound by the chain of a column step (about 2000 cycles at 256
 // rows: two reductions, a square root and two reciprocals).  256 x 64 with
 // its Q took 2.92 ms column by column (a block-wide reduction and three
-// barriers per 16 columns of every step) and takes 0.21 ms, its R alone 0.44
-// and 0.14 ms; 64 x 64 with Q 0.96 and 0.11 ms.
+// barriers per 16 columns of every step) and takes 0.19 ms, its R alone 0.44
+// and 0.11 ms (both with hh_panel8 up to 256 rows; this form alone 0.21 and
+// 0.14 ms).
 template <int LPC, int RP, int SL>
 static __device__ __noinline__ void hh_panel(double* W, i64 ld, int m, int k, double* tau) {
   constexpr int G = 32 / LPC;
