@@ -434,7 +434,7 @@ def config1_run(torch):
     out = {}
     torch.cuda.synchronize()
     t0 = time.perf_counter()
-    r = amen_persistent([(p.A, p.b, None, kw)], rmax=64)[0]
+    r = amen_persistent([(p.A, p.b, None, kw)], rmax=64, cluster=1)[0]
     torch.cuda.synchronize()
     out["persistent_s"] = time.perf_counter() - t0
     out["persistent_device_s"] = r.device_ms * 1e-3

@@ -445,22 +445,25 @@ def prepare(requests: Sequence) -> List["_Prepared"]:
 
 def amen_persistent(requests: Sequence, rmax: int = 64, max_rmax: int = 256,
                     stream: Optional[torch.cuda.Stream] = None,
-                    time_limit: Optional[float] = None, cluster: int = 1) -> List[Result]:
+                    time_limit: Optional[float] = None,
+                    cluster: Optional[int] = None) -> List[Result]:
     """Solve ``[(A, b, x0, kwargs), ...]`` in one persistent launch; solves
     whose bonds outgrow ``rmax`` are re-run with twice the capacity.  With
     ``time_limit`` (seconds) a solve still running after that long on the
-    device stops with status -6; with ``cluster`` > 1 every solve runs on a
-    cluster of that many thread blocks, and a batch that leaves the device
-    idle is spread over clusters by itself (``spread``; same results)."""
+    device stops with status -6.  Every solve runs on ``cluster`` thread
+    blocks, 1 being one block of ``k_amen``; without it a batch that leaves the
+    device idle is spread over clusters (``spread``; same results).  Callers
+    that keep the device busy from several streams or threads pass 1: a
+    cluster starts only where that many multiprocessors are free together."""
     K.device_ok()
     preps = prepare(requests)
     sms = torch.cuda.get_device_properties("cuda").multi_processor_count
     results: List[Optional[Result]] = [None] * len(preps)
     todo = list(range(len(preps)))
     while todo:
-        batch = [preps[i] for i in todo]
-        out = PersistentBatch(batch, rmax, time_limit=time_limit,
-                              cluster=cluster if cluster > 1 else spread(len(batch), sms)).run(stream)
+        size = spread(len(todo), sms) if cluster is None else cluster
+        out = PersistentBatch([preps[i] for i in todo], rmax, time_limit=time_limit,
+                              cluster=size).run(stream)
         retry = []
         for i, res in zip(todo, out):
             if res.status == -4 and rmax < max_rmax:
