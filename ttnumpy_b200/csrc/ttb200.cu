@@ -222,48 +222,222 @@ __global__ void __launch_bounds__(TTB_THREADS) k_copy(const __grid_constant__ CB
 constexpr int kMaxK = 32;
 struct KBatch {
   int count;
+  int rows;  // rows (a, i) of the operator core that a block multiplies with its slab
   ttb_kron_t d[kMaxK];
 };
 
-// Rows (a, i) of the operator core that a block multiplies with its slab.
-constexpr int kKronRows = 32;
+// A row of the operator core is searched for its nonzeros where that saves
+// more than the search costs, a ballot for each bond of a row whatever the mode:
+// from modes of 32 on, and of 16 where there are many outputs.  Otherwise the
+// outputs are formed one by one.  Mode 2, bond 64, times bond 8: 8 us one by one
+// and 142 searched; banded mode 16, bond 4, times bond 64: 34 us one by one and 9
+// searched (dense 16), times bond 20 5.6 and 12.9; banded mode 32, bond 4, times
+// bond 8: 7.3 and 5.0 us (dense 6.0).
+constexpr int kKronMode = 32, kKronSmallMode = 16;
+constexpr i64 kKronMany = 1 << 17;
+// Rows of a block where the launch fills the device (two blocks for each of
+// 148 multiprocessors), and where it does not: a row per warp, or two of modes
+// past kKronMidMode, whose slabs take as long to read as a row to multiply.
+// Mode 64, bond 4, banded, times bond 1: 15 us with 32 rows, 5 us with 8.
+constexpr int kKronRows = 32, kKronFewRows = TTB_WARPS, kKronFull = 296, kKronMidMode = 256;
 // Shared memory of a slab: columns (k, y) of core[x, :, :, :] taken together.
 constexpr int kKronSlab = 48 * 1024;
+// Blocks that take the outputs one by one.
+constexpr i64 kKronFlat = 2048;
 
+__host__ __device__ inline i64 kron_outputs(const ttb_kron_t& q) {
+  return (i64)q.ra * q.rx * q.n * q.kk * q.ra2 * q.rx2;
+}
+// How a product is formed: each output by a thread; rows (b, y) of at least 32
+// outputs by a warp each, where there are enough of them (no division for each
+// output: mode 2, bond 64 times 64, 298 and 149 us); or rows searched, their
+// columns and numbers counted in 32 bits.
+enum { KRON_FLAT = 0, KRON_ROWS = 1, KRON_SEARCH = 2 };
+__host__ __device__ inline int kron_form(const ttb_kron_t& q) {
+  const i64 outputs = kron_outputs(q), wide = (i64)q.ra2 * q.rx2;
+  if ((q.m >= kKronMode || (q.m >= kKronSmallMode && outputs >= kKronMany)) &&
+      (i64)q.kk * q.rx2 <= 0x7fffffff - 512 && (i64)q.ra * q.n <= 0x7fffffff - 512)
+    return KRON_SEARCH;
+  return wide >= 32 && wide <= 0x7fffffff && outputs >= wide * kKronFull * TTB_WARPS ? KRON_ROWS
+                                                                                      : KRON_FLAT;
+}
 // A mode so large that 32 columns do not fit reads the core from memory.
 __host__ __device__ inline bool kron_in_slab(const ttb_kron_t& q) {
   return (i64)q.m * 32 * 8 <= kSmemCap;
 }
 __host__ __device__ inline int kron_cols(const ttb_kron_t& q) {
-  const int fit = std::max(32, kKronSlab / 8 / std::max(q.m, 1) / 32 * 32);
+  const int fit = std::max(32, kKronSlab / 8 / q.m / 32 * 32);
   return std::min(fit, q.kk * q.rx2);
 }
-__host__ __device__ inline i64 kron_blocks(const ttb_kron_t& q) {
-  const i64 cols = (i64)q.kk * q.rx2, rows = (i64)q.ra * q.n;
-  if (cols <= 0 || rows <= 0 || q.rx <= 0 || q.ra2 <= 0) return 0;
+__host__ __device__ inline i64 kron_blocks(const ttb_kron_t& q, int rows) {
+  const i64 outputs = kron_outputs(q);
+  if (outputs <= 0) return 0;
+  if (kron_form(q) != KRON_SEARCH) {
+    const i64 all = (outputs + TTB_THREADS - 1) / TTB_THREADS;
+    return all < kKronFlat ? all : kKronFlat;
+  }
   const int ct = kron_cols(q);
-  return q.rx * ((cols + ct - 1) / ct) * ((rows + kKronRows - 1) / kKronRows);
+  return q.rx * (((i64)q.kk * q.rx2 + ct - 1) / ct) * (((i64)q.ra * q.n + rows - 1) / rows);
 }
 
-// out[(a, x), i, k, (b, y)] = sum_j op[a, i, j, b] core[x, j, k, y].  A block
-// holds the slab core[x, :, (k, y)] in shared memory and forms the rows
-// (a, i) of its share, a warp a row, a lane a column (k, y); for each b the
-// nonzero operator entries are found with a ballot and only they are
-// multiplied, in the order of j (the cores of discretised operators are
-// banded: 15 of 256 entries of a mode-64 diffusion core, where the product
-// had multiplied them all).  A slab that holds an infinity or a NaN is
-// multiplied with the zeros too, so that they spread as they should.  Bound
-// by writing ``out``: the twelve cores of a mode-64 diffusion operator times
-// a rank-32 train (84 MB) take 0.10 ms a product, where a launch per core and
-// all the zeros took 1.31 ms.
-__global__ void __launch_bounds__(TTB_THREADS) k_kron(const __grid_constant__ KBatch kb) {
-  extern __shared__ double slab[];
+// One row (a, i) of a searched product: the columns c0 .. c0 + w - 1 (at most
+// 32 NU of them), column c of core[x, j, :, :] at from[j * step + c - c0], the
+// row's outputs for b = 0 from ``out`` on.  The warp has the operator entries
+// of the next 32 j or the next b under way while it multiplies.
+template <int NU>
+__device__ __forceinline__ void kron_row(const ttb_kron_t& q, const double* op, double* out,
+                                         const double* from, i64 step, int c0, int w, bool odd,
+                                         double2* entries) {
+  const int lane = threadIdx.x & 31, m = q.m, chunks = (m + 31) / 32;
+  const i64 wide = (i64)q.ra2 * q.rx2;
+  int at[NU];  // the lanes past w repeat the last column
+#pragma unroll
+  for (int u = 0; u < NU; ++u) at[u] = min(32 * u + lane, w - 1);
+  auto entry = [&](int b, int chunk) {
+    const int j = 32 * chunk + lane;
+    return j < m ? op[(i64)j * q.ra2 + b] : 0.0;
+  };
+  double ahead = entry(0, 0);
+  for (int b = 0; b < q.ra2; ++b) {
+    double acc[NU];
+#pragma unroll
+    for (int u = 0; u < NU; ++u) acc[u] = 0.0;
+    for (int chunk = 0; chunk < chunks; ++chunk) {
+      const double v = ahead;
+      if (chunk + 1 < chunks) ahead = entry(b, chunk + 1);
+      else if (b + 1 < q.ra2) ahead = entry(b + 1, 0);
+      const int left = min(32, m - 32 * chunk);
+      unsigned todo = __ballot_sync(0xffffffffu, odd ? lane < left : v != 0.0);
+      const double* s = from + 32 * chunk * step;
+      if (todo == 0xffffffffu) {
+        // dense: through shared memory, two entries a load (a shuffle each took
+        // twice the time)
+        __syncwarp();
+        reinterpret_cast<double*>(entries)[lane] = v;
+        __syncwarp();
+#pragma unroll(NU == 4 ? 1 : 4)
+        for (int j = 0; j < 32; j += 2) {
+          const double2 o = entries[j / 2];
+#pragma unroll
+          for (int u = 0; u < NU; ++u) {
+            acc[u] = fma(o.x, s[j * step + at[u]], acc[u]);
+            acc[u] = fma(o.y, s[(j + 1) * step + at[u]], acc[u]);
+          }
+        }
+        continue;
+      }
+      while (todo) {
+        const int j = __ffs(todo) - 1;
+        todo &= todo - 1;
+        const double o = __shfl_sync(0xffffffffu, v, j);
+#pragma unroll
+        for (int u = 0; u < NU; ++u) acc[u] = fma(o, s[j * step + at[u]], acc[u]);
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < NU; ++u) {
+      if (32 * u + lane >= w) continue;
+      const int c = c0 + 32 * u + lane, k = q.kk == 1 ? 0 : c / q.rx2;
+      out[k * wide + (i64)b * q.rx2 + (c - k * q.rx2)] = acc[u];
+    }
+  }
+}
+
+// The rows r0 + warp, ... of a block's share, 128 columns at a time.
+__device__ __forceinline__ void kron_rows(const ttb_kron_t& q, const double* from, i64 step,
+                                          int x, int r0, int rows, int c0, int w, bool odd,
+                                          double2 (*entries)[16]) {
+  double2* mine = entries[threadIdx.x >> 5];
+  for (int r = r0 + (threadIdx.x >> 5); r < min(r0 + rows, q.ra * q.n); r += TTB_WARPS) {
+    const int a = r / q.n, i = r - a * q.n;
+    const double* op = q.op + (i64)r * q.m * q.ra2;  // op[a, i, :, :]
+    double* out = q.out + (((i64)a * q.rx + x) * q.n + i) * q.kk * q.ra2 * q.rx2;
+    for (int cc = 0; cc < w; cc += 128) {
+      const int n = min(128, w - cc);
+      if (n <= 32) kron_row<1>(q, op, out, from + cc, step, c0 + cc, n, odd, mine);
+      else if (n <= 64) kron_row<2>(q, op, out, from + cc, step, c0 + cc, n, odd, mine);
+      else kron_row<4>(q, op, out, from + cc, step, c0 + cc, n, odd, mine);
+    }
+  }
+}
+
+// out[(a, x), i, k, (b, y)] = sum_j op[a, i, j, b] core[x, j, k, y], the
+// outputs dealt out to the threads; I indexes them.
+template <typename I>
+__global__ void __launch_bounds__(TTB_THREADS, 4) k_kron_flat(const __grid_constant__ KBatch kb) {
   const ttb_kron_t& q = kb.d[blockIdx.y];
-  if ((i64)blockIdx.x >= kron_blocks(q)) return;
-  const int cols = q.kk * q.rx2, rows = q.ra * q.n, ct = kron_cols(q);
-  const int nrc = (rows + kKronRows - 1) / kKronRows;
+  const i64 blocks = kron_blocks(q, kb.rows), total = kron_outputs(q);
+  if ((i64)blockIdx.x >= blocks) return;
+  const i64 astep = q.ra2, cstep = (i64)q.kk * q.rx2;
+  for (i64 e = (i64)blockIdx.x * TTB_THREADS + threadIdx.x; e < total; e += blocks * TTB_THREADS) {
+    I r = (I)e;
+    const I y = r % (I)q.rx2; r /= (I)q.rx2;
+    const I b = r % (I)q.ra2; r /= (I)q.ra2;
+    const I k = r % (I)q.kk; r /= (I)q.kk;
+    const I i = r % (I)q.n; r /= (I)q.n;
+    const I x = r % (I)q.rx, a = r / (I)q.rx;
+    const double* op = q.op + ((i64)a * q.n + i) * q.m * astep + b;
+    const double* cr = q.core + (i64)x * q.m * cstep + (i64)k * q.rx2 + y;
+    double s = 0.0;
+    for (int j = 0; j < q.m; ++j) s = fma(op[j * astep], cr[j * cstep], s);
+    q.out[e] = s;
+  }
+}
+
+// The same, the rows (a, x, i, k) dealt out to the warps.
+__global__ void __launch_bounds__(TTB_THREADS, 3) k_kron_rows(const __grid_constant__ KBatch kb) {
+  const ttb_kron_t& q = kb.d[blockIdx.y];
+  const i64 blocks = kron_blocks(q, kb.rows);
+  if ((i64)blockIdx.x >= blocks) return;
+  const int wide = q.ra2 * q.rx2, lane = threadIdx.x & 31;
+  const i64 rows = kron_outputs(q) / wide, astep = q.ra2, cstep = (i64)q.kk * q.rx2;
+  const int on = 32 / q.rx2, rest = 32 - on * q.rx2;  // 32 outputs on: b and y
+  const int b0 = lane / q.rx2, y0 = lane - b0 * q.rx2;
+  for (i64 e = (i64)blockIdx.x * TTB_WARPS + (threadIdx.x >> 5); e < rows;
+       e += blocks * TTB_WARPS) {
+    i64 r = e;
+    const i64 k = r % q.kk; r /= q.kk;
+    const i64 i = r % q.n; r /= q.n;
+    const i64 x = r % q.rx, a = r / q.rx;
+    const double* op = q.op + (a * q.n + i) * q.m * astep;
+    const double* cr = q.core + x * q.m * cstep + k * q.rx2;
+    double* out = q.out + e * wide;
+    int b = b0, y = y0;
+    for (int c = lane; c < wide; c += 32) {
+      double s = 0.0;
+      for (int j = 0; j < q.m; ++j) s = fma(op[j * astep + b], cr[j * cstep + y], s);
+      out[c] = s;
+      b += on;
+      y += rest;
+      if (y >= q.rx2) {
+        y -= q.rx2;
+        ++b;
+      }
+    }
+  }
+}
+
+// The product of a TTM and a TT core where rows are searched.  A block holds
+// the slab core[x, :, (k, y)] in shared memory and forms the rows (a, i) of its
+// share, a warp a row, a lane a column (k, y); for each b a ballot finds the
+// nonzero operator entries and only they are multiplied, in the order of j (the
+// cores of discretised operators are banded: 15 of 256 entries of a mode-64
+// diffusion core).  A slab that holds an infinity or a NaN is multiplied with
+// the zeros too, so that they spread as they should.  Bound by the issue of a
+// row's ballots, shuffles and 256-byte stores: the twelve cores of a mode-64
+// diffusion operator times a rank-32 train (84 MB written, 13 us at the rate of
+// HBM) take 88 us a product; a launch per core that multiplies the zeros takes
+// 1310.  A dense core of mode 64 and bond 4 times bond 32 takes 33 us, with a
+// thread for each output 101.
+__global__ void __launch_bounds__(TTB_THREADS, 4) k_kron(const __grid_constant__ KBatch kb) {
+  extern __shared__ double slab[];
+  __shared__ double2 entries[TTB_WARPS][16];
+  const ttb_kron_t& q = kb.d[blockIdx.y];
+  if ((i64)blockIdx.x >= kron_blocks(q, kb.rows)) return;
+  const int cols = q.kk * q.rx2, ct = kron_cols(q);
+  const int nrc = (q.ra * q.n + kb.rows - 1) / kb.rows;
   const int nct = (cols + ct - 1) / ct;
-  const int r0 = (int)(blockIdx.x % nrc) * kKronRows;
+  const int r0 = (int)(blockIdx.x % nrc) * kb.rows;
   const int c0 = (int)(blockIdx.x / nrc % nct) * ct;
   const int x = (int)(blockIdx.x / nrc / nct);
   const int w = min(ct, cols - c0);
@@ -276,41 +450,9 @@ __global__ void __launch_bounds__(TTB_THREADS) k_kron(const __grid_constant__ KB
     if (staged) slab[e] = v;
     odd |= !isfinite(v);
   }
-  const double* from = staged ? slab : core;
-  const i64 step = staged ? w : cols;
   odd = __syncthreads_or(odd);
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const i64 wide = (i64)q.ra2 * q.rx2;
-  for (int r = r0 + warp; r < min(r0 + kKronRows, rows); r += TTB_WARPS) {
-    const int a = r / q.n, i = r - a * q.n;
-    const double* op = q.op + (i64)r * q.m * q.ra2;  // op[a, i, :, :]
-    double* out = q.out + (((i64)a * q.rx + x) * q.n + i) * q.kk * wide;
-    for (int b = 0; b < q.ra2; ++b) {
-      for (int cc = 0; cc < w; cc += 128) {
-        double acc[4] = {0.0, 0.0, 0.0, 0.0};
-        for (int j0 = 0; j0 < q.m; j0 += 32) {
-          const double v = j0 + lane < q.m ? op[(i64)(j0 + lane) * q.ra2 + b] : 0.0;
-          unsigned todo = __ballot_sync(0xffffffffu, odd ? j0 + lane < q.m : v != 0.0);
-          while (todo) {
-            const int j = __ffs(todo) - 1;
-            todo &= todo - 1;
-            const double o = __shfl_sync(0xffffffffu, v, j);
-            const double* s = from + (j0 + j) * step + cc + lane;
-#pragma unroll
-            for (int u = 0; u < 4; ++u)
-              if (cc + 32 * u + lane < w) acc[u] = fma(o, s[32 * u], acc[u]);
-          }
-        }
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const int c = cc + 32 * u + lane;
-          if (c >= w) continue;
-          const int k = q.kk == 1 ? 0 : (c0 + c) / q.rx2, y = c0 + c - k * q.rx2;
-          out[k * wide + (i64)b * q.rx2 + y] = acc[u];
-        }
-      }
-    }
-  }
+  if (staged) kron_rows(q, slab, w, x, r0, kb.rows, c0, w, odd, entries);
+  else kron_rows(q, core, cols, x, r0, kb.rows, c0, w, odd, entries);
 }
 
 struct HBatch {
@@ -2113,19 +2255,34 @@ int ttb_kron(const ttb_kron_t* ps, int count, void* stream) {
   cudaStream_t s = as_stream(stream);
   if (int e = smem_limit_once((const void*)k_kron, kSmemCap, g_smem_kron)) return e;
   for (int i0 = 0; i0 < count; i0 += kMaxK) {
-    KBatch kb;
-    kb.count = std::min(kMaxK, count - i0);
-    i64 most = 1, smem = 0;
-    for (int j = 0; j < kb.count; ++j) {
-      kb.d[j] = ps[i0 + j];
-      most = std::max(most, kron_blocks(kb.d[j]));
-      if (kron_in_slab(kb.d[j]))
-        smem = std::max(smem, (i64)kb.d[j].m * kron_cols(kb.d[j]) * 8);
+    ProfScope prof(P_KRON, s, 0.0, 0.0);
+    for (int form = KRON_FLAT; form <= KRON_SEARCH; ++form) {  // a launch for each there is
+      KBatch kb;
+      kb.count = 0;
+      i64 most = 0, smem = 0, all = 0, outputs = 0;
+      int modes = 0;
+      for (int j = i0; j < std::min(count, i0 + kMaxK); ++j) {
+        if (kron_form(ps[j]) != form) continue;
+        kb.d[kb.count++] = ps[j];
+        all += kron_blocks(ps[j], kKronRows);
+        outputs = std::max(outputs, kron_outputs(ps[j]));
+        modes = std::max(modes, ps[j].m);
+      }
+      kb.rows = all >= kKronFull ? kKronRows : modes <= kKronMidMode ? kKronFewRows : 2 * kKronFewRows;
+      for (int j = 0; j < kb.count; ++j) {
+        most = std::max(most, kron_blocks(kb.d[j], kb.rows));
+        if (form == KRON_SEARCH && kron_in_slab(kb.d[j]))
+          smem = std::max(smem, (i64)kb.d[j].m * kron_cols(kb.d[j]) * 8);
+      }
+      if (most == 0) continue;
+      if (most > 0x7fffffff) return (int)cudaErrorInvalidValue;
+      const dim3 grid((unsigned)most, kb.count);
+      if (form == KRON_SEARCH) k_kron<<<grid, TTB_THREADS, (size_t)smem, s>>>(kb);
+      else if (form == KRON_ROWS) k_kron_rows<<<grid, TTB_THREADS, 0, s>>>(kb);
+      else if (outputs <= 0x7fffffff) k_kron_flat<unsigned><<<grid, TTB_THREADS, 0, s>>>(kb);
+      else k_kron_flat<i64><<<grid, TTB_THREADS, 0, s>>>(kb);
+      counted();
     }
-    if (most > 0x7fffffff) return (int)cudaErrorInvalidValue;
-    ProfScope ps(P_KRON, s, 0.0, 0.0);
-    k_kron<<<dim3((unsigned)most, kb.count), TTB_THREADS, (size_t)smem, s>>>(kb);
-    counted();
   }
   return last_error();
 }
