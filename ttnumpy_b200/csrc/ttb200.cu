@@ -730,9 +730,6 @@ struct Tree {
 
 constexpr int kTreeCols = 128, kTreeRows = 512, kTreeGroup = 8;
 constexpr int kTreeSlice = 32;  // columns of Q a block takes on the way down
-// Problems of one call up to which the trees are used: more fill the chip
-// with a block each.
-constexpr int kTreeProblems = 16;
 
 // Rows of a leaf; and tall enough that two levels of blocks beat one block's
 // register tiles: 1024 x 96 takes 1.24 ms as a tree and 3.8 ms in one block,
@@ -2014,29 +2011,27 @@ long long ttb_qr_work_doubles(int m, int k) {
 int ttb_qr(const ttb_qr_t* ps, int count, void* stream) {
   if (int e = configure_smem()) return e;
   cudaStream_t s = as_stream(stream);
+  // A problem's shape alone decides how it is factored, so that its bits do not
+  // depend on the other problems of the call.
   std::vector<ttb_qr_t> rest;
   std::vector<Tree> trees;
-  for (int i = 0; i < count; ++i)
-    if (tree_shape(ps[i].m, ps[i].k)) trees.emplace_back();
-  if (!trees.empty() && (int)trees.size() <= kTreeProblems) {
-    trees.clear();
-    for (int i = 0; i < count; ++i) {
-      const ttb_qr_t& p = ps[i];
-      if (!tree_shape(p.m, p.k)) {
-        rest.push_back(p);
-        continue;
-      }
-      Tree t = {};
-      tree_layout(t, p.m, p.k);
-      t.a = p.a, t.a_rs = p.a_rs, t.a_cs = p.a_cs;
-      t.q = p.q, t.q_rs = p.q_rs, t.q_cs = p.q_cs;
-      t.r = p.r, t.r_rs = p.r_rs, t.r_cs = p.r_cs;
-      t.work = p.work;
-      trees.push_back(t);
+  double fl = 0.0;
+  for (int i = 0; i < count; ++i) {
+    const ttb_qr_t& p = ps[i];
+    if (!tree_shape(p.m, p.k)) {
+      rest.push_back(p);
+      continue;
     }
-    double fl = 0.0;
-    for (const Tree& t : trees)
-      fl += (t.q ? 2.0 : 1.0) * (2.0 * t.M * t.K * (double)t.K - 2.0 / 3.0 * t.K * (double)t.K * t.K);
+    Tree t = {};
+    tree_layout(t, p.m, p.k);
+    t.a = p.a, t.a_rs = p.a_rs, t.a_cs = p.a_cs;
+    t.q = p.q, t.q_rs = p.q_rs, t.q_cs = p.q_cs;
+    t.r = p.r, t.r_rs = p.r_rs, t.r_cs = p.r_cs;
+    t.work = p.work;
+    fl += (t.q ? 2.0 : 1.0) * (2.0 * t.M * t.K * (double)t.K - 2.0 / 3.0 * t.K * (double)t.K * t.K);
+    trees.push_back(t);
+  }
+  if (!trees.empty()) {
     ProfScope prof(P_QR, s, fl, 0.0);
     if (int e = run_trees(trees, s)) return e;
     ps = rest.data();
@@ -2124,36 +2119,30 @@ long long ttb_svd_work_doubles(int m, int k) {
 int ttb_svd(const ttb_svd_t* ps, int count, void* stream) {
   if (int e = configure_smem()) return e;
   cudaStream_t s = as_stream(stream);
-  std::vector<ttb_svd_t> rest;
+  std::vector<ttb_svd_t> rest;  // trees by the shape alone, as in ttb_qr
   std::vector<Tree> trees;
-  auto tall = [](const ttb_svd_t& p) {
-    return tree_shape(std::max(p.m, p.k), std::min(p.m, p.k));
-  };
-  for (int i = 0; i < count; ++i)
-    if (tall(ps[i])) trees.emplace_back();
-  if (!trees.empty() && (int)trees.size() <= kTreeProblems) {
-    trees.clear();
-    double fl = 0.0;
-    for (int i = 0; i < count; ++i) {
-      const ttb_svd_t& p = ps[i];
-      if (!tall(p)) {
-        rest.push_back(p);
-        continue;
-      }
-      // a wide matrix by its transpose, as k_svd does
-      const bool up = p.m >= p.k;
-      Tree t = {};
-      tree_layout(t, std::max(p.m, p.k), std::min(p.m, p.k));
-      t.svd = 1;
-      t.a = p.a, t.a_rs = up ? p.a_rs : p.a_cs, t.a_cs = up ? p.a_cs : p.a_rs;
-      t.q = up ? p.u : p.vh, t.q_rs = up ? p.u_rs : p.vh_cs, t.q_cs = up ? p.u_cs : p.vh_rs;
-      t.vh = up ? p.vh : p.u, t.vh_rs = up ? p.vh_rs : p.u_cs, t.vh_cs = up ? p.vh_cs : p.u_rs;
-      t.s = p.s;
-      t.status = p.status;
-      t.work = p.work;
-      fl += 4.0 * t.M * t.K * (double)t.K - 4.0 / 3.0 * t.K * (double)t.K * t.K;
-      trees.push_back(t);
+  double fl = 0.0;
+  for (int i = 0; i < count; ++i) {
+    const ttb_svd_t& p = ps[i];
+    if (!tree_shape(std::max(p.m, p.k), std::min(p.m, p.k))) {
+      rest.push_back(p);
+      continue;
     }
+    // a wide matrix by its transpose, as k_svd does
+    const bool up = p.m >= p.k;
+    Tree t = {};
+    tree_layout(t, std::max(p.m, p.k), std::min(p.m, p.k));
+    t.svd = 1;
+    t.a = p.a, t.a_rs = up ? p.a_rs : p.a_cs, t.a_cs = up ? p.a_cs : p.a_rs;
+    t.q = up ? p.u : p.vh, t.q_rs = up ? p.u_rs : p.vh_cs, t.q_cs = up ? p.u_cs : p.vh_rs;
+    t.vh = up ? p.vh : p.u, t.vh_rs = up ? p.vh_rs : p.u_cs, t.vh_cs = up ? p.vh_cs : p.u_rs;
+    t.s = p.s;
+    t.status = p.status;
+    t.work = p.work;
+    fl += 4.0 * t.M * t.K * (double)t.K - 4.0 / 3.0 * t.K * (double)t.K * t.K;
+    trees.push_back(t);
+  }
+  if (!trees.empty()) {
     ProfScope prof(P_SVD, s, fl, 0.0);
     if (int e = run_trees(trees, s)) return e;
     ps = rest.data();
