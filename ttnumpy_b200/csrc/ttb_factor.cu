@@ -143,33 +143,19 @@ static __device__ __noinline__ void cta_householder_short(double* W, int m, int 
   __syncthreads();
 }
 
-// In-place Householder QR of the m x k matrix W (column step ``ldw``, unit
-// row step), as LAPACK dgeqr2 lays it out: on return R is in the upper
-// triangle and the reflector vectors v_j (v_j[j] = 1 implied) below the
-// diagonal, with the scalars in tau[0 .. min(m,k)-1].  Each reflector is
-// H = I - tau v v^T built as in dlarfg: beta = -sign(alpha) ||x||,
-// tau = (beta - alpha) / beta, v = x / (alpha - beta); a column whose
-// sub-diagonal part is exactly zero gets tau = 0.
-static __device__ void cta_householder(double* W, int m, int k, i64 ldw, double* tau, double* red) {
-  // The whole block works on every reflector: the trailing columns are
-  // taken HC at a time, their dot products with v accumulated per thread
-  // over a row stripe and reduced together, and the squared norm of the
-  // next column is gathered during its update (one pass fewer per column).
-  if (m <= 33) {
-    cta_householder_short<1>(W, m, k, ldw, tau);
-    return;
-  }
-  if (m <= 65) {
-    cta_householder_short<2>(W, m, k, ldw, tau);
-    return;
-  }
-  if (m <= 129) {
-    cta_householder_short<4>(W, m, k, ldw, tau);
-    return;
-  }
-  constexpr int HC = 16;
-  __shared__ double hred[TTB_WARPS][HC];
-  __shared__ double hw[HC];
+// The general form.  The whole block works on every reflector: the trailing
+// columns are taken kHC at a time, their dot products with v accumulated per
+// thread over a row stripe and reduced together, and the squared norm of the
+// next column is gathered during its update (one pass fewer per column).
+// SHARED: W is in shared memory, and the compiler may take it for granted (R of
+// 4096 x 3 takes 31 us so and 44 us through generic addresses).
+constexpr int kHC = 16;
+template <bool SHARED>
+static __device__ __forceinline__ void householder_passes(double* W, int m, int k, i64 ldw,
+                                                          double* tau, double* red,
+                                                          double (&hred)[TTB_WARPS][kHC],
+                                                          double (&hw)[kHC]) {
+  if constexpr (SHARED) __builtin_assume(__isShared(W));
   const int p = m < k ? m : k;
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   double part = 0.0;
@@ -195,21 +181,21 @@ static __device__ void cta_householder(double* W, int m, int k, i64 ldw, double*
     }
     __syncthreads();
     double next = 0.0;  // this thread's part of |column j+1, rows > j+1|^2
-    for (int c0 = j + 1; c0 < k; c0 += HC) {
-      const int nc = min(HC, k - c0);
+    for (int c0 = j + 1; c0 < k; c0 += kHC) {
+      const int nc = min(kHC, k - c0);
       double* cb = W + (i64)c0 * ldw;
       if (t != 0.0) {
-        double w[HC];
+        double w[kHC];
 #pragma unroll
-        for (int q = 0; q < HC; ++q) w[q] = 0.0;
+        for (int q = 0; q < kHC; ++q) w[q] = 0.0;
         for (int i = j + 1 + tid; i < m; i += TTB_THREADS) {
           const double v = col[i];
 #pragma unroll
-          for (int q = 0; q < HC; ++q)
+          for (int q = 0; q < kHC; ++q)
             if (q < nc) w[q] = fma(v, cb[i + q * ldw], w[q]);
         }
 #pragma unroll
-        for (int q = 0; q < HC; ++q) {
+        for (int q = 0; q < kHC; ++q) {
           const double sw = warp_sum(w[q]);
           if (lane == 0) hred[wid][q] = sw;
         }
@@ -225,7 +211,7 @@ static __device__ void cta_householder(double* W, int m, int k, i64 ldw, double*
         for (int i = j + 1 + tid; i < m; i += TTB_THREADS) {
           const double v = col[i];
 #pragma unroll
-          for (int q = 0; q < HC; ++q) {
+          for (int q = 0; q < kHC; ++q) {
             if (q < nc) {
               const double x = fma(-hw[q], v, cb[i + q * ldw]);
               cb[i + q * ldw] = x;
@@ -240,6 +226,32 @@ static __device__ void cta_householder(double* W, int m, int k, i64 ldw, double*
     }
     if (j + 1 < p) sigma = block_sum(next, red);
   }
+}
+
+// In-place Householder QR of the m x k matrix W (column step ``ldw``, unit
+// row step), as LAPACK dgeqr2 lays it out: on return R is in the upper
+// triangle and the reflector vectors v_j (v_j[j] = 1 implied) below the
+// diagonal, with the scalars in tau[0 .. min(m,k)-1].  Each reflector is
+// H = I - tau v v^T built as in dlarfg: beta = -sign(alpha) ||x||,
+// tau = (beta - alpha) / beta, v = x / (alpha - beta); a column whose
+// sub-diagonal part is exactly zero gets tau = 0.
+static __device__ void cta_householder(double* W, int m, int k, i64 ldw, double* tau, double* red) {
+  if (m <= 33) {
+    cta_householder_short<1>(W, m, k, ldw, tau);
+    return;
+  }
+  if (m <= 65) {
+    cta_householder_short<2>(W, m, k, ldw, tau);
+    return;
+  }
+  if (m <= 129) {
+    cta_householder_short<4>(W, m, k, ldw, tau);
+    return;
+  }
+  __shared__ double hred[TTB_WARPS][kHC];
+  __shared__ double hw[kHC];
+  if (__isShared(W)) householder_passes<true>(W, m, k, ldw, tau, red, hred, hw);
+  else householder_passes<false>(W, m, k, ldw, tau, red, hred, hw);
 }
 
 // Overwrite the m x q matrix X (strided) with H_0 H_1 ... H_{p-1} X, the
@@ -850,12 +862,20 @@ static __device__ __noinline__ void cta_hh(double* W, i64 ld, int m, int k, doub
 // the trailing updates as GEMMs.
 constexpr int kHHTall = 512;
 
-// A panel's reflectors: in registers, or row by row beyond their reach.
+// Whether the register tiles take a matrix: not beyond their rows, and not
+// where a few columns leave most of a tile empty.  512 x 2 with its Q takes 22 us
+// in tiles and 11 us column by column, 256 x 4 21 and 17 us, 256 x 8 31 and 47 us.
+constexpr int kNarrow = 4;
+static __device__ __forceinline__ bool hh_tiled(int m, int k) {
+  return m <= kHHRows && k > kNarrow;
+}
+
+// A panel's reflectors: in registers, or column by column.
 template <bool TILED>
 static __device__ __forceinline__ void cta_hh_any(double* W, int m, int k, i64 ld, double* tau,
                                                   double* red) {
   if constexpr (TILED) {
-    if (m <= kHHRows) {
+    if (hh_tiled(m, k)) {
       cta_hh(W, ld, m, k, tau);
       return;
     }
@@ -874,7 +894,7 @@ __device__ __noinline__ void cta_qr(CMat A, int m, int k, double* W, i64 ldw, do
   const int p = m < k ? m : k;
   cta_load(A, W, ldw, m, k);
   __syncthreads();
-  const bool tiles = TILED && m <= kHHRows;
+  const bool tiles = TILED && hh_tiled(m, k);
   cta_hh_any<TILED>(W, m, k, ldw, tau, red);
   if (R.p) {
     for (int e = threadIdx.x; e < p * k; e += TTB_THREADS) {
@@ -1650,7 +1670,7 @@ __device__ __noinline__ int cta_svd_tall(CMat A, int m, int k, double* W, i64 ld
                                    double* tau2, Mat U, double* S, Mat Vh, double* red) {
   cta_load(A, W, ldw, m, k);
   __syncthreads();
-  const bool tiles = TILED && m <= kHHRows;
+  const bool tiles = TILED && hh_tiled(m, k);
   cta_hh_any<TILED>(W, m, k, ldw, tau, red);
   const i64 ld = TILED ? svd_step(k) : k;
   for (int e = threadIdx.x; e < k * k; e += TTB_THREADS) {
