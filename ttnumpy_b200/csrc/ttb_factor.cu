@@ -1594,9 +1594,61 @@ static __device__ __forceinline__ double* square_left(int want, int k, double* B
   return want == SQ_LEFT ? X : F;
 }
 
+// The SVD of an upper-triangular B of up to kSmall columns (column step
+// svd_step(k)): one-sided Jacobi on its own columns, B J = U S, without the
+// pivoted QRs that pay from there on.  ``want``, ``order``, S and Vh as above;
+// the left factor (columns in ``order``) takes B's place.  What the pivoted QR,
+// its factors, a second QR and five block-wide steps cost does not depend on k:
+// 64 x 1 takes 20 us with them and 8 us so, 64 x 4 42 and 26, 64 x 6 54 and 46,
+// 64 x 8 60 and 58.
+constexpr int kSmall = 6;
+static __device__ __noinline__ int cta_svd_small(int want, int k, double* B, double* V, double* sv,
+                                                 int* order, int* flag, double* S, Mat Vh,
+                                                 double* red) {
+  const i64 ld = svd_step(k);
+  const int lane = threadIdx.x & 31;
+  double* J = want == SQ_LEFT ? nullptr : V;
+  if (J)
+    for (int e = threadIdx.x; e < k * k; e += TTB_THREADS) J[e % k + (e / k) * ld] = e % k == e / k;
+  const int status = cta_jacobi(B, k, ld, J, ld, 60, square_tol(k), flag);
+  // singular values and their order, a lane a column
+  if (threadIdx.x < 32) {
+    double s = 0.0;
+    for (int i = 0; lane < k && i < k; ++i) s = fma(B[i + lane * ld], B[i + lane * ld], s);
+    s = sqrt(s);
+    int rank = 0;
+    for (int i = 0; i < k; ++i) {
+      const double si = __shfl_sync(0xffffffffu, s, i);
+      rank += (si > s) || (si == s && i < lane);
+    }
+    if (lane < k) {
+      sv[lane] = s;
+      order[lane] = lane;
+    }
+    __syncwarp();
+    if (lane < k && s == s) order[rank] = lane;  // a NaN keeps the unsorted order
+  }
+  __syncthreads();
+  const int zero = __syncthreads_or(threadIdx.x < k && sv[threadIdx.x] == 0.0);
+  if (threadIdx.x < k) S[threadIdx.x] = sv[order[threadIdx.x]];
+  for (int e = threadIdx.x; e < k * k; e += TTB_THREADS) {
+    const int i = e % k, j = e / k;
+    if (J) Vh(j, i) = J[i + order[j] * ld];
+    if (want != SQ_RIGHT && sv[j] != 0.0) B[i + j * ld] /= sv[j];
+  }
+  __syncthreads();
+  if (want != SQ_RIGHT && zero) cta_complete_rows(k, sv, order, order, Mat{B, ld, 1}, red);
+  return status;
+}
+
 static __device__ __noinline__ int cta_svd_square(int want, int k, double* Bsq, double*& V,
                                                   double* sv, int* order, double* tau2, int* flag,
                                                   Mat Us, double* S, Mat Vh, double* red) {
+  if (k <= kSmall) {
+    const int status = cta_svd_small(want, k, Bsq, V, sv, order, flag, S, Vh, red);
+    V = Bsq;
+    return status;
+  }
   square_prepare(want, k, Bsq, V, sv, order, tau2, Us, red);
   const int status = square_iterate(want, k, Bsq, V, flag);
   square_finish(want, k, Bsq, V, sv, order, tau2, flag, S, Vh, red);
