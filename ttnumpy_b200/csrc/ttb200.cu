@@ -731,12 +731,32 @@ struct Tree {
 constexpr int kTreeCols = 128, kTreeRows = 512, kTreeGroup = 8;
 constexpr int kTreeSlice = 32;  // columns of Q a block takes on the way down
 
-// Rows of a leaf; and tall enough that two levels of blocks beat one block's
-// register tiles: 1024 x 96 takes 1.24 ms as a tree and 3.8 ms in one block,
-// 512 x 96 0.95 and 0.69 ms, 512 x 32 0.25 and 0.13 ms.
-int tree_block(int K) { return K <= 96 ? 256 : 512; }
-bool tree_shape(int M, int K) {
-  return M > kTreeRows && M < (1 << 28) && K >= 1 && K <= kTreeCols && M >= 3 * K;
+int tree_block(int K) { return K <= 96 ? 256 : 512; }  // rows of a leaf
+
+// Which tall matrices are factored as trees: those above kTreeRows rows and up
+// to kTreeCols columns that are taller than their columns thrice, except where
+// one block's chain is the shorter one.  A tree costs its levels' launches and
+// nodes, 35 to 45 us for a single column.  One block is the faster one where it
+// has the matrix in shared memory and
+// - has no more than 1024 rows, in register tiles of 16 columns: with Q, block
+//   and tree, 1024 x 16 82 and 122 us, 1024 x 24 165 and 186, 768 x 32 183 and
+//   236, 600 x 40 282 and 288; past that size 900 x 32 714 and 242;
+// - has no more than 2048 rows and eight columns, one tile: 2048 x 8 76 and 80,
+//   1200 x 9 97 and 86;
+// - or little to do: with Q up to 8192 entries (8192 x 1 28 and 45, 2048 x 4 63
+//   and 58, 12000 x 1 78 and 47), for R alone up to 16384 (16384 x 1 17 and 37,
+//   4096 x 4 44 and 49, 1599 x 10 71 and 80; 6000 x 4 62 and 54).
+// An SVD's tree pays earlier, since its root has the iteration to itself: from
+// 1024 rows and 16 columns on (1024 x 16 173 and 181 us, 1025 x 16 259 and 189,
+// 600 x 20 282 and 259), but for up to 6144 entries (6000 x 1 32 and 40, 3000 x 2
+// 41 and 45, 2048 x 3 51 and 56; 8192 x 1 43 and 40, 2048 x 4 78 and 61).
+enum { TREE_QR, TREE_R, TREE_SVD };
+bool tree_shape(int M, int K, int what) {
+  if (M <= kTreeRows || M >= (1 << 28) || K < 1 || K > kTreeCols || M < 3 * K) return false;
+  const i64 entries = (i64)M * K;
+  if (what == TREE_SVD) return entries > 6144 && (M > 1024 || K > 16);
+  if (M <= 1024 && qr_need(M, K) * 8 <= kSmemCap) return false;
+  return what == TREE_R ? entries > 16384 : entries > 8192 && (M > 2048 || K > 8);
 }
 
 // Row blocks and fan-in such that a node has at most 256 rows (512 above 96
@@ -2005,7 +2025,8 @@ int ttb_project(const ttb_project_t* ps, int count, void* stream) {
 
 long long ttb_qr_work_doubles(int m, int k) {
   Tree t;
-  return tree_shape(m, k) ? std::max(qr_need(m, k), tree_layout(t, m, k)) : qr_need(m, k);
+  // the shapes whose R alone comes from a tree are among those with Q
+  return tree_shape(m, k, TREE_QR) ? std::max(qr_need(m, k), tree_layout(t, m, k)) : qr_need(m, k);
 }
 
 int ttb_qr(const ttb_qr_t* ps, int count, void* stream) {
@@ -2018,7 +2039,7 @@ int ttb_qr(const ttb_qr_t* ps, int count, void* stream) {
   double fl = 0.0;
   for (int i = 0; i < count; ++i) {
     const ttb_qr_t& p = ps[i];
-    if (!tree_shape(p.m, p.k)) {
+    if (!tree_shape(p.m, p.k, p.q ? TREE_QR : TREE_R)) {
       rest.push_back(p);
       continue;
     }
@@ -2112,8 +2133,8 @@ int ttb_qr_static(const ttb_qr_t* ps, int count, void* stream) {
 long long ttb_svd_work_doubles(int m, int k) {
   int M = std::max(m, k), K = std::min(m, k);
   Tree t;
-  return tree_shape(M, K) ? std::max(svd_tall_need(M, K), tree_layout(t, M, K))
-                          : svd_tall_need(M, K);
+  return tree_shape(M, K, TREE_SVD) ? std::max(svd_tall_need(M, K), tree_layout(t, M, K))
+                                    : svd_tall_need(M, K);
 }
 
 int ttb_svd(const ttb_svd_t* ps, int count, void* stream) {
@@ -2124,7 +2145,7 @@ int ttb_svd(const ttb_svd_t* ps, int count, void* stream) {
   double fl = 0.0;
   for (int i = 0; i < count; ++i) {
     const ttb_svd_t& p = ps[i];
-    if (!tree_shape(std::max(p.m, p.k), std::min(p.m, p.k))) {
+    if (!tree_shape(std::max(p.m, p.k), std::min(p.m, p.k), TREE_SVD)) {
       rest.push_back(p);
       continue;
     }

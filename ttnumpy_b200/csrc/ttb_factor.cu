@@ -1599,8 +1599,8 @@ static __device__ __forceinline__ double* square_left(int want, int k, double* B
 // pivoted QRs that pay from there on.  ``want``, ``order``, S and Vh as above;
 // the left factor (columns in ``order``) takes B's place.  What the pivoted QR,
 // its factors, a second QR and five block-wide steps cost does not depend on k:
-// 64 x 1 takes 20 us with them and 8 us so, 64 x 4 42 and 26, 64 x 6 54 and 46,
-// 64 x 8 60 and 58.
+// 64 x 1 takes 20 us with them and 9 us so, 64 x 4 42 and 25, 64 x 6 54 and 40,
+// 64 x 8 59 and 58.
 constexpr int kSmall = 6;
 static __device__ __noinline__ int cta_svd_small(int want, int k, double* B, double* V, double* sv,
                                                  int* order, int* flag, double* S, Mat Vh,
