@@ -139,7 +139,7 @@ __global__ void __launch_bounds__(TTB_THREADS) k_gemm(const __grid_constant__ GB
   CMat A{g.a + bi * g.a_bs, g.a_rs, g.a_cs};
   CMat B{g.b + bi * g.b_bs, g.b_rs, g.b_cs};
   Mat C{g.c + bi * g.c_bs, g.c_rs, g.c_cs};
-  cta_gemm_tile(A, B, C, g.m, g.n, g.k, m0, n0, g.alpha, g.beta, sm);
+  cta_gemm_tile<false>(A, B, C, g.m, g.n, g.k, m0, n0, g.alpha, g.beta, sm);
 }
 
 GDesc make_gemm(const double* a, i64 a_rs, i64 a_cs, i64 a_bs, const double* b, i64 b_rs,

@@ -194,8 +194,12 @@ struct OMat {
 // C[m0:m0+GBM, n0:n0+64] = alpha * A * B + beta * C over the full K range.
 // A is M x K, B is K x N.  beta == 0 never reads C.  The warps form a
 // (TTB_WARPS / 4) x 4 grid of 32 x 16 warp tiles, each 4 x 2 MMA tiles of
-// 8 x 8 (the tile is GBM = 8 * TTB_WARPS rows by 64 columns).
-static __device__ void cta_gemm_tile(CMat A, CMat B, const OMat& C, int M, int N, int K, int m0,
+// 8 x 8 (the tile is GBM = 8 * TTB_WARPS rows by 64 columns).  C_FIRST reads
+// all of a thread's C before it writes any (16 registers more): the compiler
+// cannot move a load past a store that may alias it, and a tile of small K waits
+// for one entry after the other.
+template <bool C_FIRST>
+static __device__ __forceinline__ void cta_gemm_tile(CMat A, CMat B, const OMat& C, int M, int N, int K, int m0,
                                      int n0, double alpha, double beta, GemmSmem& sm) {
   const int tid = threadIdx.x;
   const int lane = tid & 31, warp = tid >> 5;
@@ -272,6 +276,20 @@ static __device__ void cta_gemm_tile(CMat A, CMat B, const OMat& C, int M, int N
   for (int j = 0; j < 2; ++j)
 #pragma unroll
     for (int h = 0; h < 2; ++h) coff[j][h] = C.col(n0 + wn + 8 * j + 2 * t + h);
+  double old[C_FIRST ? 4 : 1][2][2];
+  if constexpr (C_FIRST) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int gm = m0 + wm + 8 * i + g;
+      const double* crow = C.p + C.row(gm);
+#pragma unroll
+      for (int j = 0; j < 2; ++j)
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+          old[i][j][h] = beta != 0.0 && gm < M && n0 + wn + 8 * j + 2 * t + h < N
+                             ? crow[coff[j][h]] : 0.0;
+    }
+  }
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     const int gm = m0 + wm + 8 * i + g;
@@ -284,7 +302,10 @@ static __device__ void cta_gemm_tile(CMat A, CMat B, const OMat& C, int M, int N
         const int gn = n0 + wn + 8 * j + 2 * t + h;
         if (gn >= N) continue;
         double v = alpha * acc[i][j][h];
-        if (beta != 0.0) v = fma(beta, crow[coff[j][h]], v);
+        if (beta != 0.0) {
+          if constexpr (C_FIRST) v = fma(beta, old[i][j][h], v);
+          else v = fma(beta, crow[coff[j][h]], v);
+        }
         crow[coff[j][h]] = v;
       }
   }
@@ -295,7 +316,8 @@ static __device__ void cta_gemm_tile(CMat A, CMat B, const OMat& C, int M, int N
 static __device__ __noinline__ void cta_gemm(CMat A, CMat B, OMat C, int M, int N, int K, double alpha, double beta,
                          GemmSmem& sm) {
   for (int m0 = 0; m0 < M; m0 += GBM)
-    for (int n0 = 0; n0 < N; n0 += GBN) cta_gemm_tile(A, B, C, M, N, K, m0, n0, alpha, beta, sm);
+    for (int n0 = 0; n0 < N; n0 += GBN)
+      cta_gemm_tile<true>(A, B, C, M, N, K, m0, n0, alpha, beta, sm);
 }
 
 // ---------------------------------------------------------------------------
