@@ -728,7 +728,7 @@ struct Tree {
   __host__ __device__ static i64 step(int rows) { return (rows + 1) & ~1; }
 };
 
-constexpr int kTreeCols = 128, kTreeRows = 512, kTreeGroup = 8;
+constexpr int kTreeCols = 128, kTreeRows = 512;
 constexpr int kTreeSlice = 32;  // columns of Q a block takes on the way down
 
 int tree_block(int K) { return K <= 96 ? 256 : 512; }  // rows of a leaf
@@ -792,17 +792,24 @@ i64 tree_layout(Tree& t, int M, int K) {
   return off;
 }
 
+// The trees of a launch: a few, or, by a larger parameter block, as many as fill
+// the device: 64 SVDs of 600 x 20 in groups of eight take 2.9 ms, of 32 1.3, and
+// 1.8 ms with a block each.
+constexpr int kTreeFew = 8, kTreeMany = 32;
+template <int N>
 struct TreeBatch {
   int count;
-  Tree d[kTreeGroup];
+  Tree d[N];
 };
+static_assert(sizeof(TreeBatch<kTreeMany>) + 64 <= 32764, "kernel parameters");
 
 __device__ __forceinline__ double* node_shared(double* dsm, int rows, int k) {
   return node_smem(rows, k) * 8 <= kSmemCap ? dsm : nullptr;
 }
 
 // Level l's nodes: factorised, R into the parent's stack (or the root).
-__global__ void __launch_bounds__(TTB_THREADS) k_tree_up(const __grid_constant__ TreeBatch tb,
+template <int N>
+__global__ void __launch_bounds__(TTB_THREADS) k_tree_up(const __grid_constant__ TreeBatch<N> tb,
                                                          int l) {
   extern __shared__ __align__(16) double dsm[];
   const Tree& t = tb.d[blockIdx.y];
@@ -823,7 +830,8 @@ __global__ void __launch_bounds__(TTB_THREADS) k_tree_up(const __grid_constant__
 
 // The SVD of a tree's root: singular values, right factor, and the left one
 // into the root's place.
-__global__ void __launch_bounds__(TTB_THREADS) k_tree_svd(const __grid_constant__ TreeBatch tb) {
+template <int N>
+__global__ void __launch_bounds__(TTB_THREADS) k_tree_svd(const __grid_constant__ TreeBatch<N> tb) {
   extern __shared__ __align__(16) double dsm[];
   __shared__ double red[TTB_WARPS];
   const Tree& t = tb.d[blockIdx.x];
@@ -840,7 +848,8 @@ __global__ void __launch_bounds__(TTB_THREADS) k_tree_svd(const __grid_constant_
 // block per kTreeSlice of its columns.
 // ``part`` 0: every node; 1: the first node only, a row block into
 // ``first``; 2: every node, the row blocks with their columns signed.
-__global__ void __launch_bounds__(TTB_THREADS) k_tree_down(const __grid_constant__ TreeBatch tb,
+template <int N>
+__global__ void __launch_bounds__(TTB_THREADS) k_tree_down(const __grid_constant__ TreeBatch<N> tb,
                                                            int l, int part) {
   extern __shared__ __align__(16) double dsm[];
   const Tree& t = tb.d[blockIdx.y];
@@ -875,7 +884,8 @@ __global__ void __launch_bounds__(TTB_THREADS) k_tree_down(const __grid_constant
 // first K rows alone by eliminating with d_j = -sign(q_jj) at each step
 // (Ballard et al., "Reconstructing Householder vectors from tall-skinny QR",
 // 2014, section IV).
-__global__ void __launch_bounds__(TTB_THREADS) k_tree_signs(const __grid_constant__ TreeBatch tb) {
+template <int N>
+__global__ void __launch_bounds__(TTB_THREADS) k_tree_signs(const __grid_constant__ TreeBatch<N> tb) {
   extern __shared__ __align__(16) double dsm[];
   const Tree& t = tb.d[blockIdx.x];
   const int K = t.K, ld = odd_step(K), rows = t.rows(0, 0);
@@ -903,16 +913,17 @@ __global__ void __launch_bounds__(TTB_THREADS) k_tree_signs(const __grid_constan
   }
 }
 
-int g_smem_tree[4][kMaxDevices];
+int g_smem_tree[2][4][kMaxDevices];
 
-int run_trees(const std::vector<Tree>& all, cudaStream_t s) {
-  const void* kernels[4] = {(const void*)k_tree_up, (const void*)k_tree_svd,
-                            (const void*)k_tree_down, (const void*)k_tree_signs};
+template <int N>
+int run_tree_groups(const std::vector<Tree>& all, cudaStream_t s) {
+  const void* kernels[4] = {(const void*)k_tree_up<N>, (const void*)k_tree_svd<N>,
+                            (const void*)k_tree_down<N>, (const void*)k_tree_signs<N>};
   for (int i = 0; i < 4; ++i)
-    if (int e = smem_limit_once(kernels[i], kSmemCap, g_smem_tree[i])) return e;
-  for (size_t i0 = 0; i0 < all.size(); i0 += kTreeGroup) {
-    TreeBatch tb;
-    tb.count = (int)std::min<size_t>(kTreeGroup, all.size() - i0);
+    if (int e = smem_limit_once(kernels[i], kSmemCap, g_smem_tree[N == kTreeMany][i])) return e;
+  for (size_t i0 = 0; i0 < all.size(); i0 += N) {
+    TreeBatch<N> tb;
+    tb.count = (int)std::min<size_t>(N, all.size() - i0);
     int levels = 0, most[kTreeLevels] = {};
     i64 smem[kTreeLevels] = {}, square = 0, signs = 0;
     int slices = 1;
@@ -938,34 +949,39 @@ int run_trees(const std::vector<Tree>& all, cudaStream_t s) {
       any_qr = any_qr || !t.svd;
     }
     for (int l = 0; l < levels; ++l) {
-      k_tree_up<<<dim3(most[l], tb.count), TTB_THREADS, (size_t)smem[l], s>>>(tb, l);
+      k_tree_up<N><<<dim3(most[l], tb.count), TTB_THREADS, (size_t)smem[l], s>>>(tb, l);
       counted();
     }
     if (any_svd) {
-      k_tree_svd<<<tb.count, TTB_THREADS, (size_t)square, s>>>(tb);
+      k_tree_svd<N><<<tb.count, TTB_THREADS, (size_t)square, s>>>(tb);
       counted();
       for (int l = levels - 1; any_q && l >= 0; --l) {
-        k_tree_down<<<dim3(most[l], tb.count, slices), TTB_THREADS, (size_t)smem[l], s>>>(tb, l, 0);
+        k_tree_down<N><<<dim3(most[l], tb.count, slices), TTB_THREADS, (size_t)smem[l], s>>>(tb, l, 0);
         counted();
       }
     } else if (any_qr) {
       // without any Q, the signs still need its first rows
       for (int l = levels - 1; l > 0; --l) {
-        k_tree_down<<<dim3(any_q ? most[l] : 1, tb.count, slices), TTB_THREADS, (size_t)smem[l],
+        k_tree_down<N><<<dim3(any_q ? most[l] : 1, tb.count, slices), TTB_THREADS, (size_t)smem[l],
                       s>>>(tb, l, any_q ? 0 : 1);
         counted();
       }
-      k_tree_down<<<dim3(1, tb.count, slices), TTB_THREADS, (size_t)smem[0], s>>>(tb, 0, 1);
+      k_tree_down<N><<<dim3(1, tb.count, slices), TTB_THREADS, (size_t)smem[0], s>>>(tb, 0, 1);
       counted();
-      k_tree_signs<<<tb.count, TTB_THREADS, (size_t)signs, s>>>(tb);
+      k_tree_signs<N><<<tb.count, TTB_THREADS, (size_t)signs, s>>>(tb);
       counted();
       if (any_q) {
-        k_tree_down<<<dim3(most[0], tb.count, slices), TTB_THREADS, (size_t)smem[0], s>>>(tb, 0, 2);
+        k_tree_down<N><<<dim3(most[0], tb.count, slices), TTB_THREADS, (size_t)smem[0], s>>>(tb, 0, 2);
         counted();
       }
     }
   }
   return last_error();
+}
+
+int run_trees(const std::vector<Tree>& all, cudaStream_t s) {
+  return all.size() <= kTreeFew ? run_tree_groups<kTreeFew>(all, s)
+                                : run_tree_groups<kTreeMany>(all, s);
 }
 
 // the one-CTA factorisations' shared-memory limit on the current device
