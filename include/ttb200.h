@@ -180,8 +180,9 @@ long long ttb_qr_work_doubles(int m, int k);
 int ttb_qr(const ttb_qr_t* problems, int count, void* stream);
 
 /* ttb_qr for callers that cannot allocate device memory (no counterpart in
- * the reference).  Same factorisation and results as ttb_qr; the ``work``
- * field is ignored and the work areas come from one fixed array of
+ * the reference).  The results of ttb_qr, bit for bit except for the tall
+ * matrices that ttb_qr factors as trees of row blocks, which agree up to
+ * rounding; the ``work`` field is ignored and the work areas come from one fixed array of
  * TTB_QR_STATIC_DOUBLES doubles (16 MiB) inside the library.  It is meant
  * for a caller whose device memory is all owned by another allocator it may
  * not call into (a serving process that reserved its HBM up front, a

@@ -546,6 +546,12 @@ struct QBatch {
   ttb_qr_t d[kMaxQ];
 };
 
+// Column step of a matrix factored in shared memory: an odd one where there is
+// room for it.
+__host__ __device__ inline int qr_step(int m, int k) {
+  return ((i64)odd_step(m) * k + (m < k ? m : k)) * 8 <= kSmemCap ? odd_step(m) : m;
+}
+
 __global__ void __launch_bounds__(TTB_THREADS) k_qr(const __grid_constant__ QBatch qb) {
   extern __shared__ double dsm[];
   __shared__ double red[TTB_WARPS];
@@ -555,7 +561,7 @@ __global__ void __launch_bounds__(TTB_THREADS) k_qr(const __grid_constant__ QBat
   if (m <= 0 || k <= 0) return;
   if (qb.mode[blockIdx.x] == 0) {
     double* W = dsm;
-    const int ldw = odd_step(m);
+    const int ldw = qr_step(m, k);
     double* tau = W + (i64)ldw * k;
     cta_qr<true>(CMat{q.a, q.a_rs, q.a_cs}, m, k, W, ldw, tau, Mat{q.q, q.q_rs, q.q_cs},
            Mat{q.r, q.r_rs, q.r_cs}, red);
@@ -568,7 +574,8 @@ __global__ void __launch_bounds__(TTB_THREADS) k_qr(const __grid_constant__ QBat
   }
 }
 
-i64 qr_need(int m, int k) { return (i64)odd_step(m) * k + std::min(m, k); }
+i64 qr_need(int m, int k) { return (i64)m * k + std::min(m, k); }
+i64 qr_shared(int m, int k) { return (i64)qr_step(m, k) * k + std::min(m, k); }
 __host__ __device__ inline i64 blocked_smem(int k) {
   return (i64)LNB * (k < 1 ? 1 : k < YCH ? k : YCH) + 2 * LNB * LNB;
 }
@@ -2084,7 +2091,7 @@ int ttb_qr(const ttb_qr_t* ps, int count, void* stream) {
       const i64 blk = blocked_smem(qb.d[j].k) * 8;
       if (whole <= kSmemCap) {
         qb.mode[j] = 0;
-        smem = std::max(smem, whole);
+        smem = std::max(smem, qr_shared(qb.d[j].m, qb.d[j].k) * 8);
       } else {
         if (blk > kSmemCap) return (int)cudaErrorInvalidValue;
         qb.mode[j] = 1;
@@ -2124,7 +2131,7 @@ int ttb_qr_static(const ttb_qr_t* ps, int count, void* stream) {
         if (whole <= kSmemCap) {
           qb.mode[j] = 0;
           qb.d[j].work = nullptr;
-          smem = std::max(smem, whole);
+          smem = std::max(smem, qr_shared(qb.d[j].m, qb.d[j].k) * 8);
         } else {
           const i64 blk = blocked_smem(qb.d[j].k) * 8;
           if (blk > kSmemCap) return (int)cudaErrorInvalidValue;
