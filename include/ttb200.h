@@ -163,8 +163,12 @@ int ttb_project(const ttb_project_t* problems, int count, void* stream);
  * left_orthonormalize / right_orthonormalize (ttnumpy/utils.py:86-136) and
  * _shift_center_right / _shift_center_left
  * (ttnumpy/solvers/one_site.py:181-209).  q or r may be NULL.  ``work``
- * holds ttb_qr_work_doubles(m, k) doubles (used when the factorisation does
- * not fit in shared memory).
+ * holds ttb_qr_work_doubles(m, k) doubles.  It may be NULL where the
+ * factorisation fits in shared memory (8 * (m*k + min(m, k)) bytes up to
+ * 200 KiB), which one thread block then does; a larger problem without it is
+ * refused (cudaErrorInvalidValue) before anything is launched.  With it, tall
+ * matrices above 512 rows go as trees of row blocks where that is faster,
+ * chosen by m, k and whether q is wanted, not by the other problems.
  * --------------------------------------------------------------------- */
 typedef struct {
   const double* a;
@@ -211,12 +215,14 @@ int ttb_qr_static(const ttb_qr_t* problems, int count, void* stream);
  * Thin SVD of an m x k strided matrix, a = u diag(s) vh with s descending,
  * p = min(m, k): u (m x p), s (p), vh (p x k).  Either u or vh may be NULL
  * (not wanted; s times it is then the other factor's product with a).
- * Householder QR followed by one-sided Jacobi on the triangular factor.  Replaces the LAPACK gesdd /
- * gesvd calls of left_svd / right_svd (ttnumpy/utils.py:336-460) and of
+ * Householder QR followed by one-sided Jacobi on the triangular factor.
+ * Replaces the LAPACK gesdd / gesvd calls of left_svd / right_svd (ttnumpy/utils.py:336-460) and of
  * _truncate_core_right / _left (ttnumpy/solvers/amen.py:254-260, 301-307).
  * ``status`` (device int, may be NULL) receives the Jacobi sweeps used or
  * -1 when the sweep cap was reached.  ``work`` holds
- * ttb_svd_work_doubles(m, k) doubles.
+ * ttb_svd_work_doubles(m, k) doubles; a problem without it goes to one thread
+ * block if its work areas fit in shared memory (200 KiB) and is refused
+ * (cudaErrorInvalidValue) otherwise.
  * --------------------------------------------------------------------- */
 typedef struct {
   const double* a;

@@ -1,5 +1,5 @@
-"""The limits that the header states for the QR entry points: what fits shared
-memory, and what ttb_qr_static takes."""
+"""The limits that the header states for the QR and SVD entry points: what fits
+shared memory, and what ttb_qr_static takes.  Each refusal is the host's."""
 
 import ctypes as C
 
@@ -53,3 +53,41 @@ def test_static_takes_what_the_header_says(K, m, k):
 def test_static_refuses_more(K):
     a = np.random.default_rng(0).standard_normal((1449, 1448))
     assert factor(K, "ttb_qr_static", a)[0] == -2
+
+
+@pytest.mark.parametrize("m,k", [(600, 8), (600, 40), (1600, 15), (3000, 8), (160, 159)])
+def test_qr_without_work_areas_in_shared_memory(K, m, k):
+    a = np.random.default_rng(m).standard_normal((m, k))
+    code, q, r = factor(K, "ttb_qr", a)
+    assert code == 0
+    check(a, q, r)
+
+
+def svd(K, a):
+    from ttnumpy_b200 import _lib
+
+    m, k = a.shape
+    dev = torch.from_numpy(a).cuda()
+    u, s, vh = K.empty(m, k), K.empty(k), K.empty(k, k)
+    d = (_lib.SVD * 1)(_lib.SVD(K.ptr(dev), k, 1, K.ptr(u), k, 1, K.ptr(s), K.ptr(vh), k, 1, None,
+                                None, m, k))
+    code = K.lib().ttb_svd(d, 1, K.stream())
+    torch.cuda.synchronize()
+    return code, u.cpu().numpy(), s.cpu().numpy(), vh.cpu().numpy()
+
+
+@pytest.mark.parametrize("m,k", [(700, 20), (2000, 10)])
+def test_svd_without_work_areas_in_shared_memory(K, m, k):
+    a = np.random.default_rng(m).standard_normal((m, k))
+    code, u, s, vh = svd(K, a)
+    assert code == 0
+    tol = (4 * k * (m / 32 + 16) + 24 * k * k) * EPS  # the QR, and six sweeps of rotations
+    assert np.linalg.norm((u * s) @ vh - a) <= tol * np.linalg.norm(a)
+
+
+def test_what_does_not_fit_is_refused_without_work_areas(K):
+    before = K.launch_count()
+    a = np.random.default_rng(0).standard_normal((900, 40))
+    assert factor(K, "ttb_qr", a)[0] == 1  # cudaErrorInvalidValue
+    assert svd(K, a)[0] == 1
+    assert K.launch_count() == before

@@ -2055,6 +2055,10 @@ long long ttb_qr_work_doubles(int m, int k) {
 int ttb_qr(const ttb_qr_t* ps, int count, void* stream) {
   if (int e = configure_smem()) return e;
   cudaStream_t s = as_stream(stream);
+  // Without work areas only what fits shared memory can be factored.
+  for (int i = 0; i < count; ++i)
+    if (!ps[i].work && qr_need(ps[i].m, ps[i].k) * 8 > kSmemCap)
+      return (int)cudaErrorInvalidValue;
   // A problem's shape alone decides how it is factored, so that its bits do not
   // depend on the other problems of the call.
   std::vector<ttb_qr_t> rest;
@@ -2062,7 +2066,7 @@ int ttb_qr(const ttb_qr_t* ps, int count, void* stream) {
   double fl = 0.0;
   for (int i = 0; i < count; ++i) {
     const ttb_qr_t& p = ps[i];
-    if (!tree_shape(p.m, p.k, p.q ? TREE_QR : TREE_R)) {
+    if (!p.work || !tree_shape(p.m, p.k, p.q ? TREE_QR : TREE_R)) {
       rest.push_back(p);
       continue;
     }
@@ -2163,12 +2167,16 @@ long long ttb_svd_work_doubles(int m, int k) {
 int ttb_svd(const ttb_svd_t* ps, int count, void* stream) {
   if (int e = configure_smem()) return e;
   cudaStream_t s = as_stream(stream);
+  for (int i = 0; i < count; ++i)
+    if (!ps[i].work &&
+        svd_tall_need(std::max(ps[i].m, ps[i].k), std::min(ps[i].m, ps[i].k)) * 8 > kSmemCap)
+      return (int)cudaErrorInvalidValue;
   std::vector<ttb_svd_t> rest;  // trees by the shape alone, as in ttb_qr
   std::vector<Tree> trees;
   double fl = 0.0;
   for (int i = 0; i < count; ++i) {
     const ttb_svd_t& p = ps[i];
-    if (!tree_shape(std::max(p.m, p.k), std::min(p.m, p.k), TREE_SVD)) {
+    if (!p.work || !tree_shape(std::max(p.m, p.k), std::min(p.m, p.k), TREE_SVD)) {
       rest.push_back(p);
       continue;
     }
