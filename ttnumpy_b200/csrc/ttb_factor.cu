@@ -1819,24 +1819,25 @@ static __device__ __forceinline__ int lu_steps(double (&x)[CPW][RPL], int (&pos)
 #pragma unroll
         for (int r = 0; r < RPL; ++r) col[r] = fma(-l[r], u, col[r]);
       }
-      // the largest entry, the lowest position on ties (a NaN is never
-      // larger): its high word, its low word, then position and row
+      // the largest entry, the lowest position on ties, a NaN only where no
+      // number is left (at -0.5, below all of them): by the high word (one up,
+      // so that a zero is not a NaN's 0), the low word, then position and row
       double best = -1.0;
       unsigned at = 0x7fffffffu;
 #pragma unroll
       for (int r = 0; r < RPL; ++r) {
         const int row = lane + 32 * r;
-        const double a = fabs(col[r]);
+        const double a = col[r] == col[r] ? fabs(col[r]) : -0.5;
         const unsigned id = ((unsigned)pos[r] << 16) | row;
         const bool in = row < rows && pos[r] >= n;
-        if (in && (a > best || (!(a < best) && id < at))) {
+        if (in && (a > best || (a == best && id < at))) {
           best = a;
           at = id;
         }
       }
-      const unsigned hi = at == 0x7fffffffu ? 0u : (unsigned)__double2hiint(best);
+      const unsigned hi = best < 0.0 ? 0u : (unsigned)__double2hiint(best) + 1u;
       const unsigned top = __reduce_max_sync(0xffffffffu, hi);
-      const unsigned lo = hi == top ? (unsigned)__double2loint(best) : 0u;
+      const unsigned lo = hi == top && hi ? (unsigned)__double2loint(best) : 0u;
       const unsigned low = __reduce_max_sync(0xffffffffu, lo);
       at = __reduce_min_sync(0xffffffffu, hi == top && lo == low ? at : 0x7fffffffu);
       const int pr = (int)(at & 0xffff);
