@@ -43,3 +43,16 @@ def test_nan_beside_numbers(K, n):
     a[n // 2, 0] = np.nan
     info, x = solve(K, a, np.ones(n))
     assert info == 0 and np.isnan(x).all()
+
+
+@pytest.mark.parametrize("n", [1030, 1700])
+def test_column_of_nan(K, n):
+    """Beyond the registers: once only rows of NaN are left, a column has no
+    largest entry; its pivot stays on the diagonal."""
+    a = np.random.default_rng(n).standard_normal((n, n))
+    a[n // 2, 0] = np.nan
+    info, x = solve(K, a, np.ones(n))
+    assert info == 0 and np.isnan(x).all()
+    a[:] = np.nan
+    info, x = solve(K, a, np.ones(n))
+    assert info == 0 and np.isnan(x).all()

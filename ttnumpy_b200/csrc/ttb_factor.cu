@@ -2223,7 +2223,8 @@ __device__ __noinline__ int cta_gepp_blocked(double* W, i64 ld, double* b, int n
         double a = fabs(P[i + (i64)c * rows]);
         if (a > best) { best = a; bi = i; }
       }
-      const int piv = block_argmax_abs(best, bi, redv, redi);
+      // a column of NaN has no largest entry (-1): its own row
+      const int piv = max(block_argmax_abs(best, bi, redv, redi), c);
       if (tid == 0) ipiv[c] = piv;
       if (piv != c) {
         for (int cc = tid; cc < jb; cc += TTB_THREADS) {
