@@ -816,8 +816,11 @@ def right_svd_sweep(cores: List[torch.Tensor], error: float, max_rank=None) -> N
         matrix = cores[i].reshape(s[0], s[1] * s[2] * s[3])
         _, sv, vh = K.svd(matrix, want_u=False)
         nb = _svd_rank(sv, delta, max_rank)
-        core = vh[:nb].view(nb, s[1], s[2], s[3])
-        carry = K.matmul(matrix, vh[:nb].t())  # U S
+        rows = vh[:nb]
+        carry = K.matmul(matrix, rows.t())  # U S
+        if nb < vh.shape[0]:  # not a view that keeps all of Vh
+            rows = K.copy_(K.empty(nb, vh.shape[1]), rows)
+        core = rows.view(nb, s[1], s[2], s[3])
         cores[i] = core
         cores[i - 1] = _apply_right(cores[i - 1], carry)
 
