@@ -839,7 +839,7 @@ def round_in_one_launch(cores: List[torch.Tensor], error: float,
     d = len(cores)
     modes = [c.shape[1] * c.shape[2] for c in cores]
     bonds = [c.shape[0] for c in cores] + [1]
-    if (d > 64 or min(modes) < 1 or min(bonds) < 1 or max(bonds) > 64
+    if (d < 2 or d > 64 or min(modes) < 1 or min(bonds) < 1 or max(bonds) > 64
             or any(modes[k] * max(bonds[k], bonds[k + 1]) > 256 for k in range(d))):
         return None
     cores = [c.contiguous() for c in cores]
