@@ -1050,9 +1050,9 @@ __device__ __noinline__ void form_local(const double* lenv, const double* core, 
                                         const LocalDims& L, double* W, int rank, int size) {
   const int Nn = L.lf * L.n * L.rf;
   constexpr int kRegs = 8;  // left operator bonds held in registers at a time
-  const int items = Nn * L.m * L.rt;
-  for (int e = rank * TTB_THREADS + threadIdx.x; e < items; e += size * TTB_THREADS) {
-    const int row = e % Nn, q = e / Nn, mt = q % L.rt, l = q / L.rt;
+  for (TableWalk e(rank * TTB_THREADS + threadIdx.x, size * TTB_THREADS, Nn); e.row < L.m * L.rt;
+       e.next()) {
+    const int row = e.at, mt = e.row % L.rt, l = e.row / L.rt;
     const int nf = row % L.rf, kr = (row / L.rf) % L.n, j = row / (L.rf * L.n);
     for (int a0 = 0; a0 < L.R; a0 += kRegs) {
       double t[kRegs];

@@ -96,6 +96,27 @@ __host__ __device__ constexpr int odd_step(int m) { return m | 1; }
 // start on 16-byte boundaries and two neighbours cover all the banks.
 __host__ __device__ constexpr int svd_step(int k) { return k + ((8 - k) & 15); }
 
+// A thread's walk over a table of rows of ``width`` entries: the entries first,
+// first + stride, ... (first < 2^31) as row and place in it, advanced without a
+// division and without a count of entries, which may pass 32 bits.
+struct TableWalk {
+  int row, at;
+  __host__ __device__ TableWalk(int first, int stride, int width_)
+      : row(first / width_), at(first % width_), rows(stride / width_), rest(stride % width_),
+        width(width_) {}
+  __host__ __device__ __forceinline__ void next() {
+    row += rows;
+    at += rest;
+    if (at >= width) {
+      at -= width;
+      ++row;
+    }
+  }
+
+ private:
+  int rows, rest, width;
+};
+
 // The first 16-byte boundary at or after p.
 __device__ __forceinline__ double* align2(double* p) {
   return reinterpret_cast<double*>((reinterpret_cast<uintptr_t>(p) + 15) & ~(uintptr_t)15);
