@@ -1254,7 +1254,7 @@ static __device__ __forceinline__ bool jacobi_round(double* B, int k, i64 ld, do
 }
 
 // Hestenes' one-sided Jacobi on the columns of the k x k matrix B (column
-// step ld; see cta_jacobi, which it replaces up to k = 256) and, with VACC,
+// step ld; see cta_jacobi, which it replaces up to k = kPivotMax) and, with VACC,
 // V (k x k, the same step) multiplied by the same rotations.  Columns go in
 // blocks of four; a warp loads a pair of blocks into registers, eight lanes
 // to a column, and rotates all their column pairs, four disjoint pairs at a
@@ -1376,9 +1376,10 @@ static __device__ __noinline__ void cta_complete_rows(int k, const double* sv, c
   }
 }
 
-// Largest k of the register-blocked Jacobi iteration, and of the pivoted
-// preconditioner in registers.
-constexpr int kJacobiMax = 256, kPivotMax = 128;
+// Largest k of the register-blocked Jacobi iteration in one block and of the
+// pivoted preconditioner in registers (beyond, a cluster iterates up to
+// kClusterMax, then the plain form).
+constexpr int kPivotMax = 128;
 
 template <bool VACC>
 static __device__ int cta_jacobi_blocks(double* B, int k, i64 ld, double* V, int max_sweeps,
@@ -1387,8 +1388,7 @@ static __device__ int cta_jacobi_blocks(double* B, int k, i64 ld, double* V, int
   if (k <= 32) return jacobi_blocks<4, VACC>(B, k, ld, V, max_sweeps, tol, flag);
   if (k <= 64) return jacobi_blocks<8, VACC>(B, k, ld, V, max_sweeps, tol, flag);
   if (k <= 96) return jacobi_blocks<12, VACC>(B, k, ld, V, max_sweeps, tol, flag);
-  if (k <= 128) return jacobi_blocks<16, VACC>(B, k, ld, V, max_sweeps, tol, flag);
-  return jacobi_blocks<32, VACC>(B, k, ld, V, max_sweeps, tol, flag);
+  return jacobi_blocks<16, VACC>(B, k, ld, V, max_sweeps, tol, flag);  // k <= kPivotMax
 }
 
 // M's upper triangle becomes its transpose in the lower one, the upper
@@ -1555,7 +1555,7 @@ static __device__ __noinline__ int square_iterate(int want, int k, double* Bsq, 
   double *F, *X;
   square_roles(want, k, Bsq, V, F, X);
   const double tol = square_tol(k);
-  if (k > kJacobiMax) return cta_jacobi(X, k, ld, want == SQ_BOTH ? F : nullptr, ld, 60, tol, flag);
+  if (k > kPivotMax) return cta_jacobi(X, k, ld, want == SQ_BOTH ? F : nullptr, ld, 60, tol, flag);
   if (want == SQ_BOTH) return cta_jacobi_blocks<true>(X, k, ld, F, 60, tol, flag);
   return cta_jacobi_blocks<false>(X, k, ld, nullptr, 60, tol, flag);
 }
