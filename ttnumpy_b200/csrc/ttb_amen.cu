@@ -932,12 +932,14 @@ __device__ __noinline__ void project(Ctx& c, const double* left, int a, int i, c
 // factorisations with the shared pool or the blocked global variants
 // ---------------------------------------------------------------------------
 
-// Economic QR of the m x k view A: Q (m x p) and R (p x k) strided outputs.
-// Rows from which a cluster shares the residual norm's factorisations (eight
-// mode-32 diffusion solves on eight blocks each: 626 ms, shared 606 ms); below,
-// the two barriers a column cost as much as a lone block's pass over it.
+// Rows from which a cluster shares the residual norm's factorisations; below,
+// the two barriers a column cost as much as a lone block's pass over it.  On
+// eight blocks each, from 256, 1024 and 2048 rows on, and never: eight mode-32
+// diffusion solves (d = 4) 471, 471, 489 and 489 ms, one of d = 6 and mode 16
+// 337, 338, 350 and 386, eight of d = 5 and mode 8 72, 74, 74 and 74.
 constexpr int kQrShare = 1024;
 
+// Economic QR of the m x k view A: Q (m x p) and R (p x k) strided outputs.
 __device__ __noinline__ void qr(Ctx& c, CMat A, int m, int k, Mat Q, Mat R) {
   const int p = min(m, k);
   if ((i64)m * k + p <= kPoolD) {
@@ -1037,7 +1039,6 @@ __device__ __noinline__ void svd(Ctx& c, CMat A, int m, int k, Mat U, double* S,
 // local solves
 // ---------------------------------------------------------------------------
 
-// Explicit local matrix (column major, n x n) and GEPP solve; u <- solution.
 // Explicit local matrix, column major: the items rank, rank + size, ... of
 // the blocks of a cluster.  An item is a row (j, kr, nf) and the part (l, mt)
 // of a column: the operator core times the right environment gives one number
@@ -1083,7 +1084,9 @@ __device__ __noinline__ void form_local(const double* lenv, const double* core, 
 }
 
 // Trailing columns from which a panel's update is worth two cluster barriers
-// and a read of the panel by every block.
+// and a read of the panel by every block: from 32, 96, 192 and 384 on, eight
+// mode-32 diffusion solves take 471, 471, 472 and 483 ms, eight of d = 5 and
+// mode 8 74.3, 74.2, 74.6 and 76.8.
 constexpr int kLuShare = 96;
 
 // cta_gepp_blocked with the strips of each panel's update shared out; W and b
@@ -1111,6 +1114,7 @@ __device__ __noinline__ int cluster_gepp(Ctx& c, double* W, double* b, int n) {
   return 0;
 }
 
+// Explicit local matrix (column major, n x n) and GEPP solve; u <- solution.
 __device__ __noinline__ void direct_solve(Ctx& c, const LocalOp& L, const double* b, double* u) {
   const i64 N = (i64)L.lf * L.n * L.rf;
   const i64 mark = c.top;
