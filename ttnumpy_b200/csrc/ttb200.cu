@@ -248,18 +248,21 @@ constexpr i64 kKronFlat = 2048;
 __host__ __device__ inline i64 kron_outputs(const ttb_kron_t& q) {
   return (i64)q.ra * q.rx * q.n * q.kk * q.ra2 * q.rx2;
 }
-// How a product is formed: each output by a thread; rows (b, y) of at least 32
-// outputs by a warp each, where there are enough of them (no division for each
-// output: mode 2, bond 64 times 64, 298 and 149 us); or rows searched, their
-// columns and numbers counted in 32 bits.
-enum { KRON_FLAT = 0, KRON_ROWS = 1, KRON_SEARCH = 2 };
-__host__ __device__ inline int kron_form(const ttb_kron_t& q) {
-  const i64 outputs = kron_outputs(q), wide = (i64)q.ra2 * q.rx2;
-  if ((q.m >= kKronMode || (q.m >= kKronSmallMode && outputs >= kKronMany)) &&
-      (i64)q.kk * q.rx2 <= 0x7fffffff - 512 && (i64)q.ra * q.n <= 0x7fffffff - 512)
-    return KRON_SEARCH;
-  return wide >= 32 && wide <= 0x7fffffff && outputs >= wide * kKronFull * TTB_WARPS ? KRON_ROWS
-                                                                                      : KRON_FLAT;
+// Whether a product may be searched (columns and rows are counted in 32 bits
+// there), and whether it should be.
+__host__ __device__ inline bool kron_may_search(const ttb_kron_t& q) {
+  return q.m >= kKronSmallMode && (i64)q.kk * q.rx2 <= 0x7fffffff - 512 &&
+         (i64)q.ra * q.n <= 0x7fffffff - 512;
+}
+__host__ __device__ inline bool kron_search(const ttb_kron_t& q) {
+  return kron_may_search(q) && (q.m >= kKronMode || kron_outputs(q) >= kKronMany);
+}
+// Outputs one by one: rows (b, y) of at least 32 go to a warp each where there
+// are enough of them (no division for each output: mode 2, bond 64 times 64,
+// 298 and 149 us).
+__host__ __device__ inline bool kron_by_rows(const ttb_kron_t& q) {
+  const i64 wide = (i64)q.ra2 * q.rx2;
+  return wide >= 32 && wide <= 0x7fffffff && kron_outputs(q) >= wide * kKronFull * TTB_WARPS;
 }
 // A mode so large that 32 columns do not fit reads the core from memory.
 __host__ __device__ inline bool kron_in_slab(const ttb_kron_t& q) {
@@ -269,10 +272,10 @@ __host__ __device__ inline int kron_cols(const ttb_kron_t& q) {
   const int fit = std::max(32, kKronSlab / 8 / q.m / 32 * 32);
   return std::min(fit, q.kk * q.rx2);
 }
-__host__ __device__ inline i64 kron_blocks(const ttb_kron_t& q, int rows) {
+__host__ __device__ inline i64 kron_blocks(const ttb_kron_t& q, int rows, bool search) {
   const i64 outputs = kron_outputs(q);
   if (outputs <= 0) return 0;
-  if (kron_form(q) != KRON_SEARCH) {
+  if (!search) {
     const i64 all = (outputs + TTB_THREADS - 1) / TTB_THREADS;
     return all < kKronFlat ? all : kKronFlat;
   }
@@ -362,46 +365,43 @@ __device__ __forceinline__ void kron_rows(const ttb_kron_t& q, const double* fro
 }
 
 // out[(a, x), i, k, (b, y)] = sum_j op[a, i, j, b] core[x, j, k, y], the
-// outputs dealt out to the threads; I indexes them.
+// outputs dealt out to the threads, or, in rows, the (a, x, i, k) to the warps;
+// I indexes them.
 template <typename I>
 __global__ void __launch_bounds__(TTB_THREADS, 4) k_kron_flat(const __grid_constant__ KBatch kb) {
   const ttb_kron_t& q = kb.d[blockIdx.y];
-  const i64 blocks = kron_blocks(q, kb.rows), total = kron_outputs(q);
+  const i64 blocks = kron_blocks(q, kb.rows, false), total = kron_outputs(q);
   if ((i64)blockIdx.x >= blocks) return;
   const i64 astep = q.ra2, cstep = (i64)q.kk * q.rx2;
-  for (i64 e = (i64)blockIdx.x * TTB_THREADS + threadIdx.x; e < total; e += blocks * TTB_THREADS) {
-    I r = (I)e;
-    const I y = r % (I)q.rx2; r /= (I)q.rx2;
-    const I b = r % (I)q.ra2; r /= (I)q.ra2;
+  if (!kron_by_rows(q)) {
+    for (i64 e = (i64)blockIdx.x * TTB_THREADS + threadIdx.x; e < total;
+         e += blocks * TTB_THREADS) {
+      I r = (I)e;
+      const I y = r % (I)q.rx2; r /= (I)q.rx2;
+      const I b = r % (I)q.ra2; r /= (I)q.ra2;
+      const I k = r % (I)q.kk; r /= (I)q.kk;
+      const I i = r % (I)q.n; r /= (I)q.n;
+      const I x = r % (I)q.rx, a = r / (I)q.rx;
+      const double* op = q.op + ((i64)a * q.n + i) * q.m * astep + b;
+      const double* cr = q.core + (i64)x * q.m * cstep + (i64)k * q.rx2 + y;
+      double s = 0.0;
+      for (int j = 0; j < q.m; ++j) s = fma(op[j * astep], cr[j * cstep], s);
+      q.out[e] = s;
+    }
+    return;
+  }
+  const int wide = q.ra2 * q.rx2, lane = threadIdx.x & 31;
+  const I rows = (I)(total / wide);
+  const int on = 32 / q.rx2, rest = 32 - on * q.rx2;  // 32 outputs on: b and y
+  const int b0 = lane / q.rx2, y0 = lane - b0 * q.rx2;
+  for (I e = (I)blockIdx.x * TTB_WARPS + (threadIdx.x >> 5); e < rows; e += (I)blocks * TTB_WARPS) {
+    I r = e;
     const I k = r % (I)q.kk; r /= (I)q.kk;
     const I i = r % (I)q.n; r /= (I)q.n;
     const I x = r % (I)q.rx, a = r / (I)q.rx;
-    const double* op = q.op + ((i64)a * q.n + i) * q.m * astep + b;
-    const double* cr = q.core + (i64)x * q.m * cstep + (i64)k * q.rx2 + y;
-    double s = 0.0;
-    for (int j = 0; j < q.m; ++j) s = fma(op[j * astep], cr[j * cstep], s);
-    q.out[e] = s;
-  }
-}
-
-// The same, the rows (a, x, i, k) dealt out to the warps.
-__global__ void __launch_bounds__(TTB_THREADS, 3) k_kron_rows(const __grid_constant__ KBatch kb) {
-  const ttb_kron_t& q = kb.d[blockIdx.y];
-  const i64 blocks = kron_blocks(q, kb.rows);
-  if ((i64)blockIdx.x >= blocks) return;
-  const int wide = q.ra2 * q.rx2, lane = threadIdx.x & 31;
-  const i64 rows = kron_outputs(q) / wide, astep = q.ra2, cstep = (i64)q.kk * q.rx2;
-  const int on = 32 / q.rx2, rest = 32 - on * q.rx2;  // 32 outputs on: b and y
-  const int b0 = lane / q.rx2, y0 = lane - b0 * q.rx2;
-  for (i64 e = (i64)blockIdx.x * TTB_WARPS + (threadIdx.x >> 5); e < rows;
-       e += blocks * TTB_WARPS) {
-    i64 r = e;
-    const i64 k = r % q.kk; r /= q.kk;
-    const i64 i = r % q.n; r /= q.n;
-    const i64 x = r % q.rx, a = r / q.rx;
-    const double* op = q.op + (a * q.n + i) * q.m * astep;
-    const double* cr = q.core + x * q.m * cstep + k * q.rx2;
-    double* out = q.out + e * wide;
+    const double* op = q.op + ((i64)a * q.n + i) * q.m * astep;
+    const double* cr = q.core + (i64)x * q.m * cstep + (i64)k * q.rx2;
+    double* out = q.out + (i64)e * wide;
     int b = b0, y = y0;
     for (int c = lane; c < wide; c += 32) {
       double s = 0.0;
@@ -433,7 +433,7 @@ __global__ void __launch_bounds__(TTB_THREADS, 4) k_kron(const __grid_constant__
   extern __shared__ double slab[];
   __shared__ double2 entries[TTB_WARPS][16];
   const ttb_kron_t& q = kb.d[blockIdx.y];
-  if ((i64)blockIdx.x >= kron_blocks(q, kb.rows)) return;
+  if ((i64)blockIdx.x >= kron_blocks(q, kb.rows, true)) return;
   const int cols = q.kk * q.rx2, ct = kron_cols(q);
   const int nrc = (q.ra * q.n + kb.rows - 1) / kb.rows;
   const int nct = (cols + ct - 1) / ct;
@@ -2297,29 +2297,34 @@ int ttb_kron(const ttb_kron_t* ps, int count, void* stream) {
   if (int e = smem_limit_once((const void*)k_kron, kSmemCap, g_smem_kron)) return e;
   for (int i0 = 0; i0 < count; i0 += kMaxK) {
     ProfScope prof(P_KRON, s, 0.0, 0.0);
-    for (int form = KRON_FLAT; form <= KRON_SEARCH; ++form) {  // a launch for each there is
+    const int n = std::min(count, i0 + kMaxK);
+    // one launch where one form does: a product too small to be searched for
+    // itself is, beside others that are (a second launch adds 3 us to a call)
+    bool any = false;
+    for (int j = i0; j < n; ++j) any = any || kron_search(ps[j]);
+    for (const bool search : {false, true}) {
       KBatch kb;
       kb.count = 0;
       i64 most = 0, smem = 0, all = 0, outputs = 0;
       int modes = 0;
-      for (int j = i0; j < std::min(count, i0 + kMaxK); ++j) {
-        if (kron_form(ps[j]) != form) continue;
+      for (int j = i0; j < n; ++j) {
+        if ((any && kron_may_search(ps[j])) != search) continue;
         kb.d[kb.count++] = ps[j];
-        all += kron_blocks(ps[j], kKronRows);
+        all += kron_blocks(ps[j], kKronRows, search);
         outputs = std::max(outputs, kron_outputs(ps[j]));
         modes = std::max(modes, ps[j].m);
       }
-      kb.rows = all >= kKronFull ? kKronRows : modes <= kKronMidMode ? kKronFewRows : 2 * kKronFewRows;
+      kb.rows = all >= kKronFull ? kKronRows
+                                 : modes <= kKronMidMode ? kKronFewRows : 2 * kKronFewRows;
       for (int j = 0; j < kb.count; ++j) {
-        most = std::max(most, kron_blocks(kb.d[j], kb.rows));
-        if (form == KRON_SEARCH && kron_in_slab(kb.d[j]))
+        most = std::max(most, kron_blocks(kb.d[j], kb.rows, search));
+        if (search && kron_in_slab(kb.d[j]))
           smem = std::max(smem, (i64)kb.d[j].m * kron_cols(kb.d[j]) * 8);
       }
       if (most == 0) continue;
       if (most > 0x7fffffff) return (int)cudaErrorInvalidValue;
       const dim3 grid((unsigned)most, kb.count);
-      if (form == KRON_SEARCH) k_kron<<<grid, TTB_THREADS, (size_t)smem, s>>>(kb);
-      else if (form == KRON_ROWS) k_kron_rows<<<grid, TTB_THREADS, 0, s>>>(kb);
+      if (search) k_kron<<<grid, TTB_THREADS, (size_t)smem, s>>>(kb);
       else if (outputs <= 0x7fffffff) k_kron_flat<unsigned><<<grid, TTB_THREADS, 0, s>>>(kb);
       else k_kron_flat<i64><<<grid, TTB_THREADS, 0, s>>>(kb);
       counted();
