@@ -70,3 +70,11 @@ def test_small_svd_of_nan_ends(K):
     a = torch.full((20, 3), float("nan"), dtype=torch.float64, device="cuda")
     u, s, vh = K.svd(a)
     assert torch.isnan(s).all() and u.shape == (20, 3) and vh.shape == (3, 3)
+
+
+@pytest.mark.parametrize("k", [1, 3, 6, 8])
+def test_a_nan_leaves_no_singular_value(K, k):
+    a = np.random.default_rng(k).standard_normal((40, k))
+    a[7, k // 2] = np.nan
+    u, s, vh = K.svd(torch.from_numpy(a).cuda())
+    assert torch.isnan(s).all() and torch.isnan(vh).all() and torch.isnan(u).any()

@@ -1631,6 +1631,16 @@ static __device__ __noinline__ int cta_svd_small(int want, int k, double* B, dou
   }
   __syncthreads();
   const int zero = __syncthreads_or(threadIdx.x < k && sv[threadIdx.x] == 0.0);
+  // a NaN anywhere leaves no value or vector defined, as after the pivoted QRs
+  if (__syncthreads_or(threadIdx.x < k && sv[threadIdx.x] != sv[threadIdx.x])) {
+    if (threadIdx.x < k) S[threadIdx.x] = NAN;
+    for (int e = threadIdx.x; e < k * k; e += TTB_THREADS) {
+      if (J) Vh(e / k, e % k) = NAN;
+      B[e % k + (e / k) * ld] = NAN;
+    }
+    __syncthreads();
+    return status;
+  }
   if (threadIdx.x < k) S[threadIdx.x] = sv[order[threadIdx.x]];
   for (int e = threadIdx.x; e < k * k; e += TTB_THREADS) {
     const int i = e % k, j = e / k;
