@@ -186,12 +186,12 @@ int ttb_qr(const ttb_qr_t* problems, int count, void* stream);
 /* ttb_qr for callers that cannot allocate device memory (no counterpart in
  * the reference).  The results of ttb_qr, bit for bit except for the tall
  * matrices that ttb_qr factors as trees of row blocks, which agree up to
- * rounding; the ``work`` field is ignored and the work areas come from one fixed array of
- * TTB_QR_STATIC_DOUBLES doubles (16 MiB) inside the library.  It is meant
- * for a caller whose device memory is all owned by another allocator it may
- * not call into (a serving process that reserved its HBM up front, a
- * host-language binding that holds only its input and output buffers), or
- * that must not take the implicit device synchronisation of
+ * rounding; the ``work`` field is ignored and the work areas come from one
+ * fixed array of TTB_QR_STATIC_DOUBLES doubles (16 MiB) inside the library.
+ * It is meant for a caller whose device memory is all owned by another
+ * allocator it may not call into (a serving process that reserved its HBM up
+ * front, a host-language binding that holds only its input and output
+ * buffers), or that must not take the implicit device synchronisation of
  * cudaMalloc/cudaFree.
  *
  * Limit: the problems of one call that do not fit in shared memory
@@ -245,8 +245,10 @@ int ttb_svd(const ttb_svd_t* problems, int count, void* stream);
  * (ttnumpy/solvers/common.py:766-774).  a is n x n column major with
  * leading dimension lda and is overwritten; b (n) is overwritten with x.
  * ``info`` (device int, may be NULL) receives 0 or the 1-based index of a
- * zero pivot.  Systems up to n = 161 are factored in shared memory; larger
- * ones by panels of 16 columns with GEMM trailing updates.
+ * zero pivot.  A NaN is a pivot only where its column has no number left.
+ * Systems up to n = 160 are factored in registers, up to 1024 by panels of 16
+ * columns in registers, larger ones by panels in shared memory (from n = 1601
+ * on in ``work``), with trailing updates on the FP64 tensor path.
  * --------------------------------------------------------------------- */
 typedef struct {
   double* a;

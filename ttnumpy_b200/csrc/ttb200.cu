@@ -229,10 +229,10 @@ struct KBatch {
 // A row of the operator core is searched for its nonzeros where that saves
 // more than the search costs, a ballot for each bond of a row whatever the mode:
 // from modes of 32 on, and of 16 where there are many outputs.  Otherwise the
-// outputs are formed one by one.  Mode 2, bond 64, times bond 8: 8 us one by one
+// outputs are formed one by one.  Mode 2, bond 64, times bond 8: 7 us one by one
 // and 142 searched; banded mode 16, bond 4, times bond 64: 34 us one by one and 9
 // searched (dense 16), times bond 20 5.6 and 12.9; banded mode 32, bond 4, times
-// bond 8: 7.3 and 5.0 us (dense 6.0).
+// bond 8: 7.3 and 4.8 us (dense 6.0).
 constexpr int kKronMode = 32, kKronSmallMode = 16;
 constexpr i64 kKronMany = 1 << 17;
 // Rows of a block where the launch fills the device (two blocks for each of
@@ -259,7 +259,7 @@ __host__ __device__ inline bool kron_search(const ttb_kron_t& q) {
 }
 // Outputs one by one: rows (b, y) of at least 32 go to a warp each where there
 // are enough of them (no division for each output: mode 2, bond 64 times 64,
-// 298 and 149 us).
+// 298 and 108 us).
 __host__ __device__ inline bool kron_by_rows(const ttb_kron_t& q) {
   const i64 wide = (i64)q.ra2 * q.rx2;
   return wide >= 32 && wide <= 0x7fffffff && kron_outputs(q) >= wide * kKronFull * TTB_WARPS;

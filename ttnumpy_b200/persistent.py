@@ -1,7 +1,7 @@
 """Many AMEn solves in one persistent launch (``ttb_amen_persistent``).
 
-Each request becomes one thread block that runs the whole solve on the
-device (``csrc/ttb_amen.cu``).  The host packs every request's operator,
+Each request becomes one thread block, or one cluster of blocks, that runs the
+whole solve on the device (``csrc/ttb_amen.cu``).  The host packs every request's operator,
 right-hand side, initial guess and random residual start into a few large
 buffers (one host-to-device copy), builds the task table, launches once and
 reads back the bonds, stop reasons and residual histories.  A solve whose
@@ -419,11 +419,12 @@ def spread(count: int, sms: int) -> int:
     cluster shares out its products, eliminations and long vector passes,
     each block computing its share as the lone block would, so results are
     the same bits.  Eight 4-dimensional diffusion solves on 1 / 2 / 8 blocks
-    each: mode 32 960 / 766 / 626 ms, mode 16 186 / 163 / 140 ms; 5
-    dimensions of mode 8 123 / 103 / 85 ms; 32 Poisson systems on trains of
-    mode 2 68 / 61 ms on 1 / 2.  Past the multiprocessors clusters wait for
-    one another: 36 solves of mode 32 took 1156 ms alone, 992 ms in pairs
-    and 1213 ms in fours."""
+    each: mode 32 932 / 739 / 583 ms, mode 16 178 / 155 / 136 ms; 5
+    dimensions of mode 8 113 / 94 / 78 ms; 32 Poisson systems on trains of
+    mode 2 56 / 51 ms on 1 / 2 (a lone one of 2^16 unknowns, whose matrices are
+    too small to share, 25.8 / 25.8 / 26.2).  Past the multiprocessors clusters
+    wait for one another: 36 solves of mode 32 took 1124 ms alone, 886 ms in
+    pairs and 1021 ms in fours."""
     size = 1
     while size < SPREAD_MOST and 4 * size * count <= sms:
         size *= 2
