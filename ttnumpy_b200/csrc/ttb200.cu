@@ -750,13 +750,13 @@ int tree_block(int K) { return K <= 96 ? 256 : 512; }  // rows of a leaf
 //   236, 600 x 40 282 and 288; past that size 900 x 32 714 and 242;
 // - has no more than 2048 rows and eight columns, one tile: 2048 x 8 76 and 80,
 //   1200 x 9 97 and 86;
-// - or little to do: with Q up to 8192 entries (8192 x 1 28 and 45, 2048 x 4 63
+// - or little to do: with Q up to 8192 entries (8192 x 1 28 and 45, 2048 x 4 44
 //   and 58, 12000 x 1 78 and 47), for R alone up to 16384 (16384 x 1 17 and 37,
-//   4096 x 4 44 and 49, 1599 x 10 71 and 80; 6000 x 4 62 and 54).
+//   4096 x 4 45 and 49, 1599 x 10 71 and 80; 6000 x 4 63 and 55).
 // An SVD's tree pays earlier, since its root has the iteration to itself: from
 // 1024 rows and 16 columns on (1024 x 16 173 and 181 us, 1025 x 16 259 and 189,
 // 600 x 20 282 and 259), but for up to 6144 entries (6000 x 1 32 and 40, 3000 x 2
-// 41 and 45, 2048 x 3 51 and 56; 8192 x 1 43 and 40, 2048 x 4 78 and 61).
+// 41 and 45, 2048 x 3 54 and 56; 8192 x 1 43 and 40, 2048 x 4 63 and 62).
 enum { TREE_QR, TREE_R, TREE_SVD };
 bool tree_shape(int M, int K, int what) {
   if (M <= kTreeRows || M >= (1 << 28) || K < 1 || K > kTreeCols || M < 3 * K) return false;

@@ -863,12 +863,14 @@ static __device__ __noinline__ void cta_hh(double* W, i64 ld, int m, int k, doub
 constexpr int kHHTall = 512;
 
 // Whether the register tiles take a matrix: not beyond their rows, and not
-// where a few columns leave most of a tile empty.  512 x 2 with its Q takes 22 us
-// in tiles and 11 us column by column, 256 x 4 21 and 17 us, 256 x 8 31 and 47 us;
-// 64 x 4 10.5 and 11.4, 64 x 3 9.1 and 8.6.
-constexpr int kNarrow = 4, kNarrowRows = 128;
+// where a few columns leave most of a tile empty.  With Q, in tiles and column by
+// column: 512 x 2 22 and 11 us, 256 x 4 21 and 17, 256 x 8 31 and 47; of four
+// columns the shortest and the tallest stay in tiles (64 x 4 10.5 and 11.4,
+// 1024 x 4 30 and 36).
+constexpr int kNarrow = 4, kNarrowShort = 128, kNarrowTall = 640;
 static __device__ __forceinline__ bool hh_tiled(int m, int k) {
-  return m <= kHHRows && (k > kNarrow || (k == kNarrow && m <= kNarrowRows));
+  if (m > kHHRows || k < kNarrow) return false;
+  return k > kNarrow || m <= kNarrowShort || m > kNarrowTall;
 }
 
 // A panel's reflectors: in registers, or column by column.
